@@ -288,10 +288,12 @@ int pppm_pair_weights_static(int device, void *stream, float dt, float dl, float
  * of 4 or more steps with the absorbing boundary).  A change takes effect at the next such call,
  * which records new graphs. */
 #define PPPM_OPT_CONV_PAIRS 0   /* 1 (default): the face-pair convolution streams the pairs' weights
-                                   once for two consecutive steps; 0: once per step             */
+                                   once for several consecutive steps (four, at a call's end two);
+                                   0: once per step                                             */
 #define PPPM_OPT_FACE_THREADS 1 /* threads per block of the face-stage kernels: 64, 128, 256    */
 #define PPPM_OPT_TERMS_PAIRS 2  /* 1 (default): the triangles' grid-cache near-field terms are
-                                   evaluated two steps per pass over their records; 0: per step */
+                                   evaluated several steps per pass over their records (as
+                                   PPPM_OPT_CONV_PAIRS); 0: per step                            */
 #define PPPM_OPT_SPLIT_STENCIL 3 /* 1 (default): the stencil of the corrected cells stays on the
                                     graph's critical branch (the face and near stages read no other
                                     cell) and the rest of the grid runs on a branch beside them;
@@ -300,7 +302,8 @@ int pppm_pair_weights_static(int device, void *stream, float dt, float dl, float
                                    this many steps as often as it fits, then a graph of the 1..32
                                    steps left, so frames of uneven length record a few short
                                    graphs instead of one long graph per length; 0: one graph per
-                                   call; otherwise an even number in [2, 4096].  Same results. */
+                                   call; otherwise an even number in [2, 4096] (rounded up
+                                   to whole passes of four steps).  Same results.               */
 #define PPPM_OPT_STENCIL_VEC4 5 /* the FP32 interior stencil with res a multiple of 4: 1 four
                                    consecutive z cells per thread with 16-byte loads, 0 one cell per
                                    thread, -1 (default) four from res 96 up; pppm_autotune times both
@@ -357,7 +360,11 @@ int pppm_kernel_times(pppm_handle *h, float *us_stencil, float *us_face, float *
                                  convolution: the event-to-event floor of this measurement      */
 #define PPPM_KERNEL_STENCIL_BULK 11 /* the split stencil: every cell but the corrected ones     */
 #define PPPM_KERNEL_STENCIL_CORR 12 /* the split stencil: the corrected cells                   */
-#define PPPM_KERNEL_KINDS 13
+#define PPPM_KERNEL_CONV4 13   /* face-pair convolution, four steps per pass                   */
+#define PPPM_KERNEL_FIX4 14    /* completion of the last step of a four-step pass              */
+#define PPPM_KERNEL_FINISH4 15 /* finish, first step of a four-step pass over the records      */
+#define PPPM_KERNEL_FINISH4C 16 /* ... its last step (completion of its terms)                 */
+#define PPPM_KERNEL_KINDS 17
 int pppm_kernel_profile(pppm_handle *h, int nkinds, float *us_per_launch, long long *launches);
 /* No counterpart in the reference.  Duration of each step kernel kind on the current mesh and
  * state: reps back-to-back launches of the kind (those of the next step) recorded as one CUDA

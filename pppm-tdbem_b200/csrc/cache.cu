@@ -805,7 +805,7 @@ inline long long gather_face_threads(long long pf)
 // step evaluates it) into d1 (float for FP32 handles, double for FP64), which the two-step
 // convolution of the step reads (step.cu: fix_kernel).
 __global__ void denom_kernel(const int *face_start, int nt, const float *area, const __half2 *face_w,
-                             const float2 *face_scale, const double2 *face_wd, double *denom, void *d1)
+                             const float2 *face_scale, const double2 *face_wd, double *denom, void *d, long long pitch)
 {
     int i = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     int lane = threadIdx.x & 31;
@@ -824,14 +824,17 @@ __global__ void denom_kernel(const int *face_start, int nt, const float *area, c
             if (face_wd)
             {
                 fd = face_wd[(size_t)p * kTaps].y;
-                if (d1)
-                    ((double *)d1)[p] = face_wd[(size_t)p * kTaps + 1].y;
+                for (int m = 1; m <= 3; m++)
+                    ((double *)d)[(m - 1) * pitch + p] = face_wd[(size_t)p * kTaps + m].y;
             }
             else
             {
-                f = (float)__high2half(face_w[(size_t)p * kTaps]) * face_scale[p].y;
-                if (d1)
-                    ((float *)d1)[p] = __high2float(face_w[(size_t)p * kTaps + 1]) * face_scale[p].y;
+                const float s = face_scale[p].y;
+                const int4 w = *(const int4 *)(face_w + (size_t)p * kTaps);  // taps 0..3
+                f = (float)__high2half(*(const __half2 *)&w.x) * s;
+                ((float *)d)[p] = __high2float(*(const __half2 *)&w.y) * s;
+                ((float *)d)[pitch + p] = __high2float(*(const __half2 *)&w.z) * s;
+                ((float *)d)[2 * pitch + p] = __high2float(*(const __half2 *)&w.w) * s;
             }
         }
         int cnt = min(32, e - base);
@@ -869,21 +872,25 @@ DevConsts make_consts(const Handle &h)
     return dc;
 }
 
-// Per grid-cache record, the factor of the triangle's NEW Dirichlet value in the record's term
-// one step later (the step's two-step near-field terms, step.cu: near_terms2): double-layer tap 1
-// of the FDTD-near records (r < 27; they pair record tap j + 1 with history tap j) and tap 0 of the
-// BEM-near records, with the record's scale applied as the step applies it.
+// Per grid-cache record, the factors of the triangle's Dirichlet values D[t], D[t-1], D[t-2] in the
+// record's term of time t (the step's passes over several steps leave those products out and add
+// them afterwards, step.cu: near_terms_complete): double-layer taps 0, 1, 2 of the BEM-near records,
+// taps 1, 2, 3 of the FDTD-near records (they pair record tap j + 1 with history tap j), with the
+// record's scale applied; in the terms' order [triangle][offset][FDTD-near, BEM-near], one array
+// per value.
 __global__ void gc_factor_kernel(const __half2 *w, const float2 *scale, const double2 *wd, long long n, float *f,
                                  double *fd)
 {
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
-    const int tap = (i % 54) < 27 ? 1 : 0;
-    if (wd)
-        fd[i] = wd[i * kTaps + tap].y;
-    else
-        f[i] = __high2float(w[i * kTaps + tap]) * scale[i].y;
+    const int k = (int)(i % 54), tap = k & 1 ? 0 : 1;
+    const long long r = i - k + (k >> 1) + (k & 1) * 27;  // the record
+    for (int m = 0; m < 3; m++)
+        if (wd)
+            fd[m * n + i] = wd[r * kTaps + tap + m].y;
+        else
+            f[m * n + i] = __high2float(w[r * kTaps + tap + m]) * scale[r].y;
 }
 
 }  // namespace
@@ -1180,7 +1187,7 @@ static int cache_alloc(Handle &h)
     const int nt = h.nt;
     const size_t rec_bytes = h.fp64 ? kTaps * sizeof(double2) : kTaps * sizeof(__half2);
     PB_TRY(dev_alloc(&h.d_gc_w, (size_t)nt * 54 * rec_bytes));
-    PB_TRY(dev_alloc(&h.d_gc_f, (size_t)nt * 54 * h.real_size));
+    PB_TRY(dev_alloc(&h.d_gc_f, 3 * (size_t)nt * 54 * h.real_size));
     if (!h.fp64)
         PB_TRY(dalloc(&h.d_gc_scale, (size_t)nt * 54));
     PB_TRY(dalloc(&h.d_gc_snap, (size_t)nt * 7));
@@ -1413,7 +1420,7 @@ int cache_refresh(Handle &h)
     denom_kernel<<<div_up((long long)nt * 32, T), T, 0, s>>>(h.d_face_start, nt, h.d_area,
                                               h.fp64 ? nullptr : (const __half2 *)h.d_face_w, h.d_face_scale,
                                               h.fp64 ? (const double2 *)h.d_face_w : nullptr, h.d_face_denom,
-                                              h.d_face_d1);
+                                              h.d_face_d, h.pf_cap);
     h.launches++;
     PB_CHECK_LAUNCH();
     return PPPM_OK;
@@ -1645,7 +1652,7 @@ int cache_regather(Handle &h)
     denom_kernel<<<div_up((long long)h.nt * 32, T), T, 0, s>>>(h.d_face_start, h.nt, h.d_area,
                                                 h.fp64 ? nullptr : (const __half2 *)h.d_face_w, h.d_face_scale,
                                                 h.fp64 ? (const double2 *)h.d_face_w : nullptr, h.d_face_denom,
-                                              h.d_face_d1);
+                                              h.d_face_d, h.pf_cap);
     h.launches++;
     PB_CHECK_LAUNCH();
     return PPPM_OK;

@@ -142,8 +142,9 @@ void free_mesh(Handle &h)
                      (void **)&h.d_face_scale, (void **)&h.d_face_corner, (void **)&h.d_pair_flag,
                      (void **)&h.d_status,     (void **)&h.d_neumann,     (void **)&h.d_dirichlet,
                      (void **)&h.d_hist,       (void **)&h.d_terms,       (void **)&h.d_conv,
-                     (void **)&h.d_gneu,       (void **)&h.d_gneu_old,    (void **)&h.d_face_d1,
-                     (void **)&h.d_conv1,      (void **)&h.d_dlast,       (void **)&h.d_terms1};
+                     (void **)&h.d_gneu,       (void **)&h.d_gneu_old,    (void **)&h.d_face_d,
+                     (void **)&h.d_nfut,       (void **)&h.d_dlast,       (void **)&h.d_part,
+                     (void **)&h.d_groups};
     for (void **q : ptrs)
     {
         dev_free(*q);
@@ -498,11 +499,12 @@ int pppm_set_mesh(pppm_handle *ph, const float *verts, int nv, const int *tris, 
     PB_CUDA(cudaMemsetAsync(h.d_dirichlet, 0, (size_t)nt * kRing * h.real_size, h.stream));
     PB_TRY(dev_alloc(&h.d_hist, (size_t)4 * nt * kHistRow * h.real_size));
     PB_TRY(dev_alloc(&h.d_terms, (size_t)54 * nt * h.real_size));
-    PB_TRY(dev_alloc(&h.d_conv, (size_t)nt * h.real_size));
-    PB_TRY(dev_alloc(&h.d_conv1, (size_t)nt * h.real_size));
-    PB_TRY(dev_alloc(&h.d_dlast, (size_t)nt * h.real_size));
-    PB_TRY(dev_alloc(&h.d_terms1, (size_t)54 * nt * h.real_size));
-    PB_CUDA(cudaMemsetAsync(h.d_dlast, 0, (size_t)nt * h.real_size, h.stream));
+    PB_TRY(dev_alloc(&h.d_conv, 4 * (size_t)nt * h.real_size));
+    PB_TRY(dev_alloc(&h.d_dlast, 4 * (size_t)nt * h.real_size));
+    PB_TRY(dev_alloc(&h.d_nfut, 4 * (size_t)nt * h.real_size));
+    PB_TRY(dev_alloc(&h.d_part, 3 * (size_t)54 * nt * h.real_size));
+    PB_CUDA(cudaMemsetAsync(h.d_dlast, 0, 4 * (size_t)nt * h.real_size, h.stream));
+    PB_CUDA(cudaMemsetAsync(h.d_nfut, 0, 4 * (size_t)nt * h.real_size, h.stream));
     PB_CUDA(cudaMemsetAsync(h.d_hist, 0, (size_t)4 * nt * kHistRow * h.real_size, h.stream));
     int rc = mesh_build(h);
     if (rc != PPPM_OK)

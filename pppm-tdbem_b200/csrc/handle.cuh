@@ -16,7 +16,7 @@
 //                  same for base cells
 //   3^3 pairs      n3 corrected cells: n3_cell, n3_start[n3 + 1]; p3 pairs: p3_tri, p3_woff
 //                  (the pair's record offset in the triangle's grid-cache records)
-//   near terms     terms[nt][54]: each triangle's 54 grid-cache records convolved with its own
+//   near terms     terms[nt][27][2]: each triangle's 54 grid-cache records convolved with its own
 //                  history in the current step (step.cu); a corrected cell sums its pairs' terms
 //   face pairs     face_start[nt + 1] per centre triangle; pf pairs: face_nbr; dense
 //                  weights face_half[pf][32] + face_scale[pf][2]; per centre: 8 corner cells,
@@ -42,8 +42,8 @@ struct StepState
     int n3;            // corrected cells
     long long row0;    // listener-series row of the first step
     const float *acc;  // nsteps rows of nt accelerations, or null
-    // batched runs: steps of time pair0, pair0 + 2, ... start a two-step pass over the face pairs
-    // when their partner (the next time) is at most pair_end; pair_end < pair0: one pass per step
+    // batched runs: the steps of times pair0 .. pair_end go in passes as one call of that many steps
+    // (step.cu: pass_at); pair_end < pair0: one pass per step
     int pair0 = 0, pair_end = -1;
     int conv_pairs = 0, terms_pairs = 0;  // which stages use the pairing (the handle's options)
     // listener series (R elements, row0 is its row of the first step), or null: read from here
@@ -69,6 +69,16 @@ __device__ inline StepDyn bind_step(const StepState *st, int k, int nt)
     d.series = st->series;
     return d;
 }
+
+// Centre triangles that share a base cell, hence one neighbour list in one order (mesh.cu:
+// face_fill_kernel): up to kGroup of them, where each one's face records start and the list length.
+constexpr int kGroup = 2;
+struct alignas(16) CentreGroup
+{
+    int start[kGroup];
+    int tri[kGroup];
+    int n, len;
+};
 
 // a recorded pppm_step call
 struct StepGraph
@@ -137,9 +147,11 @@ struct Handle
     // ---- face pairs (per centre triangle)
     long long pf = 0;
     int *d_face_start = nullptr, *d_face_nbr = nullptr, *d_face_pool = nullptr;
+    CentreGroup *d_groups = nullptr;  // at most nt; their number is in d_status[2]
     void *d_face_w = nullptr;
     float2 *d_face_scale = nullptr;
-    void *d_face_d1 = nullptr;  // pf: double-layer tap 1 of each pair, scale applied (step.cu: fix_kernel)
+    // 3 x pf_cap: double-layer taps 1, 2, 3 of each pair, scale applied (step.cu: face_fix)
+    void *d_face_d = nullptr;
     long long pf_cap = 0;
     int *d_face_corner = nullptr;
     float *d_face_interp = nullptr;
@@ -150,7 +162,7 @@ struct Handle
     bool gc_empty = true;
     void *d_gc_w = nullptr;        // FP32: __half2[nt][54][16]; FP64: double[nt][54][32]
     float2 *d_gc_scale = nullptr;  // FP32: [nt][54]
-    void *d_gc_f = nullptr;        // [nt][54] factor of the new Dirichlet value per record (gc_factors)
+    void *d_gc_f = nullptr;        // 3 x [nt][27][2] factors of the pass's own Dirichlet values (gc_factors)
     float *d_gc_snap = nullptr;    // nt x 7 centre, normal, area at last refresh
     int *d_gc_flag = nullptr;      // nt recompute flags
     int *d_fc_keys = nullptr;      // nt x kFaceCacheSlots neighbour ids, -1 = empty
@@ -169,7 +181,8 @@ struct Handle
     int *d_log_count = nullptr;         // [0] rewrites to log (lookup), [1] log cursor
     struct Journal *journal = nullptr;
     int *d_pair_flag = nullptr;  // pf scratch: 1 = recompute
-    int *d_status = nullptr;     // device-side status word (capacity / timeout)
+    // device words: [0] status (capacity / timeout), [1] a triangle near the boundary layer, [2] centre groups
+    int *d_status = nullptr;
     int *d_step_status = nullptr;  // step status word: non-finite values seen by the step kernels
     int *h_step_status = nullptr;  // pinned copy, written behind each pppm_step call
     cudaEvent_t ev_status = nullptr;  // recorded after that copy
@@ -183,13 +196,13 @@ struct Handle
     void *d_neumann = nullptr, *d_dirichlet = nullptr;  // reference layout: read-out and loading
     void *d_hist = nullptr;  // the step's copies: [4 copies][nt][kHistRow], both fields (step.cu)
     void *d_terms = nullptr;  // nt x 54 near-field terms of the current step (step.cu: near_terms)
-    void *d_conv = nullptr;   // nt face-pair convolution sums of the pipelined step (step.cu)
-    void *d_conv1 = nullptr;  // nt partial sums of the following step (step.cu: conv2_kernel)
-    void *d_dlast = nullptr;  // nt Dirichlet values of the last finished step (step.cu: fix_kernel)
-    void *d_terms1 = nullptr; // nt x 54 partial near-field terms of the following step (near_terms2)
-    int conv_pairs = 1;       // recorded step graphs convolve the face pairs two steps per pass
+    void *d_conv = nullptr;   // 4 x nt face-pair convolution sums of a pass of steps (step.cu)
+    void *d_dlast = nullptr;  // nt x 4 Dirichlet values of a pass's finished steps (step.cu: face_fix)
+    void *d_nfut = nullptr;   // nt x 4 Neumann values of the steps ahead in a four-step pass
+    void *d_part = nullptr;   // 3 x nt x 54 partial near-field terms of a pass's later steps
+    int conv_pairs = 1;       // recorded step graphs convolve the face pairs several steps per pass
     int face_threads = 256;   // threads per block of their face-stage kernels (step_autotune)
-    bool terms_pairs = true;  // ... and the grid-cache near-field terms two steps per pass
+    bool terms_pairs = true;  // ... and the grid-cache near-field terms
     bool split_stencil = true;  // ... and the stencil split into corrected cells and the bulk
     bool corr_near_boundary = false;  // a corrected cell may neighbour the boundary layer (mesh_build)
     int stencil_vec4 = -1;      // interior stencil four cells per thread: 1 on, 0 off, -1 by grid size

@@ -356,10 +356,12 @@ __global__ void face_len_kernel(const int *base, int nt, const int *b4_pos, cons
 
 __global__ void face_fill_kernel(const int *base, const int *basec, int nt, int res, const int *b4_pos,
                                  const int *b4_flag, const int *b4_start, const int *n4_tris, const int *face_start,
-                                 int *face_nbr, int *face_corner)
+                                 const int *base_start, const int *base_tris, int *face_nbr, int *face_corner,
+                                 CentreGroup *groups, int *ngroups)
 {
     // one warp per centre triangle: its 8 trilinear corner cells and a copy of its base cell's
-    // 4^3 list (lanes stride over the list)
+    // 4^3 list (lanes stride over the list).  Every kGroup-th triangle of a base cell also writes the
+    // group of centres it leads (their order among the groups is arbitrary; no result depends on it).
     const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (gw >= nt)
@@ -378,6 +380,33 @@ __global__ void face_fill_kernel(const int *base, const int *basec, int nt, int 
     const int o = face_start[i], s0 = b4_start[k], n = b4_start[k + 1] - s0;
     for (int j = lane; j < n; j += 32)
         face_nbr[o + j] = n4_tris[s0 + j];
+    const int c0 = base_start[b], c1 = base_start[b + 1];
+    int rank = -1;
+    for (int j = c0; j < c1 && rank < 0; j += 32)
+    {
+        const unsigned hit = __ballot_sync(0xffffffffu, j + lane < c1 && base_tris[j + lane] == i);
+        if (hit)
+            rank = j - c0 + __ffs(hit) - 1;
+    }
+    if (rank < 0 || rank % kGroup)
+        return;
+    int gi = 0;
+    if (lane == 0)
+        gi = atomicAdd(ngroups, 1);
+    gi = __shfl_sync(0xffffffffu, gi, 0);
+    CentreGroup &G = groups[gi];
+    const int members = min(kGroup, c1 - c0 - rank);
+    if (lane < kGroup)
+    {
+        const int t = lane < members ? base_tris[c0 + rank + lane] : i;
+        G.tri[lane] = t;
+        G.start[lane] = face_start[t];
+    }
+    if (lane == 0)
+    {
+        G.n = members;
+        G.len = n;
+    }
 }
 
 }  // namespace
@@ -518,6 +547,7 @@ int mesh_build(Handle &h)
         PB_TRY(dalloc(&h.d_b4_start, (size_t)b4_max));
         PB_TRY(dalloc(&h.d_face_start, (size_t)nt + 1));
         PB_TRY(dalloc(&h.d_face_corner, 8 * (size_t)nt));
+        PB_TRY(dalloc(&h.d_groups, (size_t)nt));
         PB_TRY(dalloc(&h.d_status, 4));
     }
     PB_CUDA(cudaMemsetAsync(h.d_status, 0, 4 * sizeof(int), s));
@@ -660,22 +690,23 @@ int mesh_build(Handle &h)
         dev_free(h.d_face_w);
         dev_free(h.d_face_scale);
         dev_free(h.d_pair_flag);
-        dev_free(h.d_face_d1);
+        dev_free(h.d_face_d);
         h.d_face_nbr = h.d_face_pool = h.d_pair_flag = nullptr;
         h.d_face_w = nullptr;
         h.d_face_scale = nullptr;
-        h.d_face_d1 = nullptr;
+        h.d_face_d = nullptr;
         long long cap = pf + pf / 4 + 256;
         PB_TRY(dalloc(&h.d_face_nbr, (size_t)cap));
         PB_TRY(dalloc(&h.d_face_pool, (size_t)cap));
         PB_TRY(dalloc(&h.d_pair_flag, (size_t)cap + 1));
         PB_TRY(dev_alloc(&h.d_face_w, (size_t)cap * (h.fp64 ? 16 * sizeof(double2) : 16 * sizeof(__half2))));
         PB_TRY(dalloc(&h.d_face_scale, (size_t)cap));
-        PB_TRY(dev_alloc(&h.d_face_d1, (size_t)cap * h.real_size));
+        PB_TRY(dev_alloc(&h.d_face_d, 3 * (size_t)cap * h.real_size));
         h.pf_cap = cap;
     }
     face_fill_kernel<<<div_up((long long)nt * 32, T), T, 0, s>>>(h.d_base, h.d_basec, nt, res, b4_pos, flag4, h.d_b4_start,
-                                                 h.d_n4_tris, h.d_face_start, h.d_face_nbr, h.d_face_corner);
+                                                 h.d_n4_tris, h.d_face_start, h.d_base_start, h.d_base_tris,
+                                                 h.d_face_nbr, h.d_face_corner, h.d_groups, h.d_status + 2);
     h.launches++;
     PB_CHECK_LAUNCH();
     return PPPM_OK;

@@ -17,8 +17,12 @@
 //             the grid slot the next stencil writes.  One pass over the pair list per step
 //             instead of two; no copy of the field into a separate far-field grid.
 //
-// Inside a convolution a warp handles two pairs at a time, one lane per tap, so weights
-// (fp16 pairs) and history (16 consecutive ring slots) are read as coalesced 64-byte runs;
+// Recorded calls go in passes of several steps (kPass): the face pairs' and the grid-cache records
+// are streamed once for up to four steps, and the products with the pass's own Dirichlet values
+// are added as those become known (conv_groups + face_fix, near_terms4 + near_terms_complete).
+//
+// Inside a convolution a quad of lanes handles a pair, four taps a lane, so weights (fp16 pairs) and
+// history (16 consecutive slots) are read as 16- and 32-byte vectors;
 // partial sums stay in registers and are reduced once per triangle / cell.  No atomics.
 #include <algorithm>
 #include "fdtd.cuh"
@@ -68,6 +72,13 @@ struct StepArgs
     int *status;  // the handle's step status word: kStepNonFinite once a listener sample is not finite
 };
 
+// pairs (capacity of the lists) from which the completion of the convolution goes by groups of centres
+constexpr long long kManyPairs = 1500000;
+
+// Steps of a recorded call go in passes that stream the face pairs and the grid-cache records once
+// for several steps: four while a further step of the call follows, then pairs, then one.
+constexpr int kPass = 4;
+
 // bit of the step status word: a non-finite Dirichlet value or listener sample appeared
 constexpr int kStepNonFinite = 1;
 
@@ -86,10 +97,11 @@ __device__ inline void flag_nonfinite(int *status, R v)
 // reference's ring holds it).  The taps are read from four copies of 16 slots instead: copy c
 // holds time tau at slot (c - tau) mod 16, so taps 4q..4q+3 of time t sit at slots
 // (c - t + 4q) .. +3 of copy c, ascending with the tap, and for c = t mod 4 they start on a
-// multiple of 4.  A copy's row interleaves the two fields by 4-tap chunks: chunk j holds Neumann
-// slots 4j..4j+3 then Dirichlet slots 4j..4j+3, so the Neumann and Dirichlet taps 4q..4q+3 of a
-// triangle are one aligned 32-byte load (FP32) and a triangle's whole window is one 128-byte
-// line.  A new value is written into all four copies and the canonical ring.
+// multiple of 4.  A copy's row holds (Neumann, Dirichlet) pairs, slot by slot: taps 4q..4q+3 of a
+// triangle are one aligned 32-byte load (FP32) of four pairs, each in the register pair that a
+// packed multiply-add takes against a tap's (single, double) weights, and a triangle's whole
+// window is one 128-byte line.  A new value is written into all four copies and the canonical
+// ring.
 __host__ __device__ inline int hist_index(int copy, int time) { return (copy - time) & (kHist - 1); }
 
 // the three grid time levels (and PML fields) by time index, the history copies
@@ -106,7 +118,7 @@ struct Ring
     __device__ R *pml(int time) const { return p[((time % 3) + 3) % 3]; }
     __device__ R *hrow(int copy, int tri) const { return hist + ((long long)copy * nt + tri) * kHistRow; }
     // position of slot s of a field inside a copy's row
-    __device__ static int hpos(int field, int s) { return ((s >> 2) << 3) + (field << 2) + (s & 3); }
+    __device__ static int hpos(int field, int s) { return 2 * s + field; }
     __device__ R &hat(int field, int copy, int tri, int s) const { return hrow(copy, tri)[hpos(field, s)]; }
     __device__ R &canon_at(int field, int tri, int time) const
     {
@@ -128,7 +140,7 @@ struct Ring
     // N[time + 1] of triangle tri into the Dirichlet slot of `time` in copy time mod 4: that slot
     // is tap 0 of the Dirichlet window of `time` (the step's unknown, which no reader of the
     // window uses; finish of that step overwrites it with D[time]), so a two-step pass over the
-    // face pairs at `time` receives N[time + 1] with the window (face_conv2).  acc_next: the
+    // face pairs at `time` receives N[time + 1] with the window (group_conv).  acc_next: the
     // acceleration row of time + 1, or none.
     __device__ void stash_next(int tri, int time, const float *acc_next) const
     {
@@ -558,20 +570,25 @@ __global__ void __launch_bounds__(256) pml_kernel(const __grid_constant__ StepAr
 
 // ---- convolution helpers
 // A pair is handled by a quad of 4 lanes: lane q takes taps 4q..4q+3 with one 16-byte load of
-// the pair's weights (4 fp16 (single, double) tap pairs) and one load of the neighbour's Neumann
-// and Dirichlet taps 4q..4q+3 from the history copy in which they are aligned at this time step
-// (load_window); the 8 quads of a warp take pairs g, g + 8, ...  Each lane sums its
+// the pair's weights (4 fp16 (single, double) tap pairs) and one load of the neighbour's
+// (Neumann, Dirichlet) taps 4q..4q+3 from the history copy in which they are aligned at this time
+// step (load_window); the 8 quads of a warp take pairs g, g + 8, ...  Each lane sums its
 // taps in increasing pair and tap order; the warp reduces once per triangle / cell.
-__device__ inline float conv_tap(__half2 w, float2 s, float n, float d)
-{
-    return -__low2float(w) * s.x * n + __high2float(w) * s.y * d;
-}
-__device__ inline double conv_tap(double2 w, float2, double n, double d) { return -w.x * n + w.y * d; }
-
+// The FP32 sums run two layers wide: fma.rn.f32x2 multiplies a tap's (single, double) weights by
+// its (N, D) values, so a tap costs two conversions and one multiply-add, and a record's two sums
+// meet its scales (-single, double) once.  Measured on the convolution and the near-field terms at
+// 6400 triangles, where both were bound by instruction issue: see conv_groups and near_terms2.
 template <typename T, int N>
 struct alignas(16) Vec
 {
     T v[N];
+};
+
+// A pair of floats in one 64-bit register pair, the operand of the packed instructions (kept packed
+// throughout: taken apart and put together again it costs a move per half)
+struct F32x2
+{
+    unsigned long long v;
 };
 
 template <typename R>
@@ -581,34 +598,134 @@ struct WRec<float>
 {
     using T = __half2;
     using W4 = Vec<__half2, 4>;
-    using H4 = Vec<float, 4>;
+    using P = F32x2;
 };
 template <>
 struct WRec<double>
 {
     using T = double2;
     using W4 = Vec<double2, 4>;
-    using H4 = Vec<double, 4>;
+    using P = double2;
 };
 
-// Taps 4q..4q+3 of time t of both fields of one triangle: chunk (slot of tap 0) / 4 + q of copy
+__device__ inline F32x2 make_pair2(float x, float y)
+{
+    F32x2 p;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(p.v) : "f"(x), "f"(y));
+    return p;
+}
+__device__ inline float2 halves(F32x2 p)
+{
+    float2 f;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(p.v));
+    return f;
+}
+__device__ inline double2 make_pair2(double x, double y) { return make_double2(x, y); }
+__device__ inline double2 halves(double2 p) { return p; }
+template <typename P>
+__device__ inline auto pair_sum(P p)
+{
+    const auto f = halves(p);
+    return f.x + f.y;
+}
+// p with its second half replaced
+template <typename P, typename R>
+__device__ inline P with_y(P p, R y)
+{
+    return make_pair2(halves(p).x, y);
+}
+
+// component-wise a * b + c, a * b of (single, double) pairs
+__device__ inline F32x2 fma2(F32x2 a, F32x2 b, F32x2 c)
+{
+    F32x2 d;
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(d.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return d;
+}
+__device__ inline double2 fma2(double2 a, double2 b, double2 c)
+{
+    return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));
+}
+__device__ inline F32x2 mul2(F32x2 a, F32x2 b)
+{
+    F32x2 d;
+    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
+    return d;
+}
+__device__ inline double2 mul2(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
+
+__device__ inline F32x2 weight_pair(__half2 w)
+{
+    const float2 f = __half22float2(w);
+    return make_pair2(f.x, f.y);
+}
+__device__ inline double2 weight_pair(double2 w) { return w; }
+
+// the factors that a record's (single, double) sums enter the convolution with
+__device__ inline F32x2 record_scale(const float2 *scale, long long i, float)
+{
+    const float2 s = scale[i];
+    return make_pair2(-s.x, s.y);
+}
+__device__ inline double2 record_scale(const float2 *, long long, double) { return make_double2(-1.0, 1.0); }
+
+// sum over 4 taps of weights times history, both layers
+template <typename R>
+__device__ inline typename WRec<R>::P dot4(const typename WRec<R>::P (&w)[4], const typename WRec<R>::P (&h)[4])
+{
+    typename WRec<R>::P a = mul2(w[0], h[0]);
+#pragma unroll
+    for (int i = 1; i < 4; i++)
+        a = fma2(w[i], h[i], a);
+    return a;
+}
+
+// Taps 4q..4q+3 of time t of one triangle, (N, D) pairs: chunk (slot of tap 0) / 4 + q of copy
 // t mod 4, which starts 8 values into the row per chunk.  FP32: one 32-byte load (PTX
-// ld.global.v8.f32, sm_100), so a quad reads a triangle's two windows as one 128-byte line.  The
+// ld.global.v4.b64, sm_100), so a quad reads a triangle's two windows as one 128-byte line.  The
 // asm is ordered against the kernel's own history writes (memory clobber).
 __device__ inline int window_offset(int t, int q) { return (((hist_index(t & 3, t) >> 2) + q) & 3) << 3; }
 
-__device__ inline void load_window(const float *p, Vec<float, 4> &n, Vec<float, 4> &d)
+// the same load in kernels that write no history (not ordered against other accesses)
+__device__ inline void load_window_const(const float *p, F32x2 (&h)[4])
 {
-    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=f"(n.v[0]), "=f"(n.v[1]), "=f"(n.v[2]), "=f"(n.v[3]), "=f"(d.v[0]), "=f"(d.v[1]), "=f"(d.v[2]),
-                   "=f"(d.v[3])
+    asm("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];"
+        : "=l"(h[0].v), "=l"(h[1].v), "=l"(h[2].v), "=l"(h[3].v)
+        : "l"(p));
+}
+__device__ inline void load_window(const float *p, F32x2 (&h)[4])
+{
+    asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];"
+                 : "=l"(h[0].v), "=l"(h[1].v), "=l"(h[2].v), "=l"(h[3].v)
                  : "l"(p)
                  : "memory");
 }
-__device__ inline void load_window(const double *p, Vec<double, 4> &n, Vec<double, 4> &d)
+__device__ inline void load_window(const double *p, double2 (&h)[4])
 {
-    n = *(const Vec<double, 4> *)p;
-    d = *(const Vec<double, 4> *)(p + 4);
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        h[i] = ((const double2 *)p)[i];
+}
+
+__device__ inline void load_window_const(const double *p, double2 (&h)[4]) { load_window(p, h); }
+
+// four consecutive values (16-byte aligned, 32 for FP64)
+__device__ inline void load_four(const float *p, float (&v)[4])
+{
+    const float4 x = *(const float4 *)p;
+    v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+}
+__device__ inline void load_four(const double *p, double (&v)[4])
+{
+    const double2 x = ((const double2 *)p)[0], y = ((const double2 *)p)[1];
+    v[0] = x.x, v[1] = x.y, v[2] = y.x, v[3] = y.y;
+}
+
+// the lane before it in the quad: pair v of lane q - 1 (lane 0 of the quad keeps its own)
+__device__ inline F32x2 shfl_up_quad(unsigned quad, F32x2 v) { return F32x2{__shfl_up_sync(quad, v.v, 1, 4)}; }
+__device__ inline double2 shfl_up_quad(unsigned quad, double2 v)
+{
+    return make_double2(__shfl_up_sync(quad, v.x, 1, 4), __shfl_up_sync(quad, v.y, 1, 4));
 }
 
 constexpr unsigned kFull = 0xffffffffu;
@@ -622,6 +739,35 @@ __device__ inline R warp_sum(R v)
     return v;
 }
 
+// V sums over the warp at once (V a power of two, at most 32): each exchange halves the values a
+// lane holds, so all V cost V - 1 + log2(32 / V) exchanges.  Lane l ends with the total of value
+// l >> (5 - log2 V) in v[0].
+template <typename R, int V>
+__device__ inline void warp_sums(R (&v)[V], int lane)
+{
+    int off = 16;
+#pragma unroll
+    for (int half = V / 2; half > 0; half /= 2, off >>= 1)
+    {
+        const bool up = (lane & off) != 0;
+#pragma unroll
+        for (int i = 0; i < half; i++)
+        {
+            const R send = up ? v[i] : v[i + half], keep = up ? v[i + half] : v[i];
+            v[i] = keep + __shfl_xor_sync(kFull, send, off);
+        }
+    }
+    for (; off > 0; off >>= 1)
+        v[0] += __shfl_xor_sync(kFull, v[0], off);
+}
+
+// Centres that share a base cell have the same 4^3 neighbour list in the same order.  A group is up
+// to kGroup of them (mesh.cu: face_fill_kernel): their triangles, where each one's records start,
+// the common list length.
+constexpr int kGroupSplit = 2;  // warps that share a group's list, in turn by chunks of kChunk neighbours
+constexpr int kChunk = 16;
+constexpr int kConvThreads = 32 * kGroupSplit;  // a block of the convolution kernels takes one group at a time
+
 // face stage: one warp per centre triangle.  The 8 far-field corner terms are fetched first
 // (lanes 0-7) so their latency overlaps the convolution.
 // the face-stage work of one scene's centre triangle tri (whole warp)
@@ -631,18 +777,24 @@ struct FaceArgs
     const int *face_start, *face_nbr, *face_corner;
     const typename WRec<R>::T *face_w;
     const float2 *face_scale;
-    const R *face_d1;  // per pair: double-layer tap 1 with its scale (fix_kernel)
-    const int *order;  // centre triangles in base-cell order (the convolution kernels' warp order)
-    R *dlast;          // per triangle: the Dirichlet value of the last finished step
+    const R *face_d[kPass - 1];  // per pair: double-layer taps 1, 2, 3 with their scale (face_fix)
+    const int *order;  // centre triangles in base-cell order (the completion kernel's warp order)
+    const CentreGroup *groups;  // centres that share a neighbour list (conv_groups)
+    const int *ngroups;
+    R *dlast;          // [nt][4]: the Dirichlet values of the last steps, by step of the call mod 4
+    R *nfut;           // [nt][4]: N[t+1], N[t+2], N[t+3] of a four-step pass that starts at t
     const float *interp;
     const double *interp_d, *denom;
     float reflect;
     // near-field terms of every triangle (see near_terms): its 54 grid-cache records
     const typename WRec<R>::T *gc_w;
     const float2 *gc_scale;
-    R *terms;  // [nt][54]
-    R *terms1;        // [nt][54] partial terms of the next step (near_terms2)
-    const R *gc_f;    // [nt][54] factor of the next step's Dirichlet value per record (near_terms2)
+    R *terms;  // [nt][27 offsets][FDTD-near, BEM-near]
+    // the same, one array per following step of a pass: partial terms, without the products with
+    // Dirichlet values that the pass cannot know yet (near_terms2, near_terms4)
+    R *part[kPass - 1];
+    // the same, one array per age m of the missing value: factor of D[t-m] in the term of time t
+    const R *gc_f[kPass - 1];
     int *status;      // step status word (kStepNonFinite)
 };
 
@@ -650,58 +802,54 @@ constexpr int kGcRecords = 54;  // per triangle: 27 FDTD-near then 27 BEM-near r
 
 // The near-field terms of one triangle at time t (whole warp): for each of its 54 grid-cache
 // records (27 offsets x {FDTD-near, BEM-near}) the record's convolution with the triangle's OWN
-// history window, terms[tri][r].  A corrected cell's two sums are then plain sums of these terms
-// over its 3^3 list (near_gather_body): each triangle's history is read once per step instead of
-// once per corrected cell around it, and the records stream contiguously.  The FDTD-near terms
-// belong to the next step: record tap k + 1 pairs with history tap k (taps t..t-14).  Lane q of
-// quad g takes taps 4q..4q+3 of records g, g + 8, ...; d0 != 0 replaces Dirichlet tap 0 (time t)
-// with dnew, the value this warp has just computed.
+// history window, terms[tri][offset][FDTD-near, BEM-near].  A corrected cell's two sums are then
+// plain sums of these terms over its 3^3 list (near_body): each triangle's history is read once per
+// step instead of once per corrected cell around it, and the records stream contiguously.  The
+// FDTD-near terms belong to the next step: record tap k + 1 pairs with history tap k (taps
+// t..t-14).  Lane q of quad g takes taps 4q..4q+3 of both records of offsets g, g + 8, ...;
+// d0 != 0 replaces Dirichlet tap 0 (time t) with dnew, the value this warp has just computed.
 template <typename R>
 __device__ inline void near_terms(const Ring<R> &ring, int t, const FaceArgs<R> &f, int tri, int lane, bool d0,
                                   R dnew)
 {
     using W4 = typename WRec<R>::W4;
-    using H4 = typename WRec<R>::H4;
+    using P = typename WRec<R>::P;
     const int g = lane >> 2, q = lane & 3;
-    H4 hn, hd;
-    load_window(ring.hrow(t & 3, tri) + window_offset(t, q), hn, hd);
+    const unsigned quad = 0xfu << (lane & ~3);
+    P h[4], s[4];
+    load_window(ring.hrow(t & 3, tri) + window_offset(t, q), h);
     if (d0 && q == 0)
-        hd.v[0] = dnew;
+        h[0] = with_y(h[0], dnew);
     // history taps 4q-1 .. 4q+2 for the shifted FDTD-near records (tap -1 does not exist: 0)
-    H4 sn, sd;
-    const R pn = __shfl_up_sync(kFull, hn.v[3], 1), pd = __shfl_up_sync(kFull, hd.v[3], 1);
-    sn.v[0] = q ? pn : (R)0;
-    sd.v[0] = q ? pd : (R)0;
+    const P before = shfl_up_quad(quad, h[3]);
+    s[0] = q ? before : make_pair2((R)0, (R)0);
 #pragma unroll
     for (int i = 1; i < 4; i++)
-    {
-        sn.v[i] = hn.v[i - 1];
-        sd.v[i] = hd.v[i - 1];
-    }
-    const unsigned quad = 0xfu << (lane & ~3);
+        s[i] = h[i - 1];
     const typename WRec<R>::T *rec = f.gc_w + (long long)tri * kGcRecords * kTaps;
     R *out = f.terms + (long long)tri * kGcRecords;
-    for (int r = g; r < kGcRecords; r += 8)
+    constexpr int half = kGcRecords / 2;
+    for (int o = g; o < half; o += 8)
     {
-        const W4 w = *(const W4 *)(rec + (long long)r * kTaps + 4 * q);
-        const float2 s = f.gc_scale ? f.gc_scale[(long long)tri * kGcRecords + r] : make_float2(1, 1);
-        R v = 0;
-        if (r < kGcRecords / 2)
+        R v[2];
+#pragma unroll
+        for (int b = 0; b < 2; b++)
         {
+            const int r = o + b * half;
+            const W4 w4 = *(const W4 *)(rec + (long long)r * kTaps + 4 * q);
+            const P sc = record_scale(f.gc_scale, (long long)tri * kGcRecords + r, (R)0);
+            P w[4];
 #pragma unroll
             for (int i = 0; i < 4; i++)
-                v += conv_tap(w.v[i], s, sn.v[i], sd.v[i]);
+                w[i] = weight_pair(w4.v[i]);
+            v[b] = pair_sum(mul2(dot4<R>(w, b ? h : s), sc));
         }
-        else
-        {
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-                v += conv_tap(w.v[i], s, hn.v[i], hd.v[i]);
-        }
-        v += __shfl_xor_sync(quad, v, 1);
-        v += __shfl_xor_sync(quad, v, 2);
-        if (q == 0)
-            out[r] = v;
+        // lanes 0 and 1 of the quad end with the FDTD-near sum, lanes 2 and 3 with the BEM-near sum
+        const R keep = q & 2 ? v[1] : v[0], send = q & 2 ? v[0] : v[1];
+        R x = keep + __shfl_xor_sync(quad, send, 2);
+        x += __shfl_xor_sync(quad, x, 1);
+        if (!(q & 1))
+            out[2 * o + (q >> 1)] = x;
     }
 }
 
@@ -712,89 +860,163 @@ __device__ inline void near_terms(const Ring<R> &ring, int t, const FaceArgs<R> 
 // History tap j of time t+1 is tap j-1 of time t, so the time-(t+1) windows are the time-t window
 // shifted by one and two taps (quad shuffles); tap -1 is N[t+1] = nnext (known: the acceleration
 // row of the next step) and D[t+1] (left out).  face_finish of the next step adds
-// gc_f[r] * D[t+1] to terms1[r] (gc_factors holds those factors).
+// gc_f[0][r] * D[t+1] to part[0][r] (gc_factors holds those factors).
+// Both records of an offset go together: their four sums (two records, two steps) meet in one
+// quad transpose, after which each lane holds and stores one of them.
 template <typename R>
 __device__ inline void near_terms2(const Ring<R> &ring, int t, const FaceArgs<R> &f, int tri, int lane, R dnew,
                                    R nnext)
 {
     using W4 = typename WRec<R>::W4;
-    using H4 = typename WRec<R>::H4;
+    using P = typename WRec<R>::P;
     const int g = lane >> 2, q = lane & 3;
-    H4 hn, hd;
-    load_window(ring.hrow(t & 3, tri) + window_offset(t, q), hn, hd);
+    const unsigned quad = 0xfu << (lane & ~3);
+    P h[4], s[4], b1[4], s2[4];
+    load_window(ring.hrow(t & 3, tri) + window_offset(t, q), h);
     if (q == 0)
-        hd.v[0] = dnew;
-    // time-t taps shifted by one (4q+i-1) and by two (4q+i-2)
-    const R pn3 = __shfl_up_sync(kFull, hn.v[3], 1), pd3 = __shfl_up_sync(kFull, hd.v[3], 1);
-    const R pn2 = __shfl_up_sync(kFull, hn.v[2], 1), pd2 = __shfl_up_sync(kFull, hd.v[2], 1);
-    H4 sn, sd, bn, tn, td;
-    sn.v[0] = q ? pn3 : (R)0;   // FDTD-near, time t: tap -1 does not exist
-    bn.v[0] = q ? pn3 : nnext;  // BEM-near, time t+1: tap 0 of t+1 is N[t+1]
-    sd.v[0] = q ? pd3 : (R)0;   // D: tap -1 is D[t+1], left out in both
+        h[0] = with_y(h[0], dnew);
+    // taps 4q-1 and 4q-2 of time t; tap -1 does not exist at time t, at time t+1 it is (N[t+1], the
+    // unknown)
+    const P zero = make_pair2((R)0, (R)0), next = make_pair2(nnext, (R)0);
+    const P p3 = shfl_up_quad(quad, h[3]), p2 = shfl_up_quad(quad, h[2]);
+    s[0] = q ? p3 : zero;    // FDTD-near, time t
+    b1[0] = q ? p3 : next;   // BEM-near, time t+1
+    s2[0] = q ? p2 : zero;   // FDTD-near, time t+1: record tap m pairs with time-t tap m-2
+    s2[1] = q ? p3 : next;
+    s2[2] = h[0];
+    s2[3] = h[1];
 #pragma unroll
     for (int i = 1; i < 4; i++)
-    {
-        sn.v[i] = hn.v[i - 1];
-        bn.v[i] = hn.v[i - 1];
-        sd.v[i] = hd.v[i - 1];
-    }
-    // FDTD-near, time t+1: record tap m pairs with time-t tap m-2; m = 0 has no term, m = 1 meets
-    // time t+1 (N[t+1] included, D[t+1] left out)
-    tn.v[0] = q ? pn2 : (R)0;
-    td.v[0] = q ? pd2 : (R)0;
-    tn.v[1] = q ? pn3 : nnext;
-    td.v[1] = q ? pd3 : (R)0;
-    tn.v[2] = hn.v[0];
-    td.v[2] = hd.v[0];
-    tn.v[3] = hn.v[1];
-    td.v[3] = hd.v[1];
-    const unsigned quad = 0xfu << (lane & ~3);
+        s[i] = b1[i] = h[i - 1];
     const typename WRec<R>::T *rec = f.gc_w + (long long)tri * kGcRecords * kTaps;
-    R *out = f.terms + (long long)tri * kGcRecords;
-    R *out1 = f.terms1 + (long long)tri * kGcRecords;
-    for (int r = g; r < kGcRecords; r += 8)
+    R *out = (q & 1 ? f.part[0] : f.terms) + (long long)tri * kGcRecords + (q >> 1);
+    constexpr int half = kGcRecords / 2;
+    for (int o = g; o < half; o += 8)
     {
-        const W4 w = *(const W4 *)(rec + (long long)r * kTaps + 4 * q);
-        const float2 s = f.gc_scale ? f.gc_scale[(long long)tri * kGcRecords + r] : make_float2(1, 1);
-        R v = 0, v1 = 0;
-        if (r < kGcRecords / 2)
+        R v[2][2];  // [record][step]
+#pragma unroll
+        for (int b = 0; b < 2; b++)
         {
+            const int r = o + b * half;
+            const W4 w4 = *(const W4 *)(rec + (long long)r * kTaps + 4 * q);
+            const P sc = record_scale(f.gc_scale, (long long)tri * kGcRecords + r, (R)0);
+            P w[4];
 #pragma unroll
             for (int i = 0; i < 4; i++)
-            {
-                v += conv_tap(w.v[i], s, sn.v[i], sd.v[i]);
-                v1 += conv_tap(w.v[i], s, tn.v[i], td.v[i]);
-            }
+                w[i] = weight_pair(w4.v[i]);
+            v[b][0] = pair_sum(mul2(dot4<R>(w, b ? h : s), sc));
+            v[b][1] = pair_sum(mul2(dot4<R>(w, b ? b1 : s2), sc));
         }
-        else
-        {
+        // quad transpose: lane q ends with record q >> 1, step q & 1
+        R x[2];
 #pragma unroll
-            for (int i = 0; i < 4; i++)
-            {
-                v += conv_tap(w.v[i], s, hn.v[i], hd.v[i]);
-                v1 += conv_tap(w.v[i], s, bn.v[i], sd.v[i]);
-            }
-        }
-        v += __shfl_xor_sync(quad, v, 1);
-        v += __shfl_xor_sync(quad, v, 2);
-        v1 += __shfl_xor_sync(quad, v1, 1);
-        v1 += __shfl_xor_sync(quad, v1, 2);
-        if (q == 0)
+        for (int k = 0; k < 2; k++)
         {
-            out[r] = v;
-            out1[r] = v1;
+            const R keep = q & 2 ? v[1][k] : v[0][k], send = q & 2 ? v[0][k] : v[1][k];
+            x[k] = keep + __shfl_xor_sync(quad, send, 2);
         }
+        const R keep = q & 1 ? x[1] : x[0], send = q & 1 ? x[0] : x[1];
+        out[2 * o] = keep + __shfl_xor_sync(quad, send, 1);
     }
 }
 
-// the second step of a two-step pass: its near-field terms from the partial terms and the new
-// Dirichlet value
+// Four steps in one pass over the 54 records: the terms of time t (D[t] = dnew known) and the terms
+// of t+1, t+2 and t+3 without their products with D[t+1], D[t+2] and D[t+3].  Time t+k's window is
+// time t's shifted by k taps; what lies before tap 0 is (N[t+j], the unknown), N from the
+// acceleration rows.  Each of the steps t+1..t+3 adds its missing products in face_finish
+// (near_terms_complete).  The records are what the pass moves (72 B each, 54 a triangle): at
+// res 128 they stream from HBM, and four steps share one stream.
 template <typename R>
-__device__ inline void near_terms_complete(const FaceArgs<R> &f, int tri, int lane, R dnew)
+__device__ inline void near_terms4(const Ring<R> &ring, int t, const FaceArgs<R> &f, int tri, int lane, R dnew,
+                                   const R (&nnext)[kPass - 1])
 {
-    const long long o = (long long)tri * kGcRecords;
-    for (int r = lane; r < kGcRecords; r += 32)
-        f.terms[o + r] = f.terms1[o + r] + f.gc_f[o + r] * dnew;
+    using W4 = typename WRec<R>::W4;
+    using P = typename WRec<R>::P;
+    const int g = lane >> 2, q = lane & 3;
+    const unsigned quad = 0xfu << (lane & ~3);
+    P h[4];
+    load_window(ring.hrow(t & 3, tri) + window_offset(t, q), h);
+    if (q == 0)
+        h[0] = with_y(h[0], dnew);
+    // a[i] = tap 4q + i - 3 of time t (i = 0..6); z[k] = the FDTD-near partner of record tap 4q at
+    // time t+k, tap 4q - 1 - k (record tap 0 has none)
+    P a[7], z[kPass];
+    const P zero = make_pair2((R)0, (R)0);
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+    {
+        const P up = shfl_up_quad(quad, h[i + 1]);
+        a[i] = q ? up : make_pair2(nnext[2 - i], (R)0);
+        z[2 - i] = q ? up : zero;
+    }
+    {
+        const P up = shfl_up_quad(quad, h[0]);
+        z[3] = q ? up : zero;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        a[3 + i] = h[i];
+    const typename WRec<R>::T *rec = f.gc_w + (long long)tri * kGcRecords * kTaps;
+    constexpr int half = kGcRecords / 2;
+    R *out = q == 0 ? f.terms : q == 1 ? f.part[0] : q == 2 ? f.part[1] : f.part[2];
+    P *row = (P *)(out + (long long)tri * kGcRecords);
+    for (int o = g; o < half; o += 8)
+    {
+        R v[2][kPass];  // [record][step]
+#pragma unroll
+        for (int b = 0; b < 2; b++)
+        {
+            const int r = o + b * half;
+            const W4 w4 = *(const W4 *)(rec + (long long)r * kTaps + 4 * q);
+            const P sc = record_scale(f.gc_scale, (long long)tri * kGcRecords + r, (R)0);
+            P w[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                w[i] = weight_pair(w4.v[i]);
+#pragma unroll
+            for (int k = 0; k < kPass; k++)
+            {
+                // BEM-near (b = 1): tap m with tap m - k; FDTD-near: tap m with tap m - 1 - k
+                P x = mul2(w[0], b ? a[3 - k] : z[k]);
+#pragma unroll
+                for (int i = 1; i < 4; i++)
+                    x = fma2(w[i], a[2 + b + i - k], x);
+                v[b][k] = pair_sum(mul2(x, sc));
+            }
+        }
+        // quad transpose: lane q ends with both records of step q
+        R y[2];
+#pragma unroll
+        for (int b = 0; b < 2; b++)
+        {
+            R x[2];
+#pragma unroll
+            for (int k = 0; k < 2; k++)
+            {
+                const R keep = q & 2 ? v[b][k + 2] : v[b][k], send = q & 2 ? v[b][k] : v[b][k + 2];
+                x[k] = keep + __shfl_xor_sync(quad, send, 2);
+            }
+            const R keep = q & 1 ? x[1] : x[0], send = q & 1 ? x[0] : x[1];
+            y[b] = keep + __shfl_xor_sync(quad, send, 1);
+        }
+        row[o] = make_pair2(y[0], y[1]);
+    }
+}
+
+// A later step of a pass (position J = 1, 2, 3): its near-field terms from the partial terms and the
+// pass's Dirichlet values since then, d[m] = D[t-m] (d[0] = the new one).
+template <typename R, int J>
+__device__ inline void near_terms_complete(const FaceArgs<R> &f, int tri, int lane, const R (&d)[kPass - 1])
+{
+    using P = typename WRec<R>::P;
+    if (lane >= kGcRecords / 2)
+        return;
+    const long long o = (long long)tri * (kGcRecords / 2) + lane;
+    P v = ((const P *)f.part[J - 1])[o];
+#pragma unroll
+    for (int m = 0; m < J; m++)
+        v = fma2(((const P *)f.gc_f[m])[o], make_pair2(d[m], d[m]), v);
+    ((P *)f.terms)[o] = v;
 }
 
 // The face stage of centre triangle tri (whole warp) in two parts.  face_conv: the face-pair
@@ -807,79 +1029,164 @@ template <typename R>
 __device__ inline R face_conv(const Ring<R> &ring, int tnew, const FaceArgs<R> &f, int tri, int lane)
 {
     using W4 = typename WRec<R>::W4;
-    using H4 = typename WRec<R>::H4;
+    using P = typename WRec<R>::P;
     const int g = lane >> 2, q = lane & 3;
     const R *base = ring.hrow(tnew & 3, 0) + window_offset(tnew, q);
     const int b = f.face_start[tri], e = f.face_start[tri + 1];
-    R acc = 0;
+    P acc = make_pair2((R)0, (R)0);
     for (int p = b + g; p < e; p += 8)
     {
-        const W4 w = *(const W4 *)(f.face_w + (long long)p * kTaps + 4 * q);
-        const float2 s = f.face_scale ? f.face_scale[p] : make_float2(1, 1);
-        const int nb = f.face_nbr[p];
-        H4 hn, hd;
-        load_window(base + (long long)nb * kHistRow, hn, hd);
+        const W4 w4 = *(const W4 *)(f.face_w + (long long)p * kTaps + 4 * q);
+        const P sc = record_scale(f.face_scale, p, (R)0);
+        P h[4], w[4];
+        load_window(base + (long long)f.face_nbr[p] * kHistRow, h);
+        if (q == 0)
+            h[0] = with_y(h[0], (R)0);  // tap 0 of the Dirichlet history is this step's unknown: left out
 #pragma unroll
         for (int i = 0; i < 4; i++)
-        {
-            // tap 0 of the Dirichlet history is this step's unknown: left out
-            R di = (q == 0 && i == 0) ? (R)0 : hd.v[i];
-            acc += conv_tap(w.v[i], s, hn.v[i], di);
-        }
+            w[i] = weight_pair(w4.v[i]);
+        acc = fma2(dot4<R>(w, h), sc, acc);
     }
-    return warp_sum(acc);
+    return warp_sum(pair_sum(acc));
 }
 
-// Two steps from one pass over the face pairs.  c0: step k's convolution, exactly as face_conv
-// (same loads, same per-lane order).  c1: step k+1's convolution without its one term that needs
-// a value of step k: Dirichlet tap 1 of time t+1 is D[t], which finish(k) computes; fix_kernel
-// adds that term, sum_j d1_j D_j[t].  Everything else of step k+1 is final before step k:
-// Neumann taps t+1..t-14 (N[t+1] = acc[k+1], read from the acceleration row since the ring
-// receives it only in finish(k)) and Dirichlet taps t-1..t-14.  Tap 4q+i of time t+1 is tap
-// 4q+i-1 of time t, so lane q's shifted window is its own taps 4q..4q+2 plus tap 4q-1 from the
-// lane before it in the quad (tap -1: N[t+1]; for D, taps 0 and 1 of time t+1 are left out).
-// The face weights, scales and neighbour indices are read once for both steps.
-template <typename R>
-__device__ inline void face_conv2(const Ring<R> &ring, int tnew, const FaceArgs<R> &f, int tri, int lane, R &c0,
-                                  R &c1)
+// The face-pair convolution of a group of N centres that share one neighbour list, T = 1, 2 or 4
+// steps in one pass, over the list's chunks of kChunk neighbours first, first + kGroupSplit, ...  A lane
+// loads its taps of a neighbour's window once for the N centres; the records are read once for the
+// T steps.
+// Sum 0 is step k's convolution, exactly the terms of face_conv.  Sum j is step k+j's without the
+// terms that need a value the pass cannot know: Dirichlet taps 1..j of time t+j are D[t+j-1]..D[t],
+// which finish of those steps computes; face_fix adds them.  Everything else of step k+j is final
+// before step k: Neumann taps t+j..t+j-15 and Dirichlet taps t-1..t+j-15.  Tap 4q+i of time t+j is
+// tap 4q+i-j of time t, so lane q's shifted windows are its own taps after the last taps of the lane
+// before it in the quad; before tap 0 lies (N[t+1], unknown), (N[t+2], unknown), ...  The ring
+// receives those N only in finish of the steps before, so they come apart: T = 2 with the window,
+// stashed in Dirichlet tap 0 (Ring::stash_next), T = 4 from nfut.
+template <typename R, int T, int N>
+__device__ inline void group_conv(const R *window, const FaceArgs<R> &f, const CentreGroup &G, int first, int lane,
+                                  R (&out)[kGroup * T])
 {
     using W4 = typename WRec<R>::W4;
-    using H4 = typename WRec<R>::H4;
+    using P = typename WRec<R>::P;
     const int g = lane >> 2, q = lane & 3;
-    const R *base = ring.hrow(tnew & 3, 0) + window_offset(tnew, q);
     const unsigned quad = 0xfu << (lane & ~3);
-    const int b = f.face_start[tri], e = f.face_start[tri + 1];
-    R a0 = 0, a1 = 0;
-    for (int p = b + g; p < e; p += 8)
+    P tot[N][T];
+#pragma unroll
+    for (int c = 0; c < N; c++)
+#pragma unroll
+        for (int k = 0; k < T; k++)
+            tot[c][k] = make_pair2((R)0, (R)0);
+    int start[N];
+#pragma unroll
+    for (int c = 0; c < N; c++)
+        start[c] = G.start[c];
+    const int len = G.len;
+    // octet o of the warp's chunks: 8 neighbours, one a quad
+    auto place = [&](int o) { return ((o >> 1) * kGroupSplit + first) * kChunk + (o & 1) * 8 + g; };
+    int nb = place(0) < len ? f.face_nbr[start[0] + place(0)] : 0;
+    // (a quad whose place lies past the list's end in an octet has none in later ones either)
+    for (int o = 0, p = place(0); p < len; p = place(++o))
     {
-        const W4 w = *(const W4 *)(f.face_w + (long long)p * kTaps + 4 * q);
-        const float2 s = f.face_scale ? f.face_scale[p] : make_float2(1, 1);
-        const int nb = f.face_nbr[p];
-        H4 hn, hd;
-        load_window(base + (long long)nb * kHistRow, hn, hd);
-        const R nnew = hd.v[0];  // lane q = 0: N[t+1], stashed in Dirichlet tap 0 (Ring::stash_next)
-        const R un = __shfl_up_sync(quad, hn.v[3], 1, 4), ud = __shfl_up_sync(quad, hd.v[3], 1, 4);
+        P h[4], a[T + 3];  // a[i] = tap 4q + i - (T - 1) of time t
+        W4 w4[N];
+        P sc[N];
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+        for (int c = 0; c < N; c++)
         {
-            R di = (q == 0 && i == 0) ? (R)0 : hd.v[i];
-            a0 += conv_tap(w.v[i], s, hn.v[i], di);
+            const long long r = start[c] + p;
+            w4[c] = *(const W4 *)(f.face_w + r * kTaps + 4 * q);
+            sc[c] = record_scale(f.face_scale, r, (R)0);
         }
-        H4 sn, sd;
-        sn.v[0] = q ? un : nnew;
-        sd.v[0] = q ? ud : (R)0;
-        sd.v[1] = q ? hd.v[0] : (R)0;
+        load_window_const(window + (long long)nb * kHistRow, h);
+        R fut[kPass] = {0, 0, 0, 0};
+        if (T == 4 && q == 0)
+            load_four(f.nfut + (long long)nb * kPass, fut);
+        if (place(o + 1) < len)
+            nb = f.face_nbr[start[0] + place(o + 1)];
+        if constexpr (T == 2)
+            fut[0] = halves(h[0]).y;
+        if (q == 0)
+            h[0] = with_y(h[0], (R)0);  // D[t], the unknown of step k
 #pragma unroll
-        for (int i = 1; i < 4; i++)
-            sn.v[i] = hn.v[i - 1];
-        sd.v[2] = hd.v[1];
-        sd.v[3] = hd.v[2];
+        for (int i = 0; i < T - 1; i++)
+        {
+            const P up = shfl_up_quad(quad, h[5 - T + i]);
+            a[i] = q ? up : make_pair2(fut[T - 2 - i], (R)0);
+        }
 #pragma unroll
         for (int i = 0; i < 4; i++)
-            a1 += conv_tap(w.v[i], s, sn.v[i], sd.v[i]);
+            a[T - 1 + i] = h[i];
+#pragma unroll
+        for (int c = 0; c < N; c++)
+        {
+            P w[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                w[i] = weight_pair(w4[c].v[i]);
+#pragma unroll
+            for (int k = 0; k < T; k++)
+            {
+                P x = mul2(w[0], a[T - 1 - k]);
+#pragma unroll
+                for (int i = 1; i < 4; i++)
+                    x = fma2(w[i], a[T - 1 + i - k], x);
+                tot[c][k] = fma2(x, sc[c], tot[c][k]);
+            }
+        }
     }
-    c0 = warp_sum(a0);
-    c1 = warp_sum(a1);
+#pragma unroll
+    for (int c = 0; c < N; c++)
+#pragma unroll
+        for (int k = 0; k < T; k++)
+            out[c * T + k] = pair_sum(tot[c][k]);
+}
+
+// The face-pair convolution by groups of centres (block blk of nblk, kConvThreads threads): sum j of
+// triangle tri, step k+j's (partial) convolution, into conv[j * nt + tri].  kGroupSplit warps share a
+// group's list and add their sums through shared memory.
+// What bounds it: per record 64 B of weights and 8 B of scales, read once for T steps.  A window
+// gather (128 B per record, 8 lines per warp load) and an index load per record were the larger part
+// of the L1 wavefronts when every centre walked its list alone; two centres share them (more than
+// two would share more, but take registers that cost more warps than that gains: four centres,
+// 6400 triangles, conv4 13.0 against 12.2 us).  Measured, four steps against two passes over two steps
+// by the kernel before this one: res 64 (480 k pairs, in L2) 13.3 against 21.0 us, res 128 (6.0 M
+// pairs, 431 MB, from HBM) 119 against 198 us.  Weights by bulk copies into shared memory (two stages
+// a warp) were slower in both (18.7 and 150 us): the pass is then bound by its instructions.
+template <typename R, int T>
+__device__ inline void conv_groups(const Ring<R> &ring, int tnew, const FaceArgs<R> &f, int blk, int nblk, R *conv)
+{
+    constexpr int V = kGroup * T;
+    __shared__ R part[kGroupSplit][V];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int ng = *f.ngroups;
+    const R *window = ring.hrow(tnew & 3, 0) + window_offset(tnew, lane & 3);
+    for (int gi = blk; gi < ng; gi += nblk)
+    {
+        const CentreGroup &G = f.groups[gi];
+        const int n = G.n;
+        R v[V];
+#pragma unroll
+        for (int i = 0; i < V; i++)
+            v[i] = 0;
+        if (n == 2)
+            group_conv<R, T, 2>(window, f, G, warp, lane, v);
+        else
+            group_conv<R, T, 1>(window, f, G, warp, lane, v);
+        warp_sums<R, V>(v, lane);
+        if (lane % (32 / V) == 0)
+            part[warp][lane / (32 / V)] = v[0];
+        __syncthreads();
+        const int i = threadIdx.x, c = i / T, k = i % T;
+        if (i < V && c < n)
+        {
+            R sum = part[0][i];
+#pragma unroll
+            for (int w = 1; w < kGroupSplit; w++)
+                sum += part[w][i];
+            conv[(long long)k * ring.nt + G.tri[c]] = sum;
+        }
+        __syncthreads();
+    }
 }
 
 // far-field corner values of triangle tri (lanes 0-7; the others 0)
@@ -896,40 +1203,91 @@ __device__ inline void face_corners(const Ring<R> &ring, int tnew, const FaceArg
     }
 }
 
-// mode 0: one step; 1: first step of a two-step pass (nnext = N[t+1] of this triangle);
-// 2: second step of a two-step pass.  commit = false: no history / Dirichlet writes (timing)
-template <typename R>
+// mode 0: one step; 1: first step of a two-step pass; 2: its second step; 3: first step of a
+// four-step pass; 4, 5, 6: its later steps.  nnext: N[t+1], ... of the pass's later steps.  slot: the
+// step's place in the dlast rows (its index in the call mod kPass: passes never wrap).
+// commit = false: no history / Dirichlet writes (timing)
+__host__ __device__ constexpr int pass_position(int mode) { return mode == 2 ? 1 : mode > 3 ? mode - 3 : 0; }
+
+template <typename R, int mode>
 __device__ inline void face_finish(const Ring<R> &ring, int tnew, const FaceArgs<R> &f, int tri, int lane, R iw, R pv,
-                                   R conv, int mode = 0, R nnext = 0, bool commit = true)
+                                   R conv, const R (&nnext)[kPass - 1], int slot, bool commit = true)
 {
+    constexpr int pos = pass_position(mode);
+    R *dlast = f.dlast + (long long)tri * kPass;
+    // D of the pass's earlier steps, newest first
+    R d[kPass - 1] = {0, 0, 0};
+#pragma unroll
+    for (int m = 1; m < pos; m++)
+        d[m] = dlast[(slot - m) & (kPass - 1)];
     R far_sum = 0;  // corners in order 0..7
 #pragma unroll
     for (int wi = 0; wi < 8; wi++)
         far_sum += __shfl_sync(kFull, iw, wi) * __shfl_sync(kFull, pv, wi);
     R num = far_sum * (R)f.reflect + conv;
     const R dnew = (R)(num / f.denom[tri]);
+    d[0] = dnew;
     if (commit && lane < 4)
         ring.hat(1, lane, tri, hist_index(lane, tnew)) = dnew;  // lane c: copy c
-    else if (commit && lane == 4 && f.dlast)
-        f.dlast[tri] = dnew;
+    else if (commit && lane == 4)
+        dlast[slot] = dnew;
     else if (commit && lane == 5)
         flag_nonfinite(f.status, dnew);  // a NaN acceleration or field reaches D within a step or two
     else if (commit && lane == 6)
         ring.canon_at(1, tri, tnew) = dnew;
-    if (mode == 1)
-        near_terms2<R>(ring, tnew, f, tri, lane, dnew, nnext);
-    else if (mode == 2)
-        near_terms_complete<R>(f, tri, lane, dnew);
-    else
+    if constexpr (mode == 0)
         near_terms<R>(ring, tnew, f, tri, lane, true, dnew);
+    else if constexpr (mode == 1)
+        near_terms2<R>(ring, tnew, f, tri, lane, dnew, nnext[0]);
+    else if constexpr (mode == 3)
+        near_terms4<R>(ring, tnew, f, tri, lane, dnew, nnext);
+    else
+        near_terms_complete<R, pos>(f, tri, lane, d);
 }
 
-// N[t+1] of triangle tri for a two-step pass: the next step's acceleration row, or, without one,
-// the ring slot the step would read
+// N of step kstep of triangle tri ahead of time: its acceleration row, or, without one, the ring slot
+// the step would read
 template <typename R>
-__device__ inline R next_neumann(const Ring<R> &ring, const StepDyn &dn, int tri)
+__device__ inline R neumann_ahead(const Ring<R> &ring, const StepState *st, int kstep, int nt, int tri)
 {
+    const StepDyn dn = bind_step(st, kstep, nt);
     return dn.acc ? (R)dn.acc[tri] : ring.canon_at(0, tri, dn.tnew);
+}
+
+// the N values that the near-field terms of a pass starting at step kstep need ahead of time
+template <typename R, int mode>
+__device__ inline void pass_neumann(const Ring<R> &ring, const StepState *st, int kstep, int nt, int tri,
+                                    R (&n)[kPass - 1])
+{
+#pragma unroll
+    for (int j = 0; j < kPass - 1; j++)
+        n[j] = mode == 3 || (mode == 1 && j == 0) ? neumann_ahead<R>(ring, st, kstep + 1 + j, nt, tri) : (R)0;
+}
+
+// What the step after this one needs of triangle tri before its stencil (what & 1: the step is one
+// of this call's): its Neumann value kstep in the history, and, where it starts a pass, the pass's
+// later Neumann values: what & 2 two steps (Ring::stash_next), what & 4 four (nfut).
+// Lanes 0..9 of a warp.
+template <typename R>
+__device__ inline void write_neumann(const Ring<R> &ring, const StepState *st, int kstep, int nt, const FaceArgs<R> &f,
+                                     int tri, int lane, int what)
+{
+    const StepDyn dn = bind_step(st, kstep, nt);
+    if (what & 1)
+    {
+        if (lane < 5)
+        {
+            const R v = dn.acc ? (R)dn.acc[tri] : ring.canon_at(0, tri, dn.tnew);
+            if (lane < 4)
+                ring.hat(0, lane, tri, hist_index(lane, dn.tnew)) = v;
+            else
+                ring.canon_at(0, tri, dn.tnew) = v;
+        }
+    }
+    if ((what & 2) && lane == 5)
+        ring.stash_next(tri, dn.tnew, bind_step(st, kstep + 1, nt).acc);
+    if ((what & 4) && lane >= 6 && lane < 6 + kPass - 1)
+        f.nfut[(long long)tri * kPass + lane - 6] = neumann_ahead<R>(ring, st, kstep + lane - 5, nt, tri);
 }
 
 // the fused face stage (corner loads issued first so their latency overlaps the convolution)
@@ -940,82 +1298,101 @@ __device__ inline void face_body(const StepArgs &, const Ring<R> &ring, const St
     R iw, pv;
     face_corners<R>(ring, dy.tnew, f, tri, lane, iw, pv);
     const R conv = face_conv<R>(ring, dy.tnew, f, tri, lane);
-    face_finish<R>(ring, dy.tnew, f, tri, lane, iw, pv, conv);
+    const R none[kPass - 1] = {0, 0, 0};
+    face_finish<R, 0>(ring, dy.tnew, f, tri, lane, iw, pv, conv, none, 0);
 }
 
-// pipelined step: the face-pair convolution of step kstep into conv[tri]
-// Warps take the centre triangles in base-cell order: centres that share a base cell have the
-// same 4^3 neighbour list, so the warps of one block gather the same neighbours' history windows
-// and mostly hit L1.  Each centre's sum is the same whatever warp computes it.
-template <typename R>
-__device__ inline int centre_of(const FaceArgs<R> &f, int w)
+// pipelined pass: the face-pair convolution of steps kstep .. kstep + T - 1 (those after the first
+// partial, group_conv) into conv[j * nt + tri]
+// (16 blocks of 64 threads per SM, at most 64 registers, FP32: measured against 14, 12 and no bound)
+template <typename R, int T>
+__global__ void __launch_bounds__(kConvThreads, sizeof(R) == 4 ? 16 : 1) conv_kernel(const __grid_constant__ Ring<R> ring, const StepState *st,
+                                                            int kstep, const __grid_constant__ FaceArgs<R> f, R *conv)
 {
-    return f.order ? f.order[w] : w;
+    conv_groups<R, T>(ring, st->tnew0 + kstep, f, blockIdx.x, gridDim.x, conv);
 }
 
-template <typename R>
-__global__ void __launch_bounds__(256) conv_kernel(const __grid_constant__ Ring<R> ring, const StepState *st,
-                                                    int kstep, int nt, const __grid_constant__ FaceArgs<R> f, R *conv)
+// A later step of a pipelined pass (position J = 1, 2, 3): conv[J * nt + tri] += the products that its
+// pass left out, sum over the pairs of sum_m d_m D[t-m] (m = 1..J), with the D that finish of the
+// pass's steps so far has written (compact rows, small enough to stay in L1).  One warp per group of
+// centres (warps w, w + nw, ...), lanes striding over the list: a neighbour's values are gathered
+// once for the group.  slot: where D[t-J] lies in the dlast rows.
+template <typename R, int J, int N>
+__device__ inline void group_fix(const FaceArgs<R> &f, const int *starts, int len, int lane, int slot, R (&a)[kGroup])
 {
-    const int w = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (w >= nt)
-        return;
-    const int tri = centre_of(f, w);
-    const R v = face_conv<R>(ring, st->tnew0 + kstep, f, tri, threadIdx.x & 31);
-    if ((threadIdx.x & 31) == 0)
-        conv[tri] = v;
-}
-
-// pipelined step pair: the face-pair convolution of step kstep into conv[tri] and the partial
-// convolution of step kstep + 1 into conv1[tri] (face_conv2)
-template <typename R>
-__global__ void __launch_bounds__(256) conv2_kernel(const __grid_constant__ Ring<R> ring, const StepState *st,
-                                                     int kstep, int nt, const __grid_constant__ FaceArgs<R> f, R *conv,
-                                                     R *conv1)
-{
-    const int w = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (w >= nt)
-        return;
-    const int tri = centre_of(f, w);
-    R c0, c1;
-    face_conv2<R>(ring, st->tnew0 + kstep, f, tri, threadIdx.x & 31, c0, c1);
-    if ((threadIdx.x & 31) == 0)
+    int start[N];
+#pragma unroll
+    for (int c = 0; c < N; c++)
     {
-        conv[tri] = c0;
-        conv1[tri] = c1;
+        start[c] = starts[c];
+        a[c] = 0;
+    }
+    for (int p = lane; p < len; p += 32)
+    {
+        const R *row = f.dlast + (long long)f.face_nbr[start[0] + p] * kPass;
+        R w[N][J], d[kPass];
+#pragma unroll
+        for (int c = 0; c < N; c++)
+#pragma unroll
+            for (int m = 0; m < J; m++)
+                w[c][m] = f.face_d[m][start[c] + p];
+        if constexpr (J == 1)
+            d[0] = row[slot];
+        else
+            load_four(row, d);  // four-step passes start at slot 0
+#pragma unroll
+        for (int c = 0; c < N; c++)
+#pragma unroll
+            for (int m = 0; m < J; m++)
+                a[c] = fma(w[c][m], d[J - 1 - m], a[c]);
     }
 }
 
-// second step of a pipelined pair: conv[tri] = conv1[tri] + sum_j d1_j D_j[t-1], with D[t-1] the
-// Dirichlet values that finish of the step before has just written (compact per-triangle copy,
-// small enough to stay in L1), lanes striding over the pairs
-template <typename R>
-__device__ inline void face_fix(const FaceArgs<R> &f, const R *conv1, R *conv, int tri, int lane)
+template <typename R, int J>
+__device__ inline void face_fix_groups(const FaceArgs<R> &f, int nt, R *conv, int w, int nw, int lane, int slot)
 {
-    const int b = f.face_start[tri], e = f.face_start[tri + 1];
-    R a = 0;
-    for (int p = b + lane; p < e; p += 32)
-        a += f.face_d1[p] * f.dlast[f.face_nbr[p]];
-    a = warp_sum(a);
+    const int ng = *f.ngroups;
+    for (int gi = w; gi < ng; gi += nw)
+    {
+        const CentreGroup &G = f.groups[gi];
+        R a[kGroup] = {0, 0};
+        if (G.n == 2)
+            group_fix<R, J, 2>(f, G.start, G.len, lane, slot, a);
+        else
+            group_fix<R, J, 1>(f, G.start, G.len, lane, slot, a);
+        warp_sums<R, kGroup>(a, lane);
+        const int c = lane / (32 / kGroup);
+        if (lane % (32 / kGroup) == 0 && c < G.n)
+            conv[(long long)J * nt + G.tri[c]] += a[0];
+    }
+}
+
+// one warp per triangle instead: the same sums
+template <typename R, int J>
+__device__ inline void face_fix(const FaceArgs<R> &f, int nt, R *conv, int tri, int lane, int slot)
+{
+    R a[kGroup] = {0, 0};
+    const int b = f.face_start[tri];
+    group_fix<R, J, 1>(f, &b, f.face_start[tri + 1] - b, lane, slot, a);
+    a[0] = warp_sum(a[0]);
     if (lane == 0)
-        conv[tri] = conv1[tri] + a;
+        conv[(long long)J * nt + tri] += a[0];
 }
 
-template <typename R>
-__global__ void __launch_bounds__(256) fix_kernel(int nt, const __grid_constant__ FaceArgs<R> f, const R *conv1, R *conv)
+template <typename R, int J, bool groups>
+__global__ void __launch_bounds__(256) fix_kernel(int nt, const __grid_constant__ FaceArgs<R> f, R *conv, int slot)
 {
-    const int w = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (w >= nt)
-        return;
-    face_fix<R>(f, conv1, conv, centre_of(f, w), threadIdx.x & 31);
+    const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if constexpr (groups)
+        face_fix_groups<R, J>(f, nt, conv, w, (int)((gridDim.x * blockDim.x) >> 5), lane, slot);
+    else if (w < nt)
+        face_fix<R, J>(f, nt, conv, f.order[w], lane, slot);
 }
 
-// pipelined step: the rest of the face stage of step kstep; next & 1: also the Neumann value of
-// step kstep + 1 into the history (its slot is outside every window of this step), so the next
-// step's convolution can start before that step's stencil; next & 2: step kstep + 1 starts a
-// two-step pass over the face pairs, which receives N of step kstep + 2 with its history windows
-// (Ring::stash_next)
-// (one instantiation per mode: the two-step variants need more registers, which the one-step
+// pipelined step: the rest of the face stage of step kstep; next: what the following step needs of
+// this one (write_neumann), so that its convolution can start before its stencil (the slots lie
+// outside every window of this step)
+// (one instantiation per mode: the several-step variants need more registers, which the one-step
 // path should not carry)
 template <typename R, int mode>
 __global__ void __launch_bounds__(256) finish_kernel(const __grid_constant__ Ring<R> ring, const StepState *st,
@@ -1028,15 +1405,11 @@ __global__ void __launch_bounds__(256) finish_kernel(const __grid_constant__ Rin
         return;
     const int lane = threadIdx.x & 31;
     const StepDyn dy = bind_step(st, kstep, nt);
-    const StepDyn dn = bind_step(st, kstep + 1, nt);
-    R iw, pv;
+    R iw, pv, n[kPass - 1];
     face_corners<R>(ring, dy.tnew, f, tri, lane, iw, pv);
-    face_finish<R>(ring, dy.tnew, f, tri, lane, iw, pv, conv[tri], mode,
-                   mode == 1 ? next_neumann<R>(ring, dn, tri) : (R)0);
-    if ((next & 1) && lane == 0)
-        ring.nwrite(tri, dn.tnew, dn.acc);
-    else if ((next & 2) && lane == 1)
-        ring.stash_next(tri, dn.tnew, bind_step(st, kstep + 2, nt).acc);
+    pass_neumann<R, mode>(ring, st, kstep, nt, tri, n);
+    face_finish<R, mode>(ring, dy.tnew, f, tri, lane, iw, pv, conv[tri], n, kstep & (kPass - 1));
+    write_neumann<R>(ring, st, kstep + 1, nt, f, tri, lane, next);
 }
 
 // the autotuner's finish: the same work without the history and Dirichlet writes, so that timing
@@ -1052,25 +1425,28 @@ __global__ void __launch_bounds__(256) finish_dry_kernel(const __grid_constant__
         return;
     const int lane = threadIdx.x & 31;
     const StepDyn dy = bind_step(st, kstep, nt);
-    const StepDyn dn = bind_step(st, kstep + 1, nt);
-    R iw, pv;
+    R iw, pv, n[kPass - 1];
     face_corners<R>(ring, dy.tnew, f, tri, lane, iw, pv);
-    face_finish<R>(ring, dy.tnew, f, tri, lane, iw, pv, conv[tri], mode,
-                   mode == 1 ? next_neumann<R>(ring, dn, tri) : (R)0, false);
+    pass_neumann<R, mode>(ring, st, kstep, nt, tri, n);
+    face_finish<R, mode>(ring, dy.tnew, f, tri, lane, iw, pv, conv[tri], n, 0, false);
 }
 
-// the Neumann value of step kstep into the history (first step of a pipelined call); stash: the step
-// starts a two-step pass over the face pairs (Ring::stash_next)
+// the Neumann value of step kstep into the history (first step of a pipelined call); what: as
+// write_neumann
 template <typename R>
-__global__ void nwrite_kernel(const __grid_constant__ Ring<R> ring, const StepState *st, int kstep, int nt, int stash)
+__global__ void nwrite_kernel(const __grid_constant__ Ring<R> ring, const StepState *st, int kstep, int nt,
+                              const __grid_constant__ FaceArgs<R> f, int what)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const StepDyn dy = bind_step(st, kstep, nt);
     if (i < nt)
     {
         ring.nwrite(i, dy.tnew, dy.acc);
-        if (stash)
+        if (what & 2)
             ring.stash_next(i, dy.tnew, bind_step(st, kstep + 1, nt).acc);
+        if (what & 4)
+            for (int j = 0; j < kPass - 1; j++)
+                f.nfut[(long long)i * kPass + j] = neumann_ahead<R>(ring, st, kstep + 1 + j, nt, i);
     }
 }
 
@@ -1122,10 +1498,10 @@ __device__ inline void near_body(const StepArgs &a, const Ring<R> &ring, const S
         R acc_f = 0, acc_b = 0;
         for (int p = b + lane; p < e; p += 32)
         {
-            const R *t = na.terms + (long long)na.p3_tri[p] * kGcRecords + na.p3_woff[p];
-            acc_f += t[0];
-            if (!prime)
-                acc_b += t[kGcRecords / 2];
+            const auto t =
+                halves(((const typename WRec<R>::P *)na.terms)[(long long)na.p3_tri[p] * (kGcRecords / 2) + na.p3_woff[p]]);
+            acc_f += t.x;
+            acc_b += t.y;
         }
         acc_f = warp_sum(acc_f);
         if (!prime)
@@ -1208,11 +1584,12 @@ struct StepLaunch
     const unsigned *corr_mask;
     FaceArgs<R> fa;
     NearArgs<R> na;
-    R *conv;   // per-triangle convolution sums of the pipelined step
-    R *conv1;  // partial sums of the second step of a pipelined pair
-    int pairs;         // pipelined graphs convolve the face pairs for two steps per pass (conv2 + fix)
+    R *conv;   // [kPass][nt] convolution sums of a pipelined pass, by position
+    int conv_blocks;   // grid of the convolution kernels (blocks stride over the groups of centres)
+    int fix_groups;    // the completion kernels take a group of centres per warp (make_launch)
+    int pairs;         // pipelined graphs convolve the face pairs for several steps per pass
     int face_threads;  // threads per block of the pipelined face-stage kernels
-    int tpairs;        // the near-field terms two steps per pass (near_terms2)
+    int tpairs;        // the near-field terms several steps per pass
     int split;         // recorded graphs: corrected-cell stencil on the main branch, the bulk beside it
     int corr_blocks;   // grid of stencil_corr_kernel (threads stride over the corrected cells)
     int mesh, pml, pml_blocks, stencil_blocks, face_blocks, near_blocks;
@@ -1221,6 +1598,47 @@ struct StepLaunch
 };
 
 __global__ void set_state_kernel(StepState *dst, StepState v) { *dst = v; }
+
+// blocks of the convolution kernels: the number of groups is known on the device only and lies between
+// nt / kGroup and nt; meshes put two or three centres in a base cell
+__host__ __device__ inline int conv_blocks(int nt) { return nt / 2 + 1; }
+
+// The pass that step j of a call of n steps belongs to: its size (4, 2 or 1) and j's position in it.
+// Four while a step follows the pass (the call's last step computes its terms alone), then pairs.
+// many: the stage goes several steps per pass.
+struct PassAt
+{
+    int size, pos;
+};
+__host__ __device__ inline PassAt pass_at(int j, long long n, bool many)
+{
+    if (!many)
+        return PassAt{1, 0};
+    const int first = j & ~(kPass - 1);
+    if (first + (long long)kPass < n)
+        return PassAt{kPass, j - first};
+    if ((j & 1) || j + 1ll < n)
+        return PassAt{2, j & 1};
+    return PassAt{1, 0};
+}
+
+// mode of face_finish for step j of a call of n steps; the call's last step computes its terms in one
+// pass (mode 0): the FDTD-near sums it leaves for the next call are then exactly those that
+// prime() rebuilds after a state restore or a mesh update
+__host__ __device__ inline int finish_mode(int j, long long n, bool many)
+{
+    const PassAt p = pass_at(j, n, many);
+    if (p.size == 1 || j + 1ll >= n)
+        return 0;
+    return p.size == kPass ? 3 + p.pos : 1 + p.pos;
+}
+
+// what step j needs written before its convolution starts (write_neumann)
+__host__ __device__ inline int neumann_needs(int j, long long n, bool many)
+{
+    const PassAt p = pass_at(j, n, many);
+    return 1 | (p.size == 2 && p.pos == 0 ? 2 : 0) | (p.size == kPass && p.pos == 0 ? 4 : 0);
+}
 
 template <typename R>
 int make_launch(Handle &h, StepLaunch<R> &L)
@@ -1270,7 +1688,12 @@ int make_launch(Handle &h, StepLaunch<R> &L)
         L.fa.gc_scale = h.fp64 ? nullptr : h.d_gc_scale;
         L.fa.terms = (R *)h.d_terms;
         L.conv = (R *)h.d_conv;
-        L.conv1 = (R *)h.d_conv1;
+        L.conv_blocks = conv_blocks(h.nt);
+        // By group the completion shares its gathers and index loads, by triangle it has twice the
+        // warps to hide them: 480 k pairs (in L2) 5.7 us by triangle, 6.2 by group for a pass's last
+        // step; 6.0 M pairs (from memory) 31.7 and 22.0.  By the list arrays' capacity, which only
+        // grows, so that the choice does not flicker from frame to frame.  Same sums.
+        L.fix_groups = h.pf_cap >= kManyPairs ? 1 : 0;
         L.pairs = h.conv_pairs;
         L.face_threads = h.face_threads;
         L.tpairs = h.terms_pairs ? 1 : 0;
@@ -1278,11 +1701,17 @@ int make_launch(Handle &h, StepLaunch<R> &L)
         // cells with the next step's sums: only when no corrected cell neighbours a boundary-layer
         // cell whose solve reads it (mesh_build's check)
         L.split = h.split_stencil && !h.corr_near_boundary ? 1 : 0;
-        L.fa.face_d1 = (const R *)h.d_face_d1;
+        for (int m = 0; m < kPass - 1; m++)
+        {
+            L.fa.face_d[m] = (const R *)h.d_face_d + m * h.pf_cap;
+            L.fa.part[m] = (R *)h.d_part + (long long)m * h.nt * kGcRecords;
+            L.fa.gc_f[m] = (const R *)h.d_gc_f + (long long)m * h.nt * kGcRecords;
+        }
         L.fa.order = h.d_base_tris;
+        L.fa.groups = h.d_groups;
+        L.fa.ngroups = h.d_status + 2;
         L.fa.dlast = (R *)h.d_dlast;
-        L.fa.terms1 = (R *)h.d_terms1;
-        L.fa.gc_f = (const R *)h.d_gc_f;
+        L.fa.nfut = (R *)h.d_nfut;
         L.fa.status = h.d_step_status;
         L.na.n3_cell = h.d_n3_cell;
         L.na.n3_start = h.d_n3_start;
@@ -1340,8 +1769,8 @@ void launch_step(const StepLaunch<R> &L, int k, cudaStream_t s, Handle *timed)
 //   main   stencil(k) -> finish(k) -> near(k)   finish waits for conv(k) too
 // so each step's face-pair convolution (the heavy part of the face stage) runs beside the
 // previous step's near stage and this step's stencil; finish(k) also writes N[t+1] for conv(k+1).
-// With pair set, steps go in pairs (k, k+1): conv2(k) streams the face pairs once for both steps
-// and fix(k+1), after finish(k), adds the one term of step k+1 that needs D of step k.
+// With pair set, steps go in passes (pass_at): conv(k) streams the face pairs once for the pass's
+// steps and fix(k+j), after finish(k+j-1), adds the terms of step k+j that need D of steps k..k+j-1.
 // With the split stencil (L.split), the main branch computes only the corrected cells
 // (stencil_corr_kernel: the face stage and the near stage read and write nothing else) and a
 // third branch the rest of the grid:
@@ -1361,35 +1790,76 @@ __global__ void advance_state_kernel(StepState *st, int g, int nt)
 }
 
 // open: the nsteps steps are a chunk of a longer call (run_steps), so the last of them is no
-// call's last step: it pairs, computes its terms and writes the next Neumann value as any other
-// step does (nsteps is even then, so the pairs are those of the whole call); a kernel after the
-// joins moves the call's state on by nsteps for the next chunk.
+// call's last step (nsteps is a multiple of kPass then, so the passes are those of the whole
+// call); a kernel after the joins moves the call's state on by nsteps for the next chunk, whose
+// first kernel writes what its first step needs.
+// the face-pair convolution of step k, or the completion of its sum
+template <typename R>
+void launch_conv(const StepLaunch<R> &L, int k, PassAt p, cudaStream_t s)
+{
+    const int FT = L.face_threads, nt = L.a.nt, groups = L.fix_groups;
+    const int wblocks = div_up((groups ? nt / 2 + 1 : nt) * 32ll, FT), slot = p.pos == 1 ? (k - 1) & (kPass - 1) : 0;
+    auto fix = [&](auto by_group, auto by_triangle) {
+        (groups ? by_group : by_triangle)<<<wblocks, FT, 0, s>>>(nt, L.fa, L.conv, slot);
+    };
+    if (p.pos == 1)
+        fix(fix_kernel<R, 1, true>, fix_kernel<R, 1, false>);
+    else if (p.pos == 2)
+        fix(fix_kernel<R, 2, true>, fix_kernel<R, 2, false>);
+    else if (p.pos == 3)
+        fix(fix_kernel<R, 3, true>, fix_kernel<R, 3, false>);
+    else if (p.size == kPass)
+        conv_kernel<R, kPass><<<L.conv_blocks, kConvThreads, 0, s>>>(L.ring, L.st, k, L.fa, L.conv);
+    else if (p.size == 2)
+        conv_kernel<R, 2><<<L.conv_blocks, kConvThreads, 0, s>>>(L.ring, L.st, k, L.fa, L.conv);
+    else
+        conv_kernel<R, 1><<<L.conv_blocks, kConvThreads, 0, s>>>(L.ring, L.st, k, L.fa, L.conv);
+}
+
+// finish of step k in the given mode; conv_pos: where the step's convolution sum lies.  dependent:
+// as a programmatic dependent of the stream's last kernel.
+template <typename R>
+void launch_finish(const StepLaunch<R> &L, int k, int mode, int conv_pos, int next, cudaStream_t s, bool dependent)
+{
+    const int FT = L.face_threads, nt = L.a.nt, wblocks = div_up((long long)nt * 32, FT);
+    const R *conv = L.conv + (long long)conv_pos * nt;
+    auto go = [&](auto kern) {
+        if (dependent)
+            launch_dependent(kern, wblocks, FT, s, L.ring, L.st, k, nt, L.fa, conv, next);
+        else
+            kern<<<wblocks, FT, 0, s>>>(L.ring, L.st, k, nt, L.fa, conv, next);
+    };
+    switch (mode)
+    {
+    case 1: go(finish_kernel<R, 1>); break;
+    case 2: go(finish_kernel<R, 2>); break;
+    case 3: go(finish_kernel<R, 3>); break;
+    case 4: go(finish_kernel<R, 4>); break;
+    case 5: go(finish_kernel<R, 5>); break;
+    case 6: go(finish_kernel<R, 6>); break;
+    default: go(finish_kernel<R, 0>); break;
+    }
+}
+
 template <typename R>
 void capture_pipelined(Handle &h, const StepLaunch<R> &L, int nsteps, bool pair, bool open)
 {
-    const int T = 256, FT = L.face_threads;
+    const int T = 256;
     const int nt = L.a.nt;
-    const int wblocks = div_up((long long)nt * 32, FT);
     cudaStream_t s = h.stream, side = h.side, bulk = h.side2;
     const bool split = L.split && bulk;
     StencilSplit bsp = L.sp;
     bsp.skip_corrected = 1;
-    // step j's convolution is a two-step pass (conv2_kernel)
-    auto conv2_at = [&](int j) { return pair && !(j & 1) && j < nsteps && (open || j + 1 < nsteps); };
-    nwrite_kernel<R><<<div_up(nt, T), T, 0, s>>>(L.ring, L.st, 0, nt, conv2_at(0) ? 1 : 0);
+    const long long total = open ? nsteps + (1ll << 40) : nsteps;
+    nwrite_kernel<R><<<div_up(nt, T), T, 0, s>>>(L.ring, L.st, 0, nt, L.fa, neumann_needs(0, total, pair));
     cudaEventRecord(h.ev_fin, s);
     if (split)
         cudaEventRecord(h.ev_near, s);
     for (int k = 0; k < nsteps; k++)
     {
-        const bool more = open || k + 1 < nsteps;  // a later step follows in this call
+        const PassAt p = pass_at(k, total, pair);
         cudaStreamWaitEvent(side, h.ev_fin, 0);
-        if (pair && (k & 1))
-            fix_kernel<R><<<wblocks, FT, 0, side>>>(nt, L.fa, L.conv1, L.conv);
-        else if (pair && more)
-            conv2_kernel<R><<<wblocks, FT, 0, side>>>(L.ring, L.st, k, nt, L.fa, L.conv, L.conv1);
-        else
-            conv_kernel<R><<<wblocks, FT, 0, side>>>(L.ring, L.st, k, nt, L.fa, L.conv);
+        launch_conv<R>(L, k, p, side);
         cudaEventRecord(h.ev_conv, side);
         if (split)
         {
@@ -1404,18 +1874,9 @@ void capture_pipelined(Handle &h, const StepLaunch<R> &L, int nsteps, bool pair,
             // the stencil without its Neumann block range (finish / nwrite wrote N[t])
             stencil_kernel<R><<<L.sp.nb_bd + L.sp.nb_in, T, 0, s>>>(L.a, L.ring, L.st, k, L.sp, L.corr_mask);
         cudaStreamWaitEvent(s, h.ev_conv, 0);
-        // the call's last step computes its terms in one pass (mode 0): the FDTD-near sums it
-        // leaves for the next call are then exactly those that prime() rebuilds after a state
-        // restore or a mesh update
-        const int mode = L.tpairs && more ? ((k & 1) ? 2 : 1) : 0;
-        const int nx = (more ? 1 : 0) | (conv2_at(k + 1) ? 2 : 0);
-        const R *conv = L.conv;
-        if (mode == 1)
-            launch_dependent(finish_kernel<R, 1>, wblocks, FT, s, L.ring, L.st, k, nt, L.fa, conv, nx);
-        else if (mode == 2)
-            launch_dependent(finish_kernel<R, 2>, wblocks, FT, s, L.ring, L.st, k, nt, L.fa, conv, nx);
-        else
-            launch_dependent(finish_kernel<R, 0>, wblocks, FT, s, L.ring, L.st, k, nt, L.fa, conv, nx);
+        // (the last step of a graph leaves the next step's needs to the next graph's first kernel)
+        const int next = k + 1 < nsteps ? neumann_needs(k + 1, total, pair) : 0;
+        launch_finish<R>(L, k, finish_mode(k, total, L.tpairs != 0), p.pos, next, s, true);
         cudaEventRecord(h.ev_fin, s);
         launch_dependent(near_kernel<R>, L.near_blocks, T, s, L.a, L.ring, L.st, k, L.na, 0);
         if (split)
@@ -1433,7 +1894,7 @@ __global__ void empty_kernel() {}
 // Measurement mode per kernel: the kernels of Handle::kProfileSteps steps exactly as
 // capture_pipelined issues them for a call of that many steps, but serialised on the handle's
 // stream with an event record between consecutive kernels; evk_kind[i] names the kind of the
-// kernel between events i and i + 1.
+// kernel between events i and i + 1.  (A call of kProfileSteps = 4 steps goes in pairs.)
 template <typename R>
 int profile_graph(Handle &h, const StepLaunch<R> &L, cudaGraphExec_t *out)
 {
@@ -1447,8 +1908,7 @@ int profile_graph(Handle &h, const StepLaunch<R> &L, cudaGraphExec_t *out)
     if (g.exec)
         cudaGraphExecDestroy(g.exec);
     g.exec = nullptr;
-    const int T = 256, FT = L.face_threads, nt = L.a.nt, n = Handle::kProfileSteps;
-    const int wblocks = div_up((long long)nt * 32, FT);
+    const int T = 256, nt = L.a.nt, n = Handle::kProfileSteps;
     const bool pair = L.pairs != 0;
     cudaStream_t s = h.stream;
     int e = 0;
@@ -1464,28 +1924,15 @@ int profile_graph(Handle &h, const StepLaunch<R> &L, cudaGraphExec_t *out)
     };
     cudaGraph_t graph = nullptr;
     PB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    auto conv2_at = [&](int j) { return pair && !(j & 1) && j + 1 < n; };
     mark(PPPM_KERNEL_NWRITE);
-    nwrite_kernel<R><<<div_up(nt, T), T, 0, s>>>(L.ring, L.st, 0, nt, conv2_at(0) ? 1 : 0);
+    nwrite_kernel<R><<<div_up(nt, T), T, 0, s>>>(L.ring, L.st, 0, nt, L.fa, neumann_needs(0, n, pair));
     mark(PPPM_KERNEL_EMPTY);
     empty_kernel<<<1, 32, 0, s>>>();
     for (int k = 0; k < n; k++)
     {
-        if (pair && (k & 1))
-        {
-            mark(PPPM_KERNEL_FIX);
-            fix_kernel<R><<<wblocks, FT, 0, s>>>(nt, L.fa, L.conv1, L.conv);
-        }
-        else if (pair && k + 1 < n)
-        {
-            mark(PPPM_KERNEL_CONV2);
-            conv2_kernel<R><<<wblocks, FT, 0, s>>>(L.ring, L.st, k, nt, L.fa, L.conv, L.conv1);
-        }
-        else
-        {
-            mark(PPPM_KERNEL_CONV);
-            conv_kernel<R><<<wblocks, FT, 0, s>>>(L.ring, L.st, k, nt, L.fa, L.conv);
-        }
+        const PassAt p = pass_at(k, n, pair);
+        mark(p.pos ? PPPM_KERNEL_FIX : p.size > 1 ? PPPM_KERNEL_CONV2 : PPPM_KERNEL_CONV);
+        launch_conv<R>(L, k, p, s);
         if (L.split)
         {
             StencilSplit bsp = L.sp;
@@ -1500,23 +1947,9 @@ int profile_graph(Handle &h, const StepLaunch<R> &L, cudaGraphExec_t *out)
             mark(PPPM_KERNEL_STENCIL);
             stencil_kernel<R><<<L.sp.nb_bd + L.sp.nb_in, T, 0, s>>>(L.a, L.ring, L.st, k, L.sp, L.corr_mask);
         }
-        const int mode = L.tpairs && k + 1 < n ? ((k & 1) ? 2 : 1) : 0;
-        const int nx = (k + 1 < n ? 1 : 0) | (conv2_at(k + 1) ? 2 : 0);
-        if (mode == 1)
-        {
-            mark(PPPM_KERNEL_FINISH1);
-            finish_kernel<R, 1><<<wblocks, FT, 0, s>>>(L.ring, L.st, k, nt, L.fa, L.conv, nx);
-        }
-        else if (mode == 2)
-        {
-            mark(PPPM_KERNEL_FINISH2);
-            finish_kernel<R, 2><<<wblocks, FT, 0, s>>>(L.ring, L.st, k, nt, L.fa, L.conv, nx);
-        }
-        else
-        {
-            mark(PPPM_KERNEL_FINISH);
-            finish_kernel<R, 0><<<wblocks, FT, 0, s>>>(L.ring, L.st, k, nt, L.fa, L.conv, nx);
-        }
+        const int mode = finish_mode(k, n, L.tpairs != 0);
+        mark(mode == 1 ? PPPM_KERNEL_FINISH1 : mode == 2 ? PPPM_KERNEL_FINISH2 : PPPM_KERNEL_FINISH);
+        launch_finish<R>(L, k, mode, p.pos, k + 1 < n ? neumann_needs(k + 1, n, pair) : 0, s, false);
         mark(PPPM_KERNEL_NEAR);
         near_kernel<R><<<L.near_blocks, T, 0, s>>>(L.a, L.ring, L.st, k, L.na, 0);
     }
@@ -1699,12 +2132,12 @@ int run_steps(Handle &h, const float *acc_dev, int nsteps)
     }
     else if (cs == cudaStreamCaptureStatusNone && nsteps >= kGraphSteps)
     {
-        // Calls longer than G = h.graph_chunk steps (even) replay one recorded chunk of G steps
+        // Calls longer than G = h.graph_chunk steps (rounded up to whole passes) replay one recorded chunk of G steps
         // as often as it fits and then a graph of the remaining 1..G steps (with the call's
         // last-step work), so a run of frames of uneven length records a few short graphs
         // instead of one long graph per length (recording costs about 0.1 ms per step).  The
         // kernels, their order and their arguments are those of one graph of nsteps steps.
-        const int G = h.graph_chunk;
+        const int G = (h.graph_chunk + kPass - 1) / kPass * kPass;  // whole passes
         const int chunks = G > 0 && nsteps > G ? (nsteps - 1) / G : 0;
         const int rest = nsteps - chunks * G;
         const bool pipelined = L.mesh && !L.pml && h.side;
@@ -1782,13 +2215,9 @@ int autotune(Handle &h, int reps, float *us, int *best)
     PB_TRY(make_launch<R>(h, L));
     const int nt = h.nt;
     auto run = [&](int c, int which) {
-        const int FT = kTuneThreads[c % 3], nb = div_up((long long)nt * 32, FT);
-        if (c < 3)
-            conv_kernel<R><<<nb, FT, 0, s>>>(L.ring, L.st, which, nt, L.fa, L.conv);
-        else if (which == 1)
-            fix_kernel<R><<<nb, FT, 0, s>>>(nt, L.fa, L.conv1, L.conv);
-        else
-            conv2_kernel<R><<<nb, FT, 0, s>>>(L.ring, L.st, 0, nt, L.fa, L.conv, L.conv1);
+        const int FT = kTuneThreads[c % 3];
+        L.face_threads = FT;
+        launch_conv<R>(L, which, c < 3 ? PassAt{1, 0} : PassAt{2, which}, s);
     };
     constexpr int kConv = 6;
     for (int c = 0; c < kConv; c++)
@@ -2075,8 +2504,7 @@ int time_kernels(Handle &h, int reps, float *us)
     StepLaunch<R> L;
     PB_TRY(make_launch<R>(h, L));
     L.a.n_listen = 0;
-    const int T = 256, FT = L.face_threads, nt = L.a.nt;
-    const int wblocks = div_up((long long)nt * 32, FT);
+    const int T = 256;
     for (int k = 0; k < PPPM_KERNEL_KINDS; k++)
         us[k] = 0;
     auto launch = [&](int kind) {
@@ -2085,20 +2513,16 @@ int time_kernels(Handle &h, int reps, float *us)
         case PPPM_KERNEL_STENCIL:
             stencil_kernel<R><<<L.sp.nb_bd + L.sp.nb_in, T, 0, s>>>(L.a, L.ring, L.st, 0, L.sp, L.corr_mask);
             break;
-        case PPPM_KERNEL_CONV: conv_kernel<R><<<wblocks, FT, 0, s>>>(L.ring, L.st, 0, nt, L.fa, L.conv); break;
-        case PPPM_KERNEL_CONV2:
-            conv2_kernel<R><<<wblocks, FT, 0, s>>>(L.ring, L.st, 0, nt, L.fa, L.conv, L.conv1);
-            break;
-        case PPPM_KERNEL_FIX: fix_kernel<R><<<wblocks, FT, 0, s>>>(nt, L.fa, L.conv1, L.conv); break;
-        case PPPM_KERNEL_FINISH:
-            finish_kernel<R, 0><<<wblocks, FT, 0, s>>>(L.ring, L.st, 0, nt, L.fa, L.conv, 0);
-            break;
-        case PPPM_KERNEL_FINISH1:
-            finish_kernel<R, 1><<<wblocks, FT, 0, s>>>(L.ring, L.st, 0, nt, L.fa, L.conv, 0);
-            break;
-        case PPPM_KERNEL_FINISH2:
-            finish_kernel<R, 2><<<wblocks, FT, 0, s>>>(L.ring, L.st, 0, nt, L.fa, L.conv, 0);
-            break;
+        case PPPM_KERNEL_CONV: launch_conv<R>(L, 0, PassAt{1, 0}, s); break;
+        case PPPM_KERNEL_CONV2: launch_conv<R>(L, 0, PassAt{2, 0}, s); break;
+        case PPPM_KERNEL_CONV4: launch_conv<R>(L, 0, PassAt{kPass, 0}, s); break;
+        case PPPM_KERNEL_FIX: launch_conv<R>(L, 1, PassAt{2, 1}, s); break;
+        case PPPM_KERNEL_FIX4: launch_conv<R>(L, kPass - 1, PassAt{kPass, kPass - 1}, s); break;
+        case PPPM_KERNEL_FINISH: launch_finish<R>(L, 0, 0, 0, 0, s, false); break;
+        case PPPM_KERNEL_FINISH1: launch_finish<R>(L, 0, 1, 0, 0, s, false); break;
+        case PPPM_KERNEL_FINISH2: launch_finish<R>(L, 0, 2, 1, 0, s, false); break;
+        case PPPM_KERNEL_FINISH4: launch_finish<R>(L, 0, 3, 0, 0, s, false); break;
+        case PPPM_KERNEL_FINISH4C: launch_finish<R>(L, 0, 6, 3, 0, s, false); break;
         case PPPM_KERNEL_NEAR: near_kernel<R><<<L.near_blocks, T, 0, s>>>(L.a, L.ring, L.st, 0, L.na, 0); break;
         case PPPM_KERNEL_FACE: face_kernel<R><<<L.face_blocks, T, 0, s>>>(L.a, L.ring, L.st, 0, L.fa); break;
         case PPPM_KERNEL_STENCIL_BULK:
@@ -2117,7 +2541,8 @@ int time_kernels(Handle &h, int reps, float *us)
     const int kinds[] = {PPPM_KERNEL_STENCIL,      PPPM_KERNEL_CONV,         PPPM_KERNEL_CONV2,
                          PPPM_KERNEL_FIX,          PPPM_KERNEL_FINISH,       PPPM_KERNEL_FINISH1,
                          PPPM_KERNEL_FINISH2,      PPPM_KERNEL_NEAR,         PPPM_KERNEL_FACE,
-                         PPPM_KERNEL_STENCIL_BULK, PPPM_KERNEL_STENCIL_CORR};
+                         PPPM_KERNEL_STENCIL_BULK, PPPM_KERNEL_STENCIL_CORR, PPPM_KERNEL_CONV4,
+                         PPPM_KERNEL_FIX4,         PPPM_KERNEL_FINISH4,      PPPM_KERNEL_FINISH4C};
     // the near kernel also writes the FDTD-near sums of the step after next into the slot two
     // ahead, which is time t-1, a level the next step still reads: kept aside and put back
     const size_t slot_bytes = (size_t)h.n_cells * sizeof(R);
@@ -2230,8 +2655,7 @@ struct BatchScene
     FaceArgs<R> fa;
     NearArgs<R> na;
     StepState *st;
-    R *conv;         // the scene's per-triangle convolution sums (pipelined graphs)
-    R *conv1;        // partial sums of the second step of a pair (two steps per pass)
+    R *conv;         // the scene's convolution sums (pipelined graphs)
     int near_warps;  // warps of this scene's near grid
     int corr_threads;  // threads of this scene's corrected-cell stencil grid (they stride over the cells)
 };
@@ -2279,45 +2703,56 @@ __global__ void __launch_bounds__(256) batch_near_kernel(const BatchScene<R> *sc
 
 // the pipelined batch step (see capture_pipelined): face-pair convolutions, the rest of the face
 // stage, and the first step's Neumann values, over the same per-scene block maps
-// The face-pair convolution of step k of every scene, one pass per step or two steps per pass
-// (conv2_kernel / fix_kernel) as the scene's state says: a scene's steps pair up from the first
-// step of its batched run (pair0), so the pairs, and the results, are those of the same steps
-// run alone in one pppm_step call, wherever the batch's graphs and phases begin and end.
-// a scene's step of time t starts a two-step pass over the face pairs (batch_conv_kernel)
-__device__ inline bool batch_conv2_at(const StepState &st, int t)
+// The face-pair convolution of step k of every scene, or the completion of a pass's later step, as
+// the scene's state says: a scene's steps go in passes from the first step of its batched run
+// (pair0), so the passes, and the results, are those of the same steps run alone in one pppm_step
+// call, wherever the batch's graphs and phases begin and end.
+__device__ inline PassAt batch_pass(const StepState &st, int t)
 {
-    return st.pair_end >= st.pair0 && st.conv_pairs && !((t - st.pair0) & 1) && t + 1 <= st.pair_end;
+    return pass_at(t - st.pair0, st.pair_end - st.pair0 + 1, st.pair_end >= st.pair0 && st.conv_pairs);
+}
+
+// what the step of time t needs written before its convolution starts (write_neumann)
+__device__ inline int batch_needs(const StepState &st, int t)
+{
+    return neumann_needs(t - st.pair0, st.pair_end - st.pair0 + 1, st.pair_end >= st.pair0 && st.conv_pairs);
 }
 
 template <typename R>
-__global__ void __launch_bounds__(256) batch_conv_kernel(const BatchScene<R> *sc, const int2 *map, int k)
+__global__ void __launch_bounds__(kConvThreads, sizeof(R) == 4 ? 16 : 1) batch_conv_kernel(const BatchScene<R> *sc, const int2 *map, int k)
 {
     const int2 m = map[blockIdx.x];
     const BatchScene<R> &S = sc[m.x];
-    const int w = m.y * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (w >= S.a.nt)
-        return;
-    const int tri = centre_of(S.fa, w);
-    const int tnew = S.st->tnew0 + k, p0 = S.st->pair0, pe = S.st->pair_end;
-    const bool paired = pe >= p0 && S.st->conv_pairs;
-    if (paired && ((tnew - p0) & 1))
-        face_fix<R>(S.fa, S.conv1, S.conv, tri, lane);  // second step of a pair
-    else if (batch_conv2_at(*S.st, tnew))
+    const int tnew = S.st->tnew0 + k, nt = S.a.nt;
+    const PassAt p = batch_pass(*S.st, tnew);
+    if (p.pos)
     {
-        R c0, c1;
-        face_conv2<R>(S.ring, tnew, S.fa, tri, lane, c0, c1);
-        if (lane == 0)
-        {
-            S.conv[tri] = c0;
-            S.conv1[tri] = c1;
-        }
+        const int w = m.y * kGroupSplit + (int)(threadIdx.x >> 5), nw = conv_blocks(nt) * kGroupSplit;
+        const int lane = threadIdx.x & 31, slot = (tnew - 1 - S.st->pair0) & (kPass - 1);
+        if (p.pos == 1)
+            face_fix_groups<R, 1>(S.fa, nt, S.conv, w, nw, lane, slot);
+        else if (p.pos == 2)
+            face_fix_groups<R, 2>(S.fa, nt, S.conv, w, nw, lane, 0);
+        else
+            face_fix_groups<R, 3>(S.fa, nt, S.conv, w, nw, lane, 0);
     }
+    else if (p.size == kPass)
+        conv_groups<R, kPass>(S.ring, tnew, S.fa, m.y, conv_blocks(nt), S.conv);
+    else if (p.size == 2)
+        conv_groups<R, 2>(S.ring, tnew, S.fa, m.y, conv_blocks(nt), S.conv);
     else
-    {
-        const R v = face_conv<R>(S.ring, tnew, S.fa, tri, lane);
-        if (lane == 0)
-            S.conv[tri] = v;
-    }
+        conv_groups<R, 1>(S.ring, tnew, S.fa, m.y, conv_blocks(nt), S.conv);
+}
+
+template <typename R, int mode>
+__device__ inline void batch_finish_body(const BatchScene<R> &S, int k, int tri, int lane, int conv_pos)
+{
+    const StepDyn dy = bind_step(S.st, k, S.a.nt);
+    R iw, pv, n[kPass - 1];
+    face_corners<R>(S.ring, dy.tnew, S.fa, tri, lane, iw, pv);
+    pass_neumann<R, mode>(S.ring, S.st, k, S.a.nt, tri, n);
+    face_finish<R, mode>(S.ring, dy.tnew, S.fa, tri, lane, iw, pv, S.conv[(long long)conv_pos * S.a.nt + tri], n,
+                         (dy.tnew - S.st->pair0) & (kPass - 1));
 }
 
 template <typename R>
@@ -2329,19 +2764,21 @@ __global__ void __launch_bounds__(256) batch_finish_kernel(const BatchScene<R> *
     const int tri = m.y * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (tri >= S.a.nt)
         return;
-    const StepDyn dy = bind_step(S.st, k, S.a.nt);
-    const StepDyn dn = bind_step(S.st, k + 1, S.a.nt);
-    // the scene's pairing of steps (batch_conv_kernel)
-    const int p0 = S.st->pair0, pe = S.st->pair_end;
-    const int mode = pe >= p0 && S.st->terms_pairs && dy.tnew < pe ? (((dy.tnew - p0) & 1) ? 2 : 1) : 0;
-    R iw, pv;
-    face_corners<R>(S.ring, dy.tnew, S.fa, tri, lane, iw, pv);
-    face_finish<R>(S.ring, dy.tnew, S.fa, tri, lane, iw, pv, S.conv[tri], mode,
-                   mode == 1 ? next_neumann<R>(S.ring, dn, tri) : (R)0);
-    if (next && lane == 0)
-        S.ring.nwrite(tri, dn.tnew, dn.acc);
-    else if (next && lane == 1 && batch_conv2_at(*S.st, dn.tnew))
-        S.ring.stash_next(tri, dn.tnew, bind_step(S.st, k + 2, S.a.nt).acc);
+    // the scene's passes (batch_conv_kernel)
+    const StepState &st = *S.st;
+    const int t = st.tnew0 + k, conv_pos = batch_pass(st, t).pos;
+    switch (finish_mode(t - st.pair0, st.pair_end - st.pair0 + 1, st.pair_end >= st.pair0 && st.terms_pairs))
+    {
+    case 1: batch_finish_body<R, 1>(S, k, tri, lane, conv_pos); break;
+    case 2: batch_finish_body<R, 2>(S, k, tri, lane, conv_pos); break;
+    case 3: batch_finish_body<R, 3>(S, k, tri, lane, conv_pos); break;
+    case 4: batch_finish_body<R, 4>(S, k, tri, lane, conv_pos); break;
+    case 5: batch_finish_body<R, 5>(S, k, tri, lane, conv_pos); break;
+    case 6: batch_finish_body<R, 6>(S, k, tri, lane, conv_pos); break;
+    default: batch_finish_body<R, 0>(S, k, tri, lane, conv_pos); break;
+    }
+    if (next)
+        write_neumann<R>(S.ring, S.st, k + 1, S.a.nt, S.fa, tri, lane, batch_needs(st, t + 1));
 }
 
 template <typename R>
@@ -2353,9 +2790,13 @@ __global__ void batch_nwrite_kernel(const BatchScene<R> *sc, const int2 *map, in
     const StepDyn dy = bind_step(S.st, k, S.a.nt);
     if (i < S.a.nt)
     {
+        const int what = batch_needs(*S.st, dy.tnew);
         S.ring.nwrite(i, dy.tnew, dy.acc);
-        if (batch_conv2_at(*S.st, dy.tnew))
+        if (what & 2)
             S.ring.stash_next(i, dy.tnew, bind_step(S.st, k + 1, S.a.nt).acc);
+        if (what & 4)
+            for (int j = 0; j < kPass - 1; j++)
+                S.fa.nfut[(long long)i * kPass + j] = neumann_ahead<R>(S.ring, S.st, k + 1 + j, S.a.nt, i);
     }
 }
 
@@ -2386,6 +2827,7 @@ struct BatchGraph
 
 constexpr int kBatchGraphSteps = 16;  // steps per replayed graph
 constexpr int kBatchGraphs = 16;      // recorded graphs kept per batch
+constexpr int kBatchMaps = 7;
 
 struct Batch
 {
@@ -2396,15 +2838,15 @@ struct Batch
     std::vector<unsigned char> host_scenes;
     // block maps: 0 stencil (with the Neumann range), 1 face (8 triangles per block), 2 near,
     // 3 stencil without the Neumann range, 4 Neumann values (256 triangles per block), 5 the
-    // corrected-cell stencil
-    std::vector<int2> host_map[6];
+    // corrected-cell stencil, 6 the face-pair convolution
+    std::vector<int2> host_map[kBatchMaps];
     int face_threads = 256;  // block size of the face-stage kernels (the first scene's launch option)
     std::vector<StepState *> host_states;
     std::vector<int> host_nt;
     void *d_scenes = nullptr;
     size_t scenes_cap = 0;
-    int2 *d_map[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-    size_t map_cap[6] = {0, 0, 0, 0, 0, 0};
+    int2 *d_map[kBatchMaps] = {};
+    size_t map_cap[kBatchMaps] = {};
     cudaStream_t side = nullptr;                      // second branch while recording
     cudaStream_t side2 = nullptr;                     // third branch: the bulk of the stencil
     cudaEvent_t ev_fin = nullptr, ev_conv = nullptr;  // fork / join points while recording
@@ -2463,7 +2905,6 @@ int batch_tables(Batch &b, const std::vector<int> &active)
         S.na = L.na;
         S.st = h.d_state;
         S.conv = L.conv;
-        S.conv1 = L.conv1;
         // near-stage warps stride over the scene's corrected cells (their count is read on the
         // device), so the block map may exceed it: it grows with headroom and never shrinks, so a
         // moving scene, whose count changes at every update_mesh, keeps its recorded batch graphs
@@ -2486,6 +2927,8 @@ int batch_tables(Batch &b, const std::vector<int> &active)
             b.host_map[4].push_back(make_int2((int)ai, k));
         for (int k = 0; k < corr_blocks; k++)
             b.host_map[5].push_back(make_int2((int)ai, k));
+        for (int k = 0; k < L.conv_blocks; k++)
+            b.host_map[6].push_back(make_int2((int)ai, k));
         b.host_states[ai] = h.d_state;
         b.host_nt[ai] = h.nt;
     }
@@ -2493,7 +2936,7 @@ int batch_tables(Batch &b, const std::vector<int> &active)
     PB_TRY(grow((unsigned char **)&ds, b.scenes_cap, b.host_scenes.size()));
     b.d_scenes = ds;
     PB_CUDA(cudaMemcpyAsync(b.d_scenes, b.host_scenes.data(), b.host_scenes.size(), cudaMemcpyHostToDevice, b.stream));
-    for (int i = 0; i < 6; i++)
+    for (int i = 0; i < kBatchMaps; i++)
     {
         PB_TRY(grow(&b.d_map[i], b.map_cap[i], b.host_map[i].size()));
         PB_CUDA(cudaMemcpyAsync(b.d_map[i], b.host_map[i].data(), b.host_map[i].size() * sizeof(int2),
@@ -2513,9 +2956,9 @@ int batch_graph(Batch &b, int g, int nactive, cudaGraphExec_t *out)
 {
     std::vector<unsigned char> sig(b.host_scenes);
     const void *ptrs[] = {b.d_scenes, b.d_map[0], b.d_map[1], b.d_map[2], b.d_map[3], b.d_map[4], b.d_map[5],
-                          b.d_states, b.d_nt};
+                          b.d_map[6], b.d_states, b.d_nt};
     const size_t sizes[] = {b.host_map[0].size(), b.host_map[1].size(), b.host_map[2].size(), b.host_map[3].size(),
-                            b.host_map[4].size(), b.host_map[5].size(), (size_t)g, (size_t)nactive,
+                            b.host_map[4].size(), b.host_map[5].size(), b.host_map[6].size(), (size_t)g, (size_t)nactive,
                             (size_t)b.face_threads, (size_t)b.split};
     sig.insert(sig.end(), (const unsigned char *)ptrs, (const unsigned char *)ptrs + sizeof(ptrs));
     sig.insert(sig.end(), (const unsigned char *)sizes, (const unsigned char *)sizes + sizeof(sizes));
@@ -2536,7 +2979,7 @@ int batch_graph(Batch &b, int g, int nactive, cudaGraphExec_t *out)
     const int n3 = (int)b.host_map[3].size(), n4 = (int)b.host_map[4].size();
     const int FT = b.face_threads;
     PB_CUDA(cudaStreamBeginCapture(b.stream, cudaStreamCaptureModeThreadLocal));
-    const int n5 = (int)b.host_map[5].size();
+    const int n5 = (int)b.host_map[5].size(), n6 = (int)b.host_map[6].size();
     if (n1 > 0 && n4 > 0 && b.side && b.side2)
     {
         // the branches of one scene's recorded steps (capture_pipelined): each step's face-pair
@@ -2551,7 +2994,7 @@ int batch_graph(Batch &b, int g, int nactive, cudaGraphExec_t *out)
         for (int k = 0; k < g; k++)
         {
             cudaStreamWaitEvent(b.side, b.ev_fin, 0);
-            batch_conv_kernel<R><<<n1, FT, 0, b.side>>>(sc, m1, k);
+            batch_conv_kernel<R><<<n6, kConvThreads, 0, b.side>>>(sc, b.d_map[6], k);
             cudaEventRecord(b.ev_conv, b.side);
             if (b.split)
             {

@@ -524,7 +524,7 @@ class Solver:
 
     def set_option(self, name, value):
         """Launch option of the recorded step graphs (pppm_set_option): conv_pairs (0: one pass
-        per step, 1: two steps per pass), face_threads (64/128/256), terms_pairs (0/1),
+        per step, 1: several steps per pass), face_threads (64/128/256), terms_pairs (0/1),
         split_stencil (0/1), graph_chunk (steps per chunk graph of a long call; 0: one graph),
         stencil_vec4 (1: four interior cells per thread, 0: one, -1: by grid size)."""
         check(lib.pppm_set_option(self.h, self.OPTIONS[name], int(value)), "set_option")
@@ -556,7 +556,7 @@ class Solver:
         check(lib.pppm_enable_timing(self.h, 1 if on else 0), "enable_timing")
 
     KERNEL_KINDS = ("stencil", "conv", "conv2", "fix", "finish", "finish1", "finish2", "near", "nwrite", "face",
-                    "empty", "stencil_bulk", "stencil_corr")
+                    "empty", "stencil_bulk", "stencil_corr", "conv4", "fix4", "finish4", "finish4c")
 
     def kernel_profile(self):
         """{kind: (mean us per launch, launches)} of the kernels timed in measurement mode

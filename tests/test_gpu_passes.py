@@ -1,0 +1,65 @@
+"""Passes over several steps (four, two or one: step.cu pass_at) against one pass per step, FP64.
+
+The passes sum the same products; those with Dirichlet values of the pass's own steps are added
+after the rest.  Bound: FP64 sums of a few hundred products in another order, amplified over at most
+a hundred steps by less than 1e3 (measured 1e-15 over 64 steps), so 1e-12 relative L2.
+"""
+import numpy as np
+import pytest
+
+from helpers import rel_l2, sine_acc, sphere_small
+from pppm_b200 import Solver, scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(geom, many, calls, chunk=32):
+    v, f, h, mn, dt, res, cell = geom
+    s = Solver(res, h, dt, mn, precision="fp64")
+    s.set_option("conv_pairs", many[0])
+    s.set_option("terms_pairs", many[1])
+    s.set_option("graph_chunk", chunk)
+    s.set_mesh(v, f)
+    s.add_listener(*cell)
+    acc = sine_acc(sum(calls), len(f), 1500.0, dt)
+    # a triangle-dependent factor, so that no two neighbours' values are interchangeable
+    acc = (acc * (1 + 0.1 * np.sin(np.arange(len(f))))).astype(np.float32)
+    at = 0
+    for n in calls:
+        s.step(acc[at: at + n])
+        at += n
+    out = s.series(), s.grid(0).copy(), s.dump("dirichlet")
+    counts = s.dump("counts")
+    s.close()
+    return out, counts
+
+
+def _small():
+    v, f, h, mn, dt = sphere_small()
+    return v, f, h, mn, dt, 24, (20, 20, 20)
+
+
+# every remainder of a pass at a call's end, calls of one to three steps (direct launches) between,
+# chunks that whole passes do not divide, calls of several chunks
+@pytest.mark.parametrize("many", [(1, 1), (1, 0), (0, 1)])
+@pytest.mark.parametrize("calls,chunk", [((4, 5, 6, 7, 8, 9), 32), ((12, 1, 13, 3, 14, 2), 32), ((41, 42, 15), 6),
+                                         ((43, 40), 0), ((70,), 32)])
+def test_passes_match_single_steps(gpu, many, calls, chunk):
+    (a, ga, da), _ = _run(_small(), (0, 0), calls, chunk)
+    (b, gb, db), _ = _run(_small(), many, calls, chunk)
+    assert np.all(np.isfinite(b)) and np.abs(b).max() > 0
+    assert rel_l2(b, a) < 1e-12 and rel_l2(gb, ga) < 1e-12 and rel_l2(db, da) < 1e-12
+
+
+def test_dense_scene_completes_by_groups(gpu):
+    """5120 triangles in a res-24 grid: more pairs than the threshold from which the completion of the
+    convolution takes a group of centres per warp (capacity 5/4 of the pairs)."""
+    rng = np.random.default_rng(3)
+    v, f = scenes.perturbed_sphere(4, 0.1, 0.1, rng)
+    h, mn = scenes.grid_for_bbox(v.min(0), v.max(0), 24, 2.0)
+    dt = np.float32(0.5 * h / (np.sqrt(3) * 340.3))
+    geom = (v.astype(np.float32), f, h, mn, dt, 24, (12, 12, 20))
+    (a, ga, da), counts = _run(geom, (0, 0), (22,))
+    (b, gb, db), _ = _run(geom, (1, 1), (22,))
+    assert counts[4] * 5 // 4 > 1500000
+    assert rel_l2(b, a) < 1e-12 and rel_l2(gb, ga) < 1e-12 and rel_l2(db, da) < 1e-12
