@@ -26,7 +26,9 @@
 // its operations' adjoints into those rings with the tables of its own step only, and nothing is
 // kept per corrected cell from one step to the next, so the tables (lists, weights, corrected
 // cells, corners) may change between steps: a moving run is differentiated frame by frame with
-// each frame's tables loaded.  The reverse step at sigma runs seven kernels:
+// each frame's tables loaded.  The reverse step at sigma is eight operations in four launches (P2;
+// P3 and P4; P5 and P6; P7, which ends with P1 of the next reverse step), each a programmatic
+// dependent of the one before:
 //   P1 listeners  Lambda(sigma)[listener cell] += dL/dseries[sigma]
 //   P2 near BEM   per triangle j, over its near pairs (c, j): the BEM-near record (taps k) times
 //                 0.98 Lambda(sigma)[c] into accN/accD[j][sigma - k]; then D[j][sigma] has all its
@@ -50,6 +52,7 @@
 #include <vector>
 #include "fdtd.cuh"
 #include "handle.cuh"
+#include "packed.cuh"
 
 namespace pb
 {
@@ -57,22 +60,16 @@ namespace pb
 struct Adjoint
 {
     long long version = -1;  // Handle::mesh_version the tables were built for
-    int nt = 0, n3 = 0, ncorner = 0;
-    long long pfT = 0, p3T = 0;
     // transposed tables
     int *fT_start = nullptr, *fT_src = nullptr;  // per triangle j: the centres i whose face list holds j
-    void *fT_w = nullptr;                         // [pfT][16] (a_m, b_{m+1}) weight pairs
-    float2 *fT_scale = nullptr;                   // [pfT] (single, double) scales (FP32 weights)
-    int *nT_start = nullptr, *nT_cell = nullptr, *nT_pair = nullptr;  // per triangle: (corrected index, pair)
-    void *nT_w = nullptr;        // [p3T][2][16]: the pair's FDTD-near (shifted) and BEM-near records
-    float2 *nT_scale = nullptr;  // [p3T][2] (FP32 weights)
+    int *fT_pair = nullptr;                       // ... and the face pair (its weight record)
     int *cT_cell = nullptr, *cT_start = nullptr, *cT_ref = nullptr;    // corner cells: (tri * 8 + k)
     // the transposes' scratch; every table array grows only (a moving sweep rebuilds the tables
     // every motion frame), with its capacity in cap[] (elements; bytes for the weights)
     int *d_count = nullptr, *d_cursor = nullptr;  // per key
-    int *d_order = nullptr, *d_owner = nullptr;   // per value
+    int *d_order = nullptr, *d_owner = nullptr;   // per value (order: before its keys are sorted)
     int *d_flag = nullptr;                        // res^3 + 1 corner-cell flags, then their scan
-    long long cap[17] = {};
+    long long cap[11] = {};
     // adjoint state
     void *lam[3] = {nullptr, nullptr, nullptr};
     void *lam_b = nullptr;  // 4 x res^3 (boundary layer only)
@@ -96,52 +93,22 @@ namespace
 
 constexpr int kAdjTop = 1 << 29;  // time index where a fresh reverse sweep starts (any positive value)
 
-template <typename T, int N>
-struct alignas(16) AVec
-{
-    T v[N];
-};
-
-template <typename R>
-struct AdjWRec;
-template <>
-struct AdjWRec<float>
-{
-    using T = __half2;
-    using W4 = AVec<__half2, 4>;
-    using H4 = AVec<float, 4>;
-};
-template <>
-struct AdjWRec<double>
-{
-    using T = double2;
-    using W4 = AVec<double2, 4>;
-    using H4 = AVec<double, 4>;
-};
-
-// a_k and b_k of a weight record entry: the factors that multiply the Neumann and the
-// Dirichlet history in the forward convolution
-__device__ inline float wa(__half2 w, float2 s) { return -__low2float(w) * s.x; }
-__device__ inline float wb(__half2 w, float2 s) { return __high2float(w) * s.y; }
-__device__ inline double wa(double2 w, float2) { return -w.x; }
-__device__ inline double wb(double2 w, float2) { return w.y; }
-
+// (Pointers and sizes that do not change from motion frame to motion frame while no array grows, so a
+// recorded chunk of reverse steps serves a whole moving sweep.)
 template <typename R>
 struct AdjArgs
 {
-    using W = typename AdjWRec<R>::T;
-    int res, nt, n3, nl, ncorner;
+    using W = typename WRec<R>::T;
+    int res, nt, nl;
     long long ncells;
     int listen_cell[8];
-    const int *n3_cell;
-    const unsigned *corr_mask;  // corrected-cell bits
-    const int *fT_start, *fT_src;
-    const W *fT_w;
-    const float2 *fT_scale;
-    const int *nT_start, *nT_cell, *nT_pair;
-    const W *nT_w;
-    const float2 *nT_scale;
-    const int *cT_cell, *cT_start, *cT_ref;
+    const int *fT_start, *fT_src, *fT_pair;
+    const W *face_w;
+    const float2 *face_scale;
+    const int *cellc;  // grid coordinates of the triangles' cells
+    const W *gc_w;     // grid-cache records [nt][54]
+    const float2 *gc_scale;
+    const int *ncorner, *cT_cell, *cT_start, *cT_ref;
     const float *interp;
     const double *interp_d, *denom;
     float reflect;
@@ -173,74 +140,105 @@ struct AdjStep
 
 __device__ inline int adj_sigma(const AdjStep *st, int j) { return st->top - 1 - j; }
 
-// P1: the listener samples' adjoints
+// P1 of the call's first reverse step (the later ones run at the end of P7): the listener samples'
+// adjoints
 template <typename R>
-__global__ void adj_listen_kernel(const __grid_constant__ AdjArgs<R> a, const AdjStep *st, int jstep)
+__global__ void adj_listen_kernel(const __grid_constant__ AdjArgs<R> a, const AdjStep *st)
 {
     if (threadIdx.x != 0)
         return;
-    const int sigma = adj_sigma(st, jstep);
+    const int sigma = adj_sigma(st, 0);
     const R *g = (const R *)st->g + (long long)(sigma - st->bottom) * a.nl;
     for (int l = 0; l < a.nl; l++)  // one thread: listeners may share a cell
         a.slot(sigma)[a.listen_cell[l]] += g[l];
 }
 
+// P1 of the next reverse step at cell i, whose Lambda(sigma - 1) = v is complete but for it
 template <typename R>
-__device__ inline R warp_sum_adj(R v)
+__device__ inline R with_listeners(const AdjArgs<R> &a, const AdjStep *st, int sigma, long long i, R v)
 {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1)
-        v += __shfl_xor_sync(0xffffffffu, v, off);
+    if (sigma - 1 >= st->bottom)
+    {
+        const R *g = (const R *)st->g + (long long)(sigma - 1 - st->bottom) * a.nl;
+        for (int l = 0; l < a.nl; l++)
+            if (a.listen_cell[l] == (int)i)
+                v += g[l];
+    }
     return v;
 }
 
-// sums of the eight quads of a warp per lane position (lanes l, l ^ 4, ..., l ^ 28): lane q < 4 of
-// quad 0 ends with the totals of taps 4q .. 4q + 3
+// The pushes of one triangle: a lane of quad g sums records g, g + 8, ... times the values of their
+// readers into the (N, D) pairs of its taps 4q..4q+3; over the warp that is 16 taps x 2 fields, and
+// the eight sums a lane holds are exactly what the eight quads exchange: lane (g, q) ends with field
+// g & 1 of tap 4q + (g >> 1) and adds it to its own ring slot, 32 slots in one access.
 template <typename R>
-__device__ inline void quad_totals(R (&v)[4])
+struct PushSums
 {
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int off = 4; off < 32; off <<= 1)
-            v[i] += __shfl_xor_sync(0xffffffffu, v[i], off);
-}
-
-// the 16 taps of a near record (half = 0: FDTD-near, shifted by one tap; 1: BEM-near) of near pair p
-// times v[pair], accumulated per lane over the pairs of triangle j (quad g takes pairs g, g + 8, ...;
-// lane q taps 4q .. 4q + 3); cell_value(c) gives the factor of corrected cell c
-template <typename R, typename F>
-__device__ inline void near_push_sums(const AdjArgs<R> &a, int j, int half, int g, int q, F cell_value, R (&an)[4],
-                                      R (&ad)[4])
-{
-    using W4 = typename AdjWRec<R>::W4;
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-        an[i] = ad[i] = 0;
-    for (int p = a.nT_start[j] + g; p < a.nT_start[j + 1]; p += 8)
+    using P = typename WRec<R>::P;
+    P v[4];
+    __device__ PushSums()
     {
-        const R v = cell_value(a.n3_cell[a.nT_cell[p]]);
-        const W4 w = *(const W4 *)(a.nT_w + ((long long)p * 2 + half) * kTaps + 4 * q);
-        const float2 sc = a.nT_scale ? a.nT_scale[2 * p + half] : make_float2(1, 1);
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            v[i] = make_pair2((R)0, (R)0);
+    }
+    // record w (its 4 taps of this lane) with scale sc, times the reader's value x
+    __device__ void add(const typename WRec<R>::W4 &w4, P sc, R x)
+    {
+        const P s = mul2(sc, make_pair2(x, x));
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            v[i] = fma2(weight_pair(w4.v[i]), s, v[i]);
+    }
+    // this lane's total
+    __device__ R total(int lane) const
+    {
+        R x[8];
 #pragma unroll
         for (int i = 0; i < 4; i++)
         {
-            an[i] += (R)wa(w.v[i], sc) * v;
-            ad[i] += (R)wb(w.v[i], sc) * v;
+            x[2 * i] = halves(v[i]).x;
+            x[2 * i + 1] = halves(v[i]).y;
         }
+#pragma unroll
+        for (int half = 4, off = 16; half > 0; half /= 2, off >>= 1)
+        {
+            const bool up = (lane & off) != 0;
+#pragma unroll
+            for (int i = 0; i < half; i++)
+            {
+                const R send = up ? x[i] : x[i + half], keep = up ? x[i + half] : x[i];
+                x[i] = keep + __shfl_xor_sync(kFull, send, off);
+            }
+        }
+        return x[0];
     }
-    quad_totals<R>(an);
-    quad_totals<R>(ad);
+};
+
+// the ring slot of lane (g, q)'s total for a push whose tap k belongs to time tau - k
+template <typename R>
+__device__ inline R *push_slot(const AdjArgs<R> &a, int j, int tau, int lane)
+{
+    const int g = lane >> 2, tap = 4 * (lane & 3) + (g >> 1);
+    return (g & 1 ? a.acc_d : a.acc_n) + (long long)j * kRing + ((tau - tap) & (kRing - 1));
 }
 
-// add tap k of lane q's totals into ring slot (tau0 - k) of triangle j (lanes 0-3)
-template <typename R>
-__device__ inline void ring_add(R *ring, int j, int tau0, int q, const R (&v)[4])
+// near records of triangle j (half = 0: FDTD-near, 1: BEM-near) times value(cell) over the 27 cells
+// around it (all of them inside the grid: triangles lie at least two cells from its faces)
+template <typename R, typename F>
+__device__ inline R near_push(const AdjArgs<R> &a, int j, int half, int lane, F value)
 {
-    R *row = ring + (long long)j * kRing;
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-        row[(tau0 - 4 * q - i) & (kRing - 1)] += v[i];
+    const int g = lane >> 2, q = lane & 3;
+    const int x = a.cellc[3 * j] - 1, y = a.cellc[3 * j + 1] - 1, z = a.cellc[3 * j + 2] - 1;
+    PushSums<R> sums;
+    for (int o = g; o < 27; o += 8)
+    {
+        const long long c = ((long long)(x + o % 3) * a.res + (y + o / 3 % 3)) * a.res + (z + o / 9);
+        const long long r = (long long)j * 54 + half * 27 + o;
+        sums.add(*(const typename WRec<R>::W4 *)(a.gc_w + r * kTaps + 4 * q), record_scale(a.gc_scale, r, (R)0),
+                 value(c));
+    }
+    return sums.total(lane);
 }
 
 // P2: near BEM push, then lamF of triangle j (one warp per triangle)
@@ -248,99 +246,69 @@ template <typename R>
 __global__ void __launch_bounds__(256) adj_bem_kernel(const __grid_constant__ AdjArgs<R> a, const AdjStep *st,
                                                       int jstep)
 {
+    grid_dependency_wait();
     const int sigma = adj_sigma(st, jstep);
     const int j = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (j >= a.nt)
         return;
-    const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    const int lane = threadIdx.x & 31;
     const R *lam = a.slot(sigma);
-    R an[4], ad[4];
-    near_push_sums<R>(a, j, 1, g, q, [&](int c) { return (R)0.98 * lam[c]; }, an, ad);
-    if (lane < 4)
+    const R v = near_push<R>(a, j, 1, lane, [&](long long c) { return (R)0.98 * lam[c]; });
+    R *slot = push_slot(a, j, sigma, lane);
+    const R sum = *slot + v;
+    if (lane == 4)  // D[j][sigma] has all its readers
     {
-        ring_add<R>(a.acc_n, j, sigma, q, an);
-        ring_add<R>(a.acc_d, j, sigma, q, ad);
-    }
-    __syncwarp();
-    if (lane == 0)
-    {
-        R *slot = a.acc_d + (long long)j * kRing + (sigma & (kRing - 1));
-        a.lam_f[j] = (R)(*slot / a.denom[j]);
+        a.lam_f[j] = (R)(sum / a.denom[j]);
         *slot = 0;  // the slot is reused for time sigma - 32
     }
+    else
+        *slot = sum;
 }
 
 // P3: face push (one warp per triangle j over the centres i whose face list holds j), then
-// dL/dacc[sigma][j]
+// dL/dacc[sigma][j].  The records are the forward pass's, found by the pair's index (64 B each, so
+// a gather of whole sectors); Dirichlet tap 0 is the forward step's unknown, no reader of D.
 template <typename R>
-__global__ void __launch_bounds__(256) adj_face_kernel(const __grid_constant__ AdjArgs<R> a, const AdjStep *st,
-                                                       int jstep)
+__device__ inline void adj_face(const AdjArgs<R> &a, const AdjStep *st, int sigma, int j, int lane)
 {
-    const int sigma = adj_sigma(st, jstep);
     R *out_row = st->out ? (R *)st->out + (long long)(sigma - st->bottom) * a.nt : nullptr;
-    using W4 = typename AdjWRec<R>::W4;
-    const int j = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (j >= a.nt)
-        return;
-    const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-    R an[4] = {0, 0, 0, 0}, ad[4] = {0, 0, 0, 0};
-    for (int p = a.fT_start[j] + g; p < a.fT_start[j + 1]; p += 8)
+    const int g = lane >> 2, q = lane & 3;
+    PushSums<R> sums;
+    // the next pair's indices are asked for while this one's record and value are on their way
+    const int e = a.fT_start[j + 1];
+    int p = a.fT_start[j] + g;
+    int pair = p < e ? a.fT_pair[p] : 0, src = p < e ? a.fT_src[p] : 0;
+    for (; p < e; p += 8)
     {
-        const R lf = a.lam_f[a.fT_src[p]];
-        const W4 w = *(const W4 *)(a.fT_w + (long long)p * kTaps + 4 * q);  // (a_m, b_{m+1})
-        const float2 sc = a.fT_scale ? a.fT_scale[p] : make_float2(1, 1);
-#pragma unroll
-        for (int i = 0; i < 4; i++)
+        const typename WRec<R>::W4 w = *(const typename WRec<R>::W4 *)(a.face_w + (long long)pair * kTaps + 4 * q);
+        const auto sc = record_scale(a.face_scale, pair, (R)0);
+        const R x = a.lam_f[src];
+        if (p + 8 < e)
         {
-            an[i] += (R)wa(w.v[i], sc) * lf;
-            ad[i] += (R)wb(w.v[i], sc) * lf;
+            pair = a.fT_pair[p + 8];
+            src = a.fT_src[p + 8];
         }
+        sums.add(w, sc, x);
     }
-    quad_totals<R>(an);
-    quad_totals<R>(ad);
-    if (lane < 4)
+    if (q == 0)
+        sums.v[0] = with_y(sums.v[0], (R)0);
+    const R v = sums.total(lane);
+    R *slot = push_slot(a, j, sigma, lane);
+    if (lane == 0)  // N[j][sigma] has all its readers
     {
-        ring_add<R>(a.acc_n, j, sigma, q, an);
-        ring_add<R>(a.acc_d, j, sigma - 1, q, ad);
-    }
-    __syncwarp();
-    if (lane == 0)
-    {
-        R *slot = a.acc_n + (long long)j * kRing + (sigma & (kRing - 1));
         if (out_row)
-            out_row[j] = *slot;
+            out_row[j] = *slot + v;
         *slot = 0;
     }
-}
-
-// P5: the stored FDTD-near sums of step sigma (one warp per triangle)
-template <typename R>
-__global__ void __launch_bounds__(256) adj_fdtd_near_kernel(const __grid_constant__ AdjArgs<R> a, const AdjStep *st,
-                                                            int jstep)
-{
-    const int sigma = adj_sigma(st, jstep);
-    const int j = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (j >= a.nt)
-        return;
-    const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-    const R *lam = a.slot(sigma);
-    R an[4], ad[4];
-    near_push_sums<R>(a, j, 0, g, q, [&](int c) { return -lam[c]; }, an, ad);
-    if (lane < 4)
-    {
-        ring_add<R>(a.acc_n, j, sigma - 1, q, an);
-        ring_add<R>(a.acc_d, j, sigma - 1, q, ad);
-    }
+    else if (lane != 4)
+        *slot += v;
 }
 
 // P4: corner cells of the face interpolation
 template <typename R>
-__global__ void __launch_bounds__(256) adj_corner_kernel(const __grid_constant__ AdjArgs<R> a, const AdjStep *st,
-                                                         int jstep)
+__device__ inline void adj_corner(const AdjArgs<R> &a, int sigma, int i)
 {
-    const int sigma = adj_sigma(st, jstep);
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.ncorner)
+    if (i >= *a.ncorner)
         return;
     R v = 0;
     for (int r = a.cT_start[i]; r < a.cT_start[i + 1]; r++)
@@ -352,15 +320,41 @@ __global__ void __launch_bounds__(256) adj_corner_kernel(const __grid_constant__
     a.slot(sigma)[a.cT_cell[i]] += (R)a.reflect * v;
 }
 
+// P3 and P4: blocks [0, corner_blocks) the corner cells, the rest a triangle per warp
+template <typename R>
+__global__ void __launch_bounds__(256) adj_face_kernel(const __grid_constant__ AdjArgs<R> a, const AdjStep *st,
+                                                       int jstep, int corner_blocks)
+{
+    grid_dependency_wait();
+    const int sigma = adj_sigma(st, jstep);
+    if (blockIdx.x < corner_blocks)
+    {
+        adj_corner<R>(a, sigma, blockIdx.x * blockDim.x + threadIdx.x);
+        return;
+    }
+    const int j = (int)(((long long)(blockIdx.x - corner_blocks) * blockDim.x + threadIdx.x) >> 5);
+    if (j < a.nt)
+        adj_face<R>(a, st, sigma, j, threadIdx.x & 31);
+}
+
+// P5: the stored FDTD-near sums of step sigma (one warp per triangle).  Record tap k + 1 belongs to
+// time sigma - 1 - k, so tap m to sigma - m; tap 0 is 0 and stays out of the slots of time sigma,
+// which now stand for sigma - 32.
+template <typename R>
+__device__ inline void adj_fdtd_near(const AdjArgs<R> &a, int sigma, int j, int lane)
+{
+    const R *lam = a.slot(sigma);
+    const R v = near_push<R>(a, j, 0, lane, [&](long long c) { return -lam[c]; });
+    if (lane != 0 && lane != 4)
+        *push_slot(a, j, sigma, lane) += v;
+}
+
 __device__ inline int judge_of(int v, int res) { return -((int)(v == 1)) + ((int)(v == res - 2)); }
 
 // P6: the boundary-layer solve transposed
 template <typename R>
-__global__ void __launch_bounds__(256) adj_boundary_kernel(const __grid_constant__ AdjArgs<R> a, const AdjStep *st,
-                                                           int jstep)
+__device__ inline void adj_boundary(const AdjArgs<R> &a, int sigma, int i)
 {
-    const int sigma = adj_sigma(st, jstep);
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int res = a.res;
     if (i >= boundary_cells(res))
         return;
@@ -420,17 +414,77 @@ __global__ void __launch_bounds__(256) adj_boundary_kernel(const __grid_constant
             ghosts[gi[d]] = 0;
 }
 
-// P7: the transposed stencil, one thread per cell of the whole grid (ghost layer included)
+// P5 and P6: blocks [0, boundary_blocks) the boundary layer (none with the PML), the rest a triangle
+// per warp
+template <typename R>
+__global__ void __launch_bounds__(256) adj_near_kernel(const __grid_constant__ AdjArgs<R> a, const AdjStep *st,
+                                                       int jstep, int boundary_blocks)
+{
+    grid_dependency_wait();
+    const int sigma = adj_sigma(st, jstep);
+    if (blockIdx.x < boundary_blocks)
+    {
+        adj_boundary<R>(a, sigma, blockIdx.x * blockDim.x + threadIdx.x);
+        return;
+    }
+    const int j = (int)(((long long)(blockIdx.x - boundary_blocks) * blockDim.x + threadIdx.x) >> 5);
+    if (j < a.nt)
+        adj_fdtd_near<R>(a, sigma, j, threadIdx.x & 31);
+}
+
+// The cells within three of the grid's faces, by index i < shell_cells(res)
+__host__ __device__ inline long long shell_cells(int res)
+{
+    const long long m = res - 6;
+    return 6ll * res * res + 6ll * m * res + 6ll * m * m;
+}
+__device__ inline void shell_cell(int i, int res, int (&c)[3])
+{
+    const int m = res - 6;
+    auto layer = [&](int k) { return k < 3 ? k : res - 6 + k; };
+    if (i < 6 * res * res)
+    {
+        c[0] = layer(i / (res * res)), c[1] = i / res % res, c[2] = i % res;
+        return;
+    }
+    i -= 6 * res * res;
+    if (i < 6 * m * res)
+    {
+        c[1] = layer(i / (m * res)), c[0] = 3 + i / res % m, c[2] = i % res;
+        return;
+    }
+    i -= 6 * m * res;
+    c[2] = layer(i % 6), c[1] = 3 + i / 6 % m, c[0] = 3 + i / 6 / m;
+}
+
+// P7: the transposed stencil, one thread per cell of the whole grid (ghost layer included).  Blocks
+// [0, shell_blocks) take the cells within three of the faces, whose readers may be boundary cells;
+// the rest the cells whose six readers are all interior (blocks_per_plane blocks an x plane): seven
+// loads and a dozen operations instead of six readers' cases, in the same order.  Apart, because a
+// row along z starts and ends in the shell: in one range every warp took both ways (res 64: 11.5 us).
 template <typename R>
 __global__ void __launch_bounds__(256) adj_stencil_kernel(const __grid_constant__ AdjArgs<R> a, const AdjStep *st,
-                                                          int jstep)
+                                                          int jstep, int shell_blocks, int blocks_per_plane)
 {
+    grid_dependency_wait();
     const int sigma = adj_sigma(st, jstep);
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.ncells)
-        return;
-    const int res = a.res;
-    const int y[3] = {(int)(i / ((long long)res * res)), (int)((i / res) % res), (int)(i % res)};
+    const int res = a.res, b = (int)blockIdx.x - shell_blocks;
+    int y[3];
+    if (b < 0)
+    {
+        const int k = blockIdx.x * blockDim.x + threadIdx.x;
+        if (k >= shell_cells(res))
+            return;
+        shell_cell(k, res, y);
+    }
+    else
+    {
+        const int m = res - 6, k = b % blocks_per_plane * blockDim.x + threadIdx.x;
+        if (k >= m * m)
+            return;
+        y[0] = 3 + b / blocks_per_plane, y[1] = 3 + k / m, y[2] = 3 + k % m;
+    }
+    const long long i = ((long long)y[0] * res + y[1]) * res + y[2];
     const R *lq = a.slot(sigma);
     const R *lb = a.lam_b;
     const long long nc = a.ncells;
@@ -441,6 +495,22 @@ __global__ void __launch_bounds__(256) adj_stencil_kernel(const __grid_constant_
         return x0 >= 2 && x0 <= res - 3 && x1 >= 2 && x1 <= res - 3 && x2 >= 2 && x2 <= res - 3;
     };
     const double kappa = a.kappa;
+    R *lc = a.slot(sigma - 1), *lp = a.slot(sigma - 2);
+    if (b >= 0)
+    {
+        const double l = lq[i];
+        const long long sx = (long long)res * res;
+        double cur = (2 - 6 * kappa) * l;
+        cur += kappa * (double)lq[i - sx];
+        cur += kappa * (double)lq[i + sx];
+        cur += kappa * (double)lq[i - res];
+        cur += kappa * (double)lq[i + res];
+        cur += kappa * (double)lq[i - 1];
+        cur += kappa * (double)lq[i + 1];
+        lc[i] = with_listeners<R>(a, st, sigma, i, (R)((double)lc[i] + cur));
+        lp[i] = (R)-l;
+        return;
+    }
     const double coef = a.coef, coef1 = a.coef1, coef2 = a.coef2, coef3 = a.coef3;
     double cur = 0, prev = 0;
     if (interior(y[0], y[1], y[2]))
@@ -486,8 +556,7 @@ __global__ void __launch_bounds__(256) adj_stencil_kernel(const __grid_constant_
                 prev -= coef2 * jd * bd;
             }
         }
-    R *lc = a.slot(sigma - 1), *lp = a.slot(sigma - 2);
-    lc[i] = (R)((double)lc[i] + cur);
+    lc[i] = with_listeners<R>(a, st, sigma, i, (R)((double)lc[i] + cur));
     lp[i] = (R)prev;
 }
 
@@ -513,6 +582,7 @@ template <typename R>
 __global__ void __launch_bounds__(256) adj_pml_kernel(const __grid_constant__ AdjArgs<R> a, const AdjStep *st,
                                                       int jstep)
 {
+    grid_dependency_wait();
     const int sigma = adj_sigma(st, jstep);
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.ncells)
@@ -577,62 +647,11 @@ __global__ void __launch_bounds__(256) adj_pml_kernel(const __grid_constant__ Ad
                 cur += cdt * i2h * (pd + pd3);
             }
         }
-    lc[i] = (R)((double)lc[i] + cur);
+    lc[i] = with_listeners<R>(a, st, sigma, i, (R)((double)lc[i] + cur));
     lp[i] = (R)(-lj);
 #pragma unroll
     for (int k = 0; k < 6; k++)
         pc[6 * i + k] = wj != 0 ? (R)ps[k] : (R)0;  // psi^{sigma-1}[j] is zero where j is undamped
-}
-
-// ---- tables
-template <typename R>
-__global__ void shift_face_kernel(const typename AdjWRec<R>::T *w, const float2 *scale, const int *pair, long long n,
-                                  typename AdjWRec<R>::T *wt, float2 *scale_t)
-{
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n * kTaps)
-        return;
-    const long long p2 = t / kTaps;
-    const int m = (int)(t % kTaps);
-    const long long p = pair[p2];
-    const auto *src = w + p * kTaps;
-    if constexpr (sizeof(R) == 4)
-    {
-        const __half lo = __low2half(src[m]);
-        const __half hi = m + 1 < kTaps ? __high2half(src[m + 1]) : __float2half(0.0f);
-        wt[t] = __halves2half2(lo, hi);
-        if (m == 0 && scale)
-            scale_t[p2] = scale[p];
-    }
-    else
-        wt[t] = make_double2(src[m].x, m + 1 < kTaps ? src[m + 1].y : 0.0);
-}
-
-// near records of the transposed pairs: pair p2 (forward pair pair[p2] of triangle p3_tri and
-// record offset p3_woff) gets its FDTD-near record shifted by one tap (row[k] = tap k + 1, the
-// step pairs it with the next step's history) and its BEM-near record
-template <typename R>
-__global__ void near_records_kernel(const typename AdjWRec<R>::T *gc_w, const float2 *gc_scale, const int *p3_tri,
-                                    const unsigned char *p3_woff, const int *pair, long long n,
-                                    typename AdjWRec<R>::T *wt, float2 *scale_t)
-{
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n * kTaps)
-        return;
-    const long long p2 = t / kTaps;
-    const int k = (int)(t % kTaps);
-    const long long pp = pair[p2];
-    const long long rec = (long long)p3_tri[pp] * 54 + p3_woff[pp];
-    const auto *f = gc_w + rec * kTaps, *b = gc_w + (rec + 27) * kTaps;
-    typename AdjWRec<R>::T zero;
-    memset(&zero, 0, sizeof(zero));
-    wt[p2 * 2 * kTaps + k] = k + 1 < kTaps ? f[k + 1] : zero;
-    wt[p2 * 2 * kTaps + kTaps + k] = b[k];
-    if (k == 0 && gc_scale)
-    {
-        scale_t[2 * p2] = gc_scale[rec];
-        scale_t[2 * p2 + 1] = gc_scale[rec + 27];
-    }
 }
 
 // ---- transposed tables, built on the device (counting transposes, values ascending per key)
@@ -651,23 +670,27 @@ __global__ void key_fill_kernel(const int *key, long long n, const int *start, i
         order[start[key[i]] + atomicAdd(&cursor[key[i]], 1)] = (int)i;
 }
 
-// each key's values ascending: the fill's atomic order is arbitrary, the sweep's sums must not be
-__global__ void key_sort_kernel(const int *start, int nkeys, int *order)
+// each key's values ascending: the fill's atomic order is arbitrary, the sweep's sums must not be.
+// One warp per key: a value's place is the number of smaller ones (the values of a key are distinct).
+// One thread per key with an insertion sort took milliseconds where keys hold over a hundred values.
+__global__ void key_sort_kernel(const int *start, int nkeys, const int *in, int *out)
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (k >= nkeys)
         return;
     const int b = start[k], e = start[k + 1];
-    for (int i = b + 1; i < e; i++)
+    for (int i = b; i < e; i += 32)
     {
-        const int v = order[i];
-        int j = i - 1;
-        while (j >= b && order[j] > v)
+        const int v = i + lane < e ? in[i + lane] : 0;
+        int rank = 0;
+        for (int j = b; j < e; j += 32)
         {
-            order[j + 1] = order[j];
-            j--;
+            const int w = j + lane < e ? in[j + lane] : 0, n = min(32, e - j);
+            for (int m = 0; m < n; m++)
+                rank += __shfl_sync(kFull, w, m) < v;
         }
-        order[j + 1] = v;
+        if (i + lane < e)
+            out[b + rank] = v;
     }
 }
 
@@ -727,26 +750,14 @@ int grow(T **p, long long &cap, long long need)
     return PPPM_OK;
 }
 
-int grow_bytes(void **p, long long &cap, long long need)
-{
-    need = std::max<long long>(need, 1);
-    if (need <= cap)
-        return PPPM_OK;
-    dev_free(*p);
-    *p = nullptr;
-    const long long nc = need + need / 4 + 256;
-    PB_TRY(dev_alloc(p, (size_t)nc));
-    cap = nc;
-    return PPPM_OK;
-}
-
 // start[nkeys + 1], order[n]: the positions p of key[p] grouped by key, ascending inside a key
+// (scratch: A.d_order, n values)
 int transpose_dev(Handle &h, Adjoint &A, const int *key, long long n, int nkeys, int *start, int *order)
 {
     cudaStream_t s = h.stream;
     const int T = 256;
-    PB_TRY(grow(&A.d_count, A.cap[15], (long long)nkeys + 1));
-    PB_TRY(grow(&A.d_cursor, A.cap[16], (long long)nkeys + 1));
+    PB_TRY(grow(&A.d_count, A.cap[9], (long long)nkeys + 1));
+    PB_TRY(grow(&A.d_cursor, A.cap[10], (long long)nkeys + 1));
     PB_CUDA(cudaMemsetAsync(A.d_count, 0, sizeof(int) * (size_t)(nkeys + 1), s));
     PB_CUDA(cudaMemsetAsync(A.d_cursor, 0, sizeof(int) * (size_t)(nkeys + 1), s));
     if (n > 0)
@@ -754,8 +765,8 @@ int transpose_dev(Handle &h, Adjoint &A, const int *key, long long n, int nkeys,
     PB_TRY(exclusive_scan(h, A.d_count, start, nkeys));
     if (n > 0)
     {
-        key_fill_kernel<<<div_up(n, T), T, 0, s>>>(key, n, start, A.d_cursor, order);
-        key_sort_kernel<<<div_up(nkeys, T), T, 0, s>>>(start, nkeys, order);
+        key_fill_kernel<<<div_up(n, T), T, 0, s>>>(key, n, start, A.d_cursor, A.d_order);
+        key_sort_kernel<<<div_up(32ll * nkeys, T), T, 0, s>>>(start, nkeys, A.d_order, order);
         h.launches += 3;
     }
     PB_CHECK_LAUNCH();
@@ -764,11 +775,9 @@ int transpose_dev(Handle &h, Adjoint &A, const int *key, long long n, int nkeys,
 
 void adj_free_tables(Adjoint &A)
 {
-    void **ptrs[] = {(void **)&A.fT_start, (void **)&A.fT_src,   &A.fT_w,   (void **)&A.fT_scale,
-                     (void **)&A.nT_start, (void **)&A.nT_cell,  (void **)&A.nT_pair,  &A.nT_w,
-                     (void **)&A.nT_scale, (void **)&A.cT_cell,  (void **)&A.cT_start, (void **)&A.cT_ref,
-                     (void **)&A.d_count,  (void **)&A.d_cursor, (void **)&A.d_order,  (void **)&A.d_owner,
-                     (void **)&A.d_flag};
+    void **ptrs[] = {(void **)&A.fT_start, (void **)&A.fT_src,   (void **)&A.fT_pair, (void **)&A.cT_cell,
+                     (void **)&A.cT_start, (void **)&A.cT_ref,   (void **)&A.d_count, (void **)&A.d_cursor,
+                     (void **)&A.d_order,  (void **)&A.d_owner,  (void **)&A.d_flag};
     for (void **p : ptrs)
     {
         dev_free(*p);
@@ -794,81 +803,48 @@ void adj_free_state(Adjoint &A)
     A.g_cap = A.out_cap = 0;
 }
 
-// The transposed tables of the current geometry: face pairs by neighbour (with the centre and
-// the re-packed weights), 3^3 pairs by triangle (with the corrected cell and the near records),
-// corner references by cell.  All on the device; one synchronisation reads the number of
-// distinct corner cells.  Capacities only grow, so a sweep over many motion frames allocates
-// once.
-template <typename R>
+// The transposed tables of the current geometry: face pairs by neighbour (with the centre; the
+// weights stay where the forward pass keeps them, as do the near records, whose cells follow from the
+// triangle's), corner references by cell.  All on the device, without a synchronisation: the number
+// of distinct corner cells stays there and the corner lists have room for the most there can be.
+// Capacities only grow, so a sweep over many motion frames allocates once.
 int build_tables(Handle &h, Adjoint &A)
 {
-    using W = typename AdjWRec<R>::T;
     cudaStream_t s = h.stream;
-    const int nt = h.nt, n3 = h.n3, T = 256;
-    const long long pf = h.pf, p3 = h.p3, nc8 = (long long)nt * 8, ncells = h.n_cells;
-    const long long wsz = (long long)sizeof(W);
+    const int nt = h.nt, T = 256;
+    const long long pf = h.pf, nc8 = (long long)nt * 8, ncells = h.n_cells;
+    const int corners = (int)std::min(nc8, ncells);
     long long *c = A.cap;
-    PB_TRY(grow(&A.d_order, c[0], std::max(std::max(pf, p3), nc8)));
-    PB_TRY(grow(&A.d_owner, c[1], std::max(pf, p3)));
+    PB_TRY(grow(&A.d_order, c[0], std::max(pf, nc8)));
+    PB_TRY(grow(&A.d_owner, c[1], std::max(pf, nc8)));
     PB_TRY(grow(&A.fT_start, c[2], nt + 1));
     PB_TRY(grow(&A.fT_src, c[3], pf));
-    PB_TRY(grow_bytes(&A.fT_w, c[4], pf * kTaps * wsz));
-    if (!h.fp64)
-        PB_TRY(grow(&A.fT_scale, c[5], pf));
-    PB_TRY(grow(&A.nT_start, c[6], nt + 1));
-    PB_TRY(grow(&A.nT_cell, c[7], p3));
-    PB_TRY(grow(&A.nT_pair, c[8], p3));
-    PB_TRY(grow_bytes(&A.nT_w, c[9], p3 * 2 * kTaps * wsz));
-    if (!h.fp64)
-        PB_TRY(grow(&A.nT_scale, c[10], 2 * p3));
-    PB_TRY(grow(&A.d_flag, c[11], 2 * (ncells + 1)));
-    PB_TRY(grow(&A.cT_ref, c[12], nc8));
-    int *order = A.d_order, *owner = A.d_owner;
+    PB_TRY(grow(&A.fT_pair, c[4], pf));
+    PB_TRY(grow(&A.d_flag, c[5], 2 * (ncells + 1)));
+    PB_TRY(grow(&A.cT_ref, c[6], nc8));
+    PB_TRY(grow(&A.cT_cell, c[7], corners));
+    PB_TRY(grow(&A.cT_start, c[8], (long long)corners + 1));
 
     // face pairs by neighbour; fT_src = centre of each transposed pair
-    PB_TRY(transpose_dev(h, A, h.d_face_nbr, pf, nt, A.fT_start, order));
+    PB_TRY(transpose_dev(h, A, h.d_face_nbr, pf, nt, A.fT_start, A.fT_pair));
     if (pf > 0)
     {
-        owner_kernel<<<div_up((long long)nt * 32, T), T, 0, s>>>(h.d_face_start, nt, owner);
-        gather_int_kernel<<<div_up(pf, T), T, 0, s>>>(owner, order, pf, A.fT_src);
-        shift_face_kernel<R><<<div_up(pf * kTaps, T), T, 0, s>>>(
-            (const W *)h.d_face_w, h.fp64 ? nullptr : h.d_face_scale, order, pf, (W *)A.fT_w, A.fT_scale);
-        h.launches += 3;
+        owner_kernel<<<div_up((long long)nt * 32, T), T, 0, s>>>(h.d_face_start, nt, A.d_owner);
+        gather_int_kernel<<<div_up(pf, T), T, 0, s>>>(A.d_owner, A.fT_pair, pf, A.fT_src);
+        h.launches += 2;
     }
-    A.pfT = pf;
-    PB_CHECK_LAUNCH();
-
-    // 3^3 pairs by triangle; nT_cell = corrected-cell index of each transposed pair
-    PB_TRY(transpose_dev(h, A, h.d_p3_tri, p3, nt, A.nT_start, A.nT_pair));
-    if (p3 > 0)
-    {
-        owner_kernel<<<div_up((long long)std::max(n3, 1) * 32, T), T, 0, s>>>(h.d_n3_start, n3, owner);
-        gather_int_kernel<<<div_up(p3, T), T, 0, s>>>(owner, A.nT_pair, p3, A.nT_cell);
-        near_records_kernel<R><<<div_up(p3 * kTaps, T), T, 0, s>>>(
-            (const W *)h.d_gc_w, h.fp64 ? nullptr : h.d_gc_scale, h.d_p3_tri, h.d_p3_woff, A.nT_pair, p3,
-            (W *)A.nT_w, A.nT_scale);
-        h.launches += 3;
-    }
-    A.p3T = p3;
     PB_CHECK_LAUNCH();
 
     // corner references by cell: the distinct corner cells ascending, each corner's rank
-    int *flag = A.d_flag, *pos = A.d_flag + (ncells + 1);
+    int *flag = A.d_flag, *pos = A.d_flag + (ncells + 1), *rank = A.d_owner;
     PB_CUDA(cudaMemsetAsync(flag, 0, sizeof(int) * (size_t)(ncells + 1), s));
     flag_cells_kernel<<<div_up(nc8, T), T, 0, s>>>(h.d_face_corner, nc8, ncells, flag);
     h.launches++;
     PB_TRY(exclusive_scan(h, flag, pos, ncells));
-    int ncorner = 0;
-    PB_TRY(read_int(h, pos + ncells, &ncorner));
-    PB_TRY(grow(&A.cT_cell, c[13], ncorner));
-    PB_TRY(grow(&A.cT_start, c[14], (long long)ncorner + 1));
     compact_cells_kernel<<<div_up(ncells, T), T, 0, s>>>(flag, pos, ncells, A.cT_cell);
-    corner_rank_kernel<<<div_up(nc8, T), T, 0, s>>>(h.d_face_corner, nc8, ncells, pos, order);
+    corner_rank_kernel<<<div_up(nc8, T), T, 0, s>>>(h.d_face_corner, nc8, ncells, pos, rank);
     h.launches += 2;
-    PB_TRY(transpose_dev(h, A, order, nc8, ncorner, A.cT_start, A.cT_ref));
-    A.ncorner = ncorner;
-    A.nt = nt;
-    A.n3 = n3;
+    PB_TRY(transpose_dev(h, A, rank, nc8, corners, A.cT_start, A.cT_ref));
     A.version = h.mesh_version;
     return PPPM_OK;
 }
@@ -915,30 +891,26 @@ int zero_state(Handle &h, Adjoint &A)
 template <typename R>
 AdjArgs<R> make_adj_args(Handle &h, Adjoint &A)
 {
-    using W = typename AdjWRec<R>::T;
+    using W = typename WRec<R>::T;
     AdjArgs<R> a;
     memset(&a, 0, sizeof(a));
     a.res = h.res;
     a.nt = h.nt;
-    a.n3 = h.n3;
     a.ncells = h.n_cells;
     a.nl = (int)h.listen_xyz.size() / 3;
     for (int l = 0; l < a.nl; l++)
     {
         a.listen_cell[l] = (h.listen_xyz[3 * l] * h.res + h.listen_xyz[3 * l + 1]) * h.res + h.listen_xyz[3 * l + 2];
     }
-    a.ncorner = A.ncorner;
-    a.n3_cell = h.d_n3_cell;
-    a.corr_mask = h.d_corr_mask;
     a.fT_start = A.fT_start;
     a.fT_src = A.fT_src;
-    a.fT_w = (const W *)A.fT_w;
-    a.fT_scale = h.fp64 ? nullptr : A.fT_scale;
-    a.nT_start = A.nT_start;
-    a.nT_cell = A.nT_cell;
-    a.nT_pair = A.nT_pair;
-    a.nT_w = (const W *)A.nT_w;
-    a.nT_scale = h.fp64 ? nullptr : A.nT_scale;
+    a.fT_pair = A.fT_pair;
+    a.face_w = (const W *)h.d_face_w;
+    a.face_scale = h.fp64 ? nullptr : h.d_face_scale;
+    a.cellc = h.d_cellc;
+    a.gc_w = (const W *)h.d_gc_w;
+    a.gc_scale = h.fp64 ? nullptr : h.d_gc_scale;
+    a.ncorner = A.d_flag + 2 * h.n_cells + 1;  // the total of the corner flags' scan
     a.cT_cell = A.cT_cell;
     a.cT_start = A.cT_start;
     a.cT_ref = A.cT_ref;
@@ -978,30 +950,28 @@ __global__ void advance_adj_kernel(AdjStep *st, int g) { st->top -= g; }
 
 // the kernels of reverse step j of the call (no error check: may run under stream capture)
 template <typename R>
-void adj_launch_step(const AdjArgs<R> &a, const AdjStep *st, int j, cudaStream_t s, long long nbd)
+void adj_launch_step(const AdjArgs<R> &a, const AdjStep *st, int j, cudaStream_t s)
 {
     const int T = 256, tw = div_up((long long)a.nt * 32, T);
-    if (a.nl > 0)
-        adj_listen_kernel<R><<<1, 32, 0, s>>>(a, st, j);
-    adj_bem_kernel<R><<<tw, T, 0, s>>>(a, st, j);
-    adj_face_kernel<R><<<tw, T, 0, s>>>(a, st, j);
-    if (a.ncorner > 0)
-        adj_corner_kernel<R><<<div_up(a.ncorner, T), T, 0, s>>>(a, st, j);
-    adj_fdtd_near_kernel<R><<<tw, T, 0, s>>>(a, st, j);
+    const int cb = div_up(std::min<long long>(8ll * a.nt, a.ncells), T);
+    const int bb = a.pml_w > 0 ? 0 : div_up(boundary_cells(a.res), T);
+    launch_dependent(adj_bem_kernel<R>, tw, T, s, a, st, j);
+    launch_dependent(adj_face_kernel<R>, cb + tw, T, s, a, st, j, cb);
+    launch_dependent(adj_near_kernel<R>, bb + tw, T, s, a, st, j, bb);
     if (a.pml_w > 0)
-        adj_pml_kernel<R><<<div_up(a.ncells, T), T, 0, s>>>(a, st, j);
+        launch_dependent(adj_pml_kernel<R>, div_up(a.ncells, T), T, s, a, st, j);
     else
     {
-        adj_boundary_kernel<R><<<div_up(nbd, T), T, 0, s>>>(a, st, j);
-        adj_stencil_kernel<R><<<div_up(a.ncells, T), T, 0, s>>>(a, st, j);
+        const int m = a.res - 6, sb = div_up(shell_cells(a.res), T), pb = div_up((long long)m * m, T);
+        launch_dependent(adj_stencil_kernel<R>, sb + pb * m, T, s, a, st, j, sb, pb);
     }
 }
 
-// A sweep's reverse steps cost five to seven launches each, so long sweeps with fixed tables
-// replay a recorded chunk of kAdjChunk reverse steps (about 0.1 ms of host time per step to record,
-// once per handle and launch arguments); the steps left over, short calls (a moving sweep's
-// frames) and calls on a stream being captured launch the kernels directly.
-constexpr int kAdjChunk = 32;
+// A reverse step costs four launches, so sweeps replay recorded chunks of kAdjChunk reverse steps
+// (about 2 us of host time a chunk against 2-3 us a launch; recorded once per handle and launch
+// arguments, which stay the same from motion frame to motion frame); the steps left over, short
+// calls and calls on a stream being captured launch the kernels directly.
+constexpr int kAdjChunk = 16;
 
 template <typename R>
 int run_adjoint(Handle &h, const R *g, int nsteps, R *out, int fresh)
@@ -1017,7 +987,7 @@ int run_adjoint(Handle &h, const R *g, int nsteps, R *out, int fresh)
     {
         // the tables of the steps this call covers; the adjoint state (grid slots and per-triangle
         // rings) carries over, so a sweep may continue across a motion frame
-        PB_TRY(build_tables<R>(h, A));
+        PB_TRY(build_tables(h, A));
         PB_TRY(alloc_state<R>(h, A));
     }
     if (fresh || !A.started)
@@ -1028,23 +998,28 @@ int run_adjoint(Handle &h, const R *g, int nsteps, R *out, int fresh)
     }
     const AdjArgs<R> a = make_adj_args<R>(h, A);
     const int top = A.pos, bottom = A.pos - nsteps;
-    const long long nbd = boundary_cells(h.res);
     cudaStream_t s = h.stream;
     if (!A.d_step)
         PB_TRY(dev_alloc(&A.d_step, sizeof(AdjStep)));
     AdjStep *dst = (AdjStep *)A.d_step;
     set_adj_step_kernel<<<1, 1, 0, s>>>(dst, AdjStep{top, bottom, g, out});
     PB_CHECK_LAUNCH();
-    const long long per_step = 5 + (a.nl > 0) + (a.ncorner > 0) - (a.pml_w > 0);
+    const long long per_step = 4;
     h.launches += 1;
+    if (a.nl > 0)
+    {
+        adj_listen_kernel<R><<<1, 32, 0, s>>>(a, dst);
+        h.launches++;
+        PB_CHECK_LAUNCH();
+    }
     int done = 0;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     PB_CUDA(cudaStreamIsCapturing(s, &cs));
-    if (cs == cudaStreamCaptureStatusNone && nsteps >= 2 * kAdjChunk)
+    if (cs == cudaStreamCaptureStatusNone && nsteps >= kAdjChunk)
     {
         std::vector<unsigned char> sig((const unsigned char *)&a, (const unsigned char *)&a + sizeof(a));
         const bool have = A.chunk && A.chunk_sig == sig;
-        if (!have && nsteps >= 4 * kAdjChunk)
+        if (!have && nsteps >= 2 * kAdjChunk)
         {
             if (A.chunk)
                 cudaGraphExecDestroy(A.chunk);
@@ -1053,7 +1028,7 @@ int run_adjoint(Handle &h, const R *g, int nsteps, R *out, int fresh)
             cudaGraph_t graph = nullptr;
             PB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
             for (int j = 0; j < kAdjChunk; j++)
-                adj_launch_step<R>(a, dst, j, s, nbd);
+                adj_launch_step<R>(a, dst, j, s);
             advance_adj_kernel<<<1, 1, 0, s>>>(dst, kAdjChunk);
             cudaError_t e = cudaStreamEndCapture(s, &graph);
             if (e == cudaSuccess)
@@ -1079,7 +1054,7 @@ int run_adjoint(Handle &h, const R *g, int nsteps, R *out, int fresh)
     }
     for (int j = 0; j < nsteps - done; j++)  // relative to the state the chunks advanced
     {
-        adj_launch_step<R>(a, dst, j, s, nbd);
+        adj_launch_step<R>(a, dst, j, s);
         PB_CHECK_LAUNCH();
         h.launches += per_step;
     }
