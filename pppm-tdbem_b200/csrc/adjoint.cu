@@ -116,6 +116,7 @@ struct AdjArgs
     R *lam_b;
     R *acc_n, *acc_d, *lam_f;
     double kappa;                 // (c dt / h)^2: interior leapfrog coefficient
+    const R *abc;                 // inverses of the boundary systems
     R coef, coef1, coef2, coef3;  // boundary solve coefficients (fdtd.cu:88-137)
     // the PML (pml_width > 0): adjoints of the six auxiliary fields per cell at two times
     // (slot = time mod 2) and the update's coefficients (fdtd.cu:179-232)
@@ -382,29 +383,15 @@ __device__ inline void adj_boundary(const AdjArgs<R> &a, int sigma, int i)
         }
     }
     lo[3] = cur[ci];
-    // the forward matrix (same entries as the forward solve), transposed
-    R m[4][4];
-    m[3][3] = 1;
-#pragma unroll
-    for (int d = 0; d < 3; d++)
-        m[3][d] = -a.coef * (judge[d] != 0);
-#pragma unroll
-    for (int r = 0; r < 3; r++)
-    {
-        const int ax = r, ay = (r + 1) % 3, az = (r + 2) % 3;
-        m[r][3] = a.coef1;
-        m[r][ax] = a.coef2;
-        m[r][ay] = a.coef3 * (judge[ay] != 0);
-        m[r][az] = a.coef3 * (judge[az] != 0);
-    }
-    R mt[4][4];
+    // the forward solve's inverse, transposed
+    const R *m = a.abc + 16 * ((judge[0] != 0) + 2 * (judge[1] != 0) + 4 * (judge[2] != 0));
+    R lb[4] = {0, 0, 0, 0};
 #pragma unroll
     for (int r = 0; r < 4; r++)
+        if (r == 3 || judge[r < 3 ? r : 0] != 0)
 #pragma unroll
-        for (int c = 0; c < 4; c++)
-            mt[r][c] = m[c][r];
-    R lb[4];
-    solve4<R>(mt, lo, lb);
+            for (int k = 0; k < 4; k++)
+                lb[k] += m[4 * r + k] * lo[r];
 #pragma unroll
     for (int k = 0; k < 4; k++)
         a.lam_b[k * a.ncells + ci] = lb[k];
@@ -927,10 +914,12 @@ AdjArgs<R> make_adj_args(Handle &h, Adjoint &A)
     const double cd = h.prm.c, dtd = h.prm.dt, hd = h.prm.dl;
     a.kappa = cd * cd * dtd * dtd / (hd * hd);
     const R c = (R)h.prm.c, dt = (R)h.prm.dt, hh = (R)h.prm.dl;
-    a.coef = c * c * dt * dt / (hh * hh);
-    a.coef1 = 1 / (dt * dt);
-    a.coef2 = c / (2 * hh * dt);
-    a.coef3 = -(c * c) / (2 * hh * hh);
+    const AbcCoef<R> k(c, dt, hh);
+    a.coef = k.coef;
+    a.coef1 = k.coef1;
+    a.coef2 = k.coef2;
+    a.coef3 = k.coef3;
+    a.abc = (const R *)h.d_abc;
     for (int i = 0; i < 2; i++)
         a.psi[i] = (R *)A.psi[i];
     a.pml_w = h.prm.pml_width;

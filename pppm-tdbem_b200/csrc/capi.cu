@@ -359,6 +359,11 @@ int pppm_create(const pppm_params *p, pppm_handle **out)
             return fail(rc);
         cudaMemsetAsync(h.d_corr_mask, 0, sizeof(unsigned) * ((h.n_cells + 31) / 32), h.stream);
     }
+    {
+        int rc = step_boundary_table(h);
+        if (rc)
+            return fail(rc);
+    }
     for (int i = 0; i < 4; i++)
         cudaEventCreate(&h.ev[i]);
     for (auto &e : h.evk)
@@ -414,7 +419,7 @@ int pppm_destroy(pppm_handle *ph)
         cudaStreamSynchronize(h.stream);
     step_free(h);
     free_mesh(h);
-    void *ptrs[] = {h.grid[0],        h.grid[1],         h.grid[2],        h.pml[0],          h.pml[1],
+    void *ptrs[] = {h.d_abc,          h.grid[0],        h.grid[1],         h.grid[2],        h.pml[0],          h.pml[1],
                     h.pml[2],         h.d_verts,         h.d_tris,         h.d_center,        h.d_normal,
                     h.d_area,         h.d_cellc,         h.d_basec,        h.d_cell,          h.d_base,
                     h.d_cell_count,   h.d_cell_start,    h.d_cell_tris,    h.d_base_count,    h.d_base_start,

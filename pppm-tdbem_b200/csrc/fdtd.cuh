@@ -6,10 +6,10 @@
 namespace pb
 {
 
-// Closed-form 4x4 solve by 2x2 sub-determinants (the method credited at fdtd.cu:36), kept
+// Closed-form 4x4 inverse by 2x2 sub-determinants (the method credited at fdtd.cu:36), kept
 // operation for operation so the boundary values round like the reference's.
 template <typename R>
-__device__ inline void solve4(const R a[4][4], const R b[4], R out[4])
+__device__ inline void inverse4(const R a[4][4], R inv[4][4])
 {
     R s0 = a[0][0] * a[1][1] - a[1][0] * a[0][1];
     R s1 = a[0][0] * a[1][2] - a[1][0] * a[0][2];
@@ -24,7 +24,6 @@ __device__ inline void solve4(const R a[4][4], const R b[4], R out[4])
     R c1 = a[2][0] * a[3][2] - a[3][0] * a[2][2];
     R c0 = a[2][0] * a[3][1] - a[3][0] * a[2][1];
     R invdet = 1.0 / (s0 * c5 - s1 * c4 + s2 * c3 + s3 * c2 - s4 * c1 + s5 * c0);
-    R inv[4][4];
     inv[0][0] = (a[1][1] * c5 - a[1][2] * c4 + a[1][3] * c3) * invdet;
     inv[0][1] = (-a[0][1] * c5 + a[0][2] * c4 - a[0][3] * c3) * invdet;
     inv[0][2] = (a[3][1] * s5 - a[3][2] * s4 + a[3][3] * s3) * invdet;
@@ -41,14 +40,42 @@ __device__ inline void solve4(const R a[4][4], const R b[4], R out[4])
     inv[3][1] = (a[0][0] * c3 - a[0][1] * c1 + a[0][2] * c0) * invdet;
     inv[3][2] = (-a[3][0] * s3 + a[3][1] * s1 - a[3][2] * s0) * invdet;
     inv[3][3] = (a[2][0] * s3 - a[2][1] * s1 + a[2][2] * s0) * invdet;
-#pragma unroll
-    for (int i = 0; i < 4; i++)
+}
+
+// The matrix of a boundary-layer cell's system (fdtd.cu:88-137) depends only on which axes it is on
+// the boundary of, so the inverses are a table per handle, abc_table[mask] (bit d: axis d), filled
+// once: eight 4x4 matrices instead of one per cell and step.
+template <typename R>
+struct AbcCoef
+{
+    R coef, coef1, coef2, coef3;
+    __host__ __device__ AbcCoef(R c, R dt, R h)
+        : coef(c * c * dt * dt / (h * h)), coef1(1 / (dt * dt)), coef2(c / (2 * h * dt)), coef3(-(c * c) / (2 * h * h))
     {
-        out[i] = 0;
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-            out[i] += inv[i][j] * b[j];
     }
+};
+
+template <typename R>
+__global__ void abc_table_kernel(R c, R dt, R h, R *table)
+{
+    const int mask = threadIdx.x;
+    const AbcCoef<R> k(c, dt, h);
+    auto on = [&](int d) { return (mask >> d) & 1; };
+    R a[4][4], inv[4][4];
+    a[3][3] = 1;
+    for (int d = 0; d < 3; d++)
+        a[3][d] = -k.coef * on(d);
+    for (int i = 0; i < 3; i++)
+    {
+        a[i][3] = k.coef1;
+        a[i][i] = k.coef2;
+        a[i][(i + 1) % 3] = k.coef3 * on((i + 1) % 3);
+        a[i][(i + 2) % 3] = k.coef3 * on((i + 2) % 3);
+    }
+    inverse4<R>(a, inv);
+    for (int i = 0; i < 4; i++)
+        for (int j = 0; j < 4; j++)
+            table[16 * mask + 4 * i + j] = inv[i][j];
 }
 
 // number of cells in the boundary layer of [1, res-2]^3 (a coordinate equal to 1 or res-2)

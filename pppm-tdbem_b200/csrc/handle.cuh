@@ -110,6 +110,7 @@ struct Handle
     TdbemConsts tc{};
 
     void *grid[3] = {nullptr, nullptr, nullptr};  // ring slots, index (t + 3) % 3
+    void *d_abc = nullptr;                        // inverses of the boundary systems (fdtd.cuh)
     void *pml[3] = {nullptr, nullptr, nullptr};
 
     // ---- mesh
@@ -329,6 +330,7 @@ int cache_import_grid(Handle &h, const void *records);                         /
 int cache_import_face(Handle &h, const int *pairs, const void *records, int n);  // n x 72 B
 
 // step.cu
+int step_boundary_table(Handle &h);  // fills d_abc
 int step_prime(Handle &h);
 int step_autotune(Handle &h, int reps, float *us, int *best);
 int step_time_kernels(Handle &h, int reps, float *us);  // us: PPPM_KERNEL_KINDS entries
