@@ -285,7 +285,7 @@ int pppm_pair_weights_static(int device, void *stream, float dt, float dl, float
 
 /* ------------------------------------------------------------ tuning ----------------- */
 /* No counterpart in the reference.  Launch options of the recorded step graphs (pppm_step calls
- * of 4 or more steps with the absorbing boundary).  A change takes effect at the next such call,
+ * of 4 or more steps).  A change takes effect at the next such call,
  * which records new graphs. */
 #define PPPM_OPT_CONV_PAIRS 0   /* 1 (default): the face-pair convolution streams the pairs' weights
                                    once for several consecutive steps (four, at a call's end two);

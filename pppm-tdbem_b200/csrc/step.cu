@@ -475,7 +475,10 @@ __global__ void __launch_bounds__(256) stencil_corr_kernel(const __grid_constant
     stencil_corr_body<R>(a0, ring, st, k, n3_cell, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
-// split-field PML (fdtd.cu:162-232) on [1, res-2]^3; pml slots hold 6 values per cell
+// split-field PML (fdtd.cu:162-232) on [1, res-2]^3; pml slots hold 6 values per cell.  blockIdx.y is
+// the x plane.  The auxiliary fields are read where the update takes them with a factor other than 0
+// only, so cells inside the layer's inner face cost the plain leapfrog: at res 48 with 6 layers (57 %
+// of the cells in the layer) @@
 template <typename R>
 __device__ inline R pml_damp(int x, int y, int z, int res, int w, R damp)
 {
@@ -484,7 +487,7 @@ __device__ inline R pml_damp(int x, int y, int z, int res, int w, R damp)
 
 template <typename R>
 __global__ void __launch_bounds__(256) pml_kernel(const __grid_constant__ StepArgs a0, const __grid_constant__ Ring<R> ring, const StepState *st, int k,
-                                                   const unsigned *corr_mask)
+                                                   const unsigned *corr_mask, int nwrite)
 {
     const StepArgs &a = a0;
     const StepDyn dy = bind_step(st, k, a0.nt);
@@ -493,13 +496,14 @@ __global__ void __launch_bounds__(256) pml_kernel(const __grid_constant__ StepAr
     R *next = ring.slot(dy.tnew);
     const R *pcur = ring.pml(dy.tnew - 1);
     R *pnext = ring.pml(dy.tnew);
-    long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int res = a.res, m = res - 2, w = a.pml_width;
-    if (gid < a.nt)
-        ring.nwrite((int)gid, dy.tnew, dy.acc);
-    if (gid >= (long long)m * m * m)
+    const int plane = blockIdx.x * blockDim.x + threadIdx.x;
+    for (long long i = ((long long)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; i < nwrite;
+         i += (long long)gridDim.x * gridDim.y * blockDim.x)
+        ring.nwrite((int)i, dy.tnew, dy.acc);
+    if (plane >= m * m)
         return;
-    int q[3] = {1 + (int)(gid / ((long long)m * m)), 1 + (int)((gid / m) % m), 1 + (int)(gid % m)};
+    int q[3] = {1 + (int)blockIdx.y, 1 + plane / m, 1 + plane % m};
     const R c = a.c, h = a.h, dt = a.dt, damp = a.damp;
     auto idx = [&](int x, int y, int z) { return ((long long)x * res + y) * res + z; };
     long long ci = idx(q[0], q[1], q[2]);
@@ -518,9 +522,13 @@ __global__ void __launch_bounds__(256) pml_kernel(const __grid_constant__ StepAr
         ps[d] += sgn[d];
         ms[d] -= sgn[d];
         rhs += 1 / (h * h) * (cur[idx(p1[0], p1[1], p1[2])] - 2 * cur[ci] + cur[idx(m1[0], m1[1], m1[2])]);
-        rhs += 1 / h *
-               (cd * pcur[6 * idx(ps[0], ps[1], ps[2]) + 3 + d] -
-                pml_damp<R>(ms[0], ms[1], ms[2], res, w, damp) * pcur[6 * idx(ms[0], ms[1], ms[2]) + d]);
+        const R dm = pml_damp<R>(ms[0], ms[1], ms[2], res, w, damp);
+        if (cd != 0 || dm != 0)
+        {
+            const R fa = cd != 0 ? pcur[6 * idx(ps[0], ps[1], ps[2]) + 3 + d] : (R)0;
+            const R fb = dm != 0 ? pcur[6 * idx(ms[0], ms[1], ms[2]) + d] : (R)0;
+            rhs += 1 / h * (cd * fa - dm * fb);
+        }
     }
     R v = cur[ci] * 2 - prev[ci] + c * c * dt * dt * rhs;
     if (cd != 0)
@@ -1537,7 +1545,7 @@ int make_launch(Handle &h, StepLaunch<R> &L)
     L.mesh = h.mesh_set && h.prm.method == PPPM_METHOD_PPPM ? 1 : 0;
     L.pml = h.prm.pml_width > 0 ? 1 : 0;
     const int m = h.res - 2, T = 256;
-    L.pml_blocks = (int)div_up(std::max<long long>((long long)m * m * m, L.a.nt), T);
+    L.pml_blocks = div_up((long long)m * m, T);
     L.stencil_blocks = L.sp.nb_in + L.sp.nb_bd + L.sp.nb_nt;
     if (h.mesh_set && h.prm.method == PPPM_METHOD_GHOST)
     {
@@ -1575,7 +1583,8 @@ int make_launch(Handle &h, StepLaunch<R> &L)
         // the split step's bulk runs beside the near stage, which overwrites p^{t-1} at corrected
         // cells with the next step's sums: only when no corrected cell neighbours a boundary-layer
         // cell whose solve reads it (mesh_build's check)
-        L.split = h.split_stencil && !h.corr_near_boundary ? 1 : 0;
+        // (the PML update reads neighbours' auxiliary fields and is not split)
+        L.split = h.split_stencil && !h.corr_near_boundary && !L.pml ? 1 : 0;
         for (int m = 0; m < kPass - 1; m++)
         {
             L.fa.face_d[m] = (const R *)h.d_face_d + m * h.pf_cap;
@@ -1620,7 +1629,7 @@ void launch_step(const StepLaunch<R> &L, int k, cudaStream_t s, Handle *timed)
     };
     mark(0);
     if (L.pml)
-        pml_kernel<R><<<L.pml_blocks, T, 0, s>>>(L.a, L.ring, L.st, k, L.corr_mask);
+        pml_kernel<R><<<dim3(L.pml_blocks, L.a.res - 2), T, 0, s>>>(L.a, L.ring, L.st, k, L.corr_mask, L.a.nt);
     else
         stencil_kernel<R><<<L.stencil_blocks, T, 0, s>>>(L.a, L.ring, L.st, k, L.sp, L.corr_mask);
     mark(1);
@@ -1745,8 +1754,10 @@ void capture_pipelined(Handle &h, const StepLaunch<R> &L, int nsteps, bool pair,
             cudaEventRecord(h.ev_bulk, bulk);
             launch_dependent(stencil_corr_kernel<R>, L.corr_blocks, T, s, L.a, L.ring, L.st, k, L.na.n3_cell);
         }
+        else if (L.pml)
+            // the whole update without the Neumann writes (finish / nwrite wrote N[t])
+            pml_kernel<R><<<dim3(L.pml_blocks, L.a.res - 2), T, 0, s>>>(L.a, L.ring, L.st, k, L.corr_mask, 0);
         else
-            // the stencil without its Neumann block range (finish / nwrite wrote N[t])
             stencil_kernel<R><<<L.sp.nb_bd + L.sp.nb_in, T, 0, s>>>(L.a, L.ring, L.st, k, L.sp, L.corr_mask);
         cudaStreamWaitEvent(s, h.ev_conv, 0);
         // (the last step of a graph leaves the next step's needs to the next graph's first kernel)
@@ -1884,7 +1895,7 @@ int graph_for(Handle &h, const StepLaunch<R> &L, int nsteps, cudaGraphExec_t *ou
     g.exec = nullptr;
     cudaGraph_t graph = nullptr;
     PB_CUDA(cudaStreamBeginCapture(h.stream, cudaStreamCaptureModeThreadLocal));
-    if (!timed && L.mesh && !L.pml && h.side)
+    if (!timed && L.mesh && h.side)
         capture_pipelined<R>(h, L, nsteps, L.pairs != 0, open);
     else
     {
@@ -2015,7 +2026,7 @@ int run_steps(Handle &h, const float *acc_dev, int nsteps)
         const int G = (h.graph_chunk + kPass - 1) / kPass * kPass;  // whole passes
         const int chunks = G > 0 && nsteps > G ? (nsteps - 1) / G : 0;
         const int rest = nsteps - chunks * G;
-        const bool pipelined = L.mesh && !L.pml && h.side;
+        const bool pipelined = L.mesh && h.side;
         if (chunks > 0)
         {
             cudaGraphExec_t cexec = nullptr;
