@@ -17,10 +17,10 @@ namespace
 __device__ inline void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename... KArgs, typename... Args>
-void launch_dependent(void (*kern)(KArgs...), int grid, int block, cudaStream_t s, Args... args)
+void launch_dependent(void (*kern)(KArgs...), dim3 grid, int block, cudaStream_t s, Args... args)
 {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(block);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];

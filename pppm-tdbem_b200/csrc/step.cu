@@ -436,6 +436,7 @@ __global__ void __launch_bounds__(256) stencil_kernel(const __grid_constant__ St
                                                        const __grid_constant__ Ring<R> ring, const StepState *st, int k,
                                                        StencilSplit sp, const unsigned *corr_mask)
 {
+    grid_dependency_wait();
     stencil_body<R>(a0, ring, bind_step(st, k, a0.nt), blockIdx.x, sp, corr_mask);
 }
 
@@ -489,6 +490,7 @@ template <typename R>
 __global__ void __launch_bounds__(256) pml_kernel(const __grid_constant__ StepArgs a0, const __grid_constant__ Ring<R> ring, const StepState *st, int k,
                                                    const unsigned *corr_mask, int nwrite)
 {
+    grid_dependency_wait();
     const StepArgs &a = a0;
     const StepDyn dy = bind_step(st, k, a0.nt);
     R *series = (R *)dy.series;
@@ -1191,6 +1193,7 @@ template <typename R, int T>
 __global__ void __launch_bounds__(kConvThreads, sizeof(R) == 4 ? 16 : 1) conv_kernel(const __grid_constant__ Ring<R> ring, const StepState *st,
                                                             int kstep, const __grid_constant__ FaceArgs<R> f, R *conv)
 {
+    grid_dependency_wait();
     conv_groups<R, T>(ring, st->tnew0 + kstep, f, blockIdx.x, gridDim.x, conv);
 }
 
@@ -1264,6 +1267,7 @@ __device__ inline void face_fix(const FaceArgs<R> &f, int nt, R *conv, int tri, 
 template <typename R, int J, bool groups>
 __global__ void __launch_bounds__(256) fix_kernel(int nt, const __grid_constant__ FaceArgs<R> f, R *conv, int slot)
 {
+    grid_dependency_wait();
     const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if constexpr (groups)
         face_fix_groups<R, J>(f, nt, conv, w, (int)((gridDim.x * blockDim.x) >> 5), lane, slot);
@@ -1473,6 +1477,7 @@ struct StepLaunch
     int pairs;         // pipelined graphs convolve the face pairs for several steps per pass
     int face_threads;  // threads per block of the pipelined face-stage kernels
     int tpairs;        // the near-field terms several steps per pass
+    int linear;        // recorded graphs: one branch (run_steps)
     int split;         // recorded graphs: corrected-cell stencil on the main branch, the bulk beside it
     int corr_blocks;   // grid of stencil_corr_kernel (threads stride over the corrected cells)
     int mesh, pml, pml_blocks, stencil_blocks, face_blocks, near_blocks;
@@ -1648,6 +1653,14 @@ void launch_step(const StepLaunch<R> &L, int k, cudaStream_t s, Handle *timed)
     mark(3);
 }
 
+// Instantiating a recorded graph costs about 50 us for every fork of its branches (two a step) and as
+// much again when it is destroyed, 2 us a kernel otherwise: 4.9 against 1.9 ms for the first 96 steps of a
+// new scene, and 3.5 ms less when it is closed.  A handle's first steps therefore replay graphs of
+// one branch (capture_pipelined with L.linear: the same kernels one after another as dependent
+// launches, the stencil unsplit; same results), which run 3 (res 27) to 5 us a step (res 64) slower,
+// and the branched graphs are recorded once a handle has this many steps behind or before it.
+constexpr long long kBranchSteps = 1024;
+
 // The kernels of nsteps steps as a multi-branch graph (absorbing boundary with a mesh).  Per step:
 //   side   conv(k)                       after finish(k-1): needs D[t-1] and N[t]
 //   main   stencil(k) -> finish(k) -> near(k)   finish waits for conv(k) too
@@ -1679,13 +1692,20 @@ __global__ void advance_state_kernel(StepState *st, int g, int nt)
 // first kernel writes what its first step needs.
 // the face-pair convolution of step k, or the completion of its sum
 template <typename R>
-void launch_conv(const StepLaunch<R> &L, int k, PassAt p, cudaStream_t s)
+void launch_conv(const StepLaunch<R> &L, int k, PassAt p, cudaStream_t s, bool dependent = false)
 {
     const int FT = L.face_threads, nt = L.a.nt, groups = L.fix_groups;
     const int wblocks = div_up((groups ? nt / 2 + 1 : nt) * 32ll, FT), slot = p.pos == 1 ? (k - 1) & (kPass - 1) : 0;
-    auto fix = [&](auto by_group, auto by_triangle) {
-        (groups ? by_group : by_triangle)<<<wblocks, FT, 0, s>>>(nt, L.fa, L.conv, slot);
+    auto go = [&](auto kern, int grid, int block, auto... args) {
+        if (dependent)
+            launch_dependent(kern, grid, block, s, args...);
+        else
+            kern<<<grid, block, 0, s>>>(args...);
     };
+    auto fix = [&](auto by_group, auto by_triangle) {
+        go(groups ? by_group : by_triangle, wblocks, FT, nt, L.fa, L.conv, slot);
+    };
+    auto conv = [&](auto kern) { go(kern, L.conv_blocks, kConvThreads, L.ring, L.st, k, L.fa, L.conv); };
     if (p.pos == 1)
         fix(fix_kernel<R, 1, true>, fix_kernel<R, 1, false>);
     else if (p.pos == 2)
@@ -1693,11 +1713,11 @@ void launch_conv(const StepLaunch<R> &L, int k, PassAt p, cudaStream_t s)
     else if (p.pos == 3)
         fix(fix_kernel<R, 3, true>, fix_kernel<R, 3, false>);
     else if (p.size == kPass)
-        conv_kernel<R, kPass><<<L.conv_blocks, kConvThreads, 0, s>>>(L.ring, L.st, k, L.fa, L.conv);
+        conv(conv_kernel<R, kPass>);
     else if (p.size == 2)
-        conv_kernel<R, 2><<<L.conv_blocks, kConvThreads, 0, s>>>(L.ring, L.st, k, L.fa, L.conv);
+        conv(conv_kernel<R, 2>);
     else
-        conv_kernel<R, 1><<<L.conv_blocks, kConvThreads, 0, s>>>(L.ring, L.st, k, L.fa, L.conv);
+        conv(conv_kernel<R, 1>);
 }
 
 // finish of step k in the given mode; conv_pos: where the step's convolution sum lies.  dependent:
@@ -1731,20 +1751,26 @@ void capture_pipelined(Handle &h, const StepLaunch<R> &L, int nsteps, bool pair,
     const int T = 256;
     const int nt = L.a.nt;
     cudaStream_t s = h.stream, side = h.side, bulk = h.side2;
-    const bool split = L.split && bulk;
+    const bool split = L.split && bulk && !L.linear;
     StencilSplit bsp = L.sp;
     bsp.skip_corrected = 1;
     const long long total = open ? nsteps + (1ll << 40) : nsteps;
     nwrite_kernel<R><<<div_up(nt, T), T, 0, s>>>(L.ring, L.st, 0, nt, L.fa, neumann_needs(0, total, pair));
-    cudaEventRecord(h.ev_fin, s);
+    if (!L.linear)
+        cudaEventRecord(h.ev_fin, s);
     if (split)
         cudaEventRecord(h.ev_near, s);
     for (int k = 0; k < nsteps; k++)
     {
         const PassAt p = pass_at(k, total, pair);
-        cudaStreamWaitEvent(side, h.ev_fin, 0);
-        launch_conv<R>(L, k, p, side);
-        cudaEventRecord(h.ev_conv, side);
+        if (L.linear)
+            launch_conv<R>(L, k, p, s, true);
+        else
+        {
+            cudaStreamWaitEvent(side, h.ev_fin, 0);
+            launch_conv<R>(L, k, p, side);
+            cudaEventRecord(h.ev_conv, side);
+        }
         if (split)
         {
             if (k > 0)
@@ -1754,16 +1780,18 @@ void capture_pipelined(Handle &h, const StepLaunch<R> &L, int nsteps, bool pair,
             cudaEventRecord(h.ev_bulk, bulk);
             launch_dependent(stencil_corr_kernel<R>, L.corr_blocks, T, s, L.a, L.ring, L.st, k, L.na.n3_cell);
         }
+        // (below: the whole update without the Neumann writes; finish / nwrite wrote N[t])
         else if (L.pml)
-            // the whole update without the Neumann writes (finish / nwrite wrote N[t])
-            pml_kernel<R><<<dim3(L.pml_blocks, L.a.res - 2), T, 0, s>>>(L.a, L.ring, L.st, k, L.corr_mask, 0);
+            launch_dependent(pml_kernel<R>, dim3(L.pml_blocks, L.a.res - 2), T, s, L.a, L.ring, L.st, k, L.corr_mask, 0);
         else
-            stencil_kernel<R><<<L.sp.nb_bd + L.sp.nb_in, T, 0, s>>>(L.a, L.ring, L.st, k, L.sp, L.corr_mask);
-        cudaStreamWaitEvent(s, h.ev_conv, 0);
+            launch_dependent(stencil_kernel<R>, L.sp.nb_bd + L.sp.nb_in, T, s, L.a, L.ring, L.st, k, L.sp, L.corr_mask);
+        if (!L.linear)
+            cudaStreamWaitEvent(s, h.ev_conv, 0);
         // (the last step of a graph leaves the next step's needs to the next graph's first kernel)
         const int next = k + 1 < nsteps ? neumann_needs(k + 1, total, pair) : 0;
         launch_finish<R>(L, k, finish_mode(k, total, L.tpairs != 0), p.pos, next, s, true);
-        cudaEventRecord(h.ev_fin, s);
+        if (!L.linear)
+            cudaEventRecord(h.ev_fin, s);
         launch_dependent(near_kernel<R>, L.near_blocks, T, s, L.a, L.ring, L.st, k, L.na, 0);
         if (split)
             cudaEventRecord(h.ev_near, s);
@@ -1937,6 +1965,8 @@ int run_steps(Handle &h, const float *acc_dev, int nsteps)
     PB_CHECK_LAUNCH();
     StepLaunch<R> L;
     PB_TRY(make_launch<R>(h, L));
+    L.linear = h.steps_run + nsteps < kBranchSteps ? 1 : 0;
+    h.steps_run += nsteps;
     const long long per_step = 1 + (h.mesh_set ? 2 : 0);
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     PB_CUDA(cudaStreamIsCapturing(s, &cs));
@@ -2041,7 +2071,7 @@ int run_steps(Handle &h, const float *acc_dev, int nsteps)
         // stencil (and its bulk), finish and near: counted here in place of per_step below; a
         // chunk also advances the state
         if (pipelined)
-            h.launches += (chunks + 1) + (4 + L.split - per_step) * (long long)nsteps;
+            h.launches += (chunks + 1) + (4 + (L.split && !L.linear) - per_step) * (long long)nsteps;
         h.launches += chunks;
     }
     else
@@ -2516,13 +2546,16 @@ int step_run(Handle &h, const float *acc_dev, int nsteps)
 
 int step_free(Handle &h)
 {
-    for (auto *g : {&h.graphs[0], &h.graphs[1], &h.graphs[2], &h.graphs[3], &h.timing_graph, &h.profile_graph})
-    {
-        if (g->exec)
-            cudaGraphExecDestroy(g->exec);
-        g->exec = nullptr;
-        g->sig.clear();
-    }
+    auto release = [](StepGraph &g) {
+        if (g.exec)
+            cudaGraphExecDestroy(g.exec);
+        g.exec = nullptr;
+        g.sig.clear();
+    };
+    for (StepGraph &g : h.graphs)
+        release(g);
+    release(h.timing_graph);
+    release(h.profile_graph);
     dev_free(h.d_state);
     h.d_state = nullptr;
     return PPPM_OK;
