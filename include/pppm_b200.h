@@ -93,10 +93,10 @@ int pppm_update_mesh(pppm_handle *h, const float *verts, int verts_on_device);
  * acc holds nsteps rows of nt per-triangle normal accelerations (row s drives step s);
  * acc_on_device != 0: acc is a device pointer.  Listener values are recorded on the device
  * after every step (the demo's per-step read, experiments/demo/main.cu:266).  The call returns
- * once the steps are queued.  The step kernels raise a device status bit when a Dirichlet value
+ * once the steps are queued.  The step kernels raise a status bit when a Dirichlet value
  * or a listener sample is not finite (the reference aborts on a NaN listener sample,
- * experiments/demo/main.cu:161-168); a copy of that word is queued behind the steps, and a later
- * pppm_step whose predecessors' copy has arrived returns PPPM_ERR_NAN without queuing anything,
+ * experiments/demo/main.cu:161-168) and tell the host; a later pppm_step that finds it raised
+ * returns PPPM_ERR_NAN without queuing anything,
  * until pppm_reset_fields or pppm_restore_state clears it. */
 int pppm_step(pppm_handle *h, const float *acc, int acc_on_device, int nsteps);
 

@@ -217,22 +217,13 @@ int d2h(Handle &h, std::vector<T> &v, const void *src, size_t n)
 
 extern "C" {
 
-// The step status of the calls whose copy has arrived: PPPM_ERR_NAN once a step kernel saw a
-// non-finite Dirichlet value or listener sample.  wait: block until the last copy has arrived.
-static int poll_step_status(Handle &h, bool wait)
+// The step status as far as it has reached the host: PPPM_ERR_NAN once a step kernel saw a
+// non-finite Dirichlet value or listener sample (it writes the host's mapped word; a queued copy and
+// an event behind every call cost a step-by-step program 4 us a step).
+static int poll_step_status(Handle &h)
 {
-    if (h.status_pending)
-    {
-        cudaError_t e = wait ? cudaEventSynchronize(h.ev_status) : cudaEventQuery(h.ev_status);
-        if (e == cudaSuccess)
-        {
-            h.status_pending = false;
-            if (*h.h_step_status & 1)
-                h.nonfinite = true;
-        }
-        else if (e != cudaErrorNotReady)
-            PB_CUDA(e);
-    }
+    if (*(volatile int *)h.h_step_status & 1)
+        h.nonfinite = true;
     if (h.nonfinite)
     {
         set_error("a non-finite Dirichlet value or listener sample appeared in an earlier step (reset the fields or "
@@ -242,26 +233,10 @@ static int poll_step_status(Handle &h, bool wait)
     return PPPM_OK;
 }
 
-// queue a copy of the step status word behind the work on the handle's stream (not while the
-// caller captures the stream: the copy would become part of the graph)
-static int queue_step_status(Handle &h)
-{
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    PB_CUDA(cudaStreamIsCapturing(h.stream, &cs));
-    if (cs != cudaStreamCaptureStatusNone)
-        return PPPM_OK;
-    PB_CUDA(cudaMemcpyAsync(h.h_step_status, h.d_step_status, sizeof(int), cudaMemcpyDeviceToHost, h.stream));
-    PB_CUDA(cudaEventRecord(h.ev_status, h.stream));
-    h.status_pending = true;
-    return PPPM_OK;
-}
-
 // forget a non-finite flag: the fields it concerned are being replaced
 static int clear_step_status(Handle &h)
 {
-    if (h.status_pending)
-        PB_CUDA(cudaEventSynchronize(h.ev_status));
-    h.status_pending = false;
+    PB_CUDA(cudaStreamSynchronize(h.stream));  // queued steps may still raise it
     h.nonfinite = false;
     *h.h_step_status = 0;
     PB_CUDA(cudaMemsetAsync(h.d_step_status, 0, sizeof(int), h.stream));
@@ -369,18 +344,28 @@ int pppm_create(const pppm_params *p, pppm_handle **out)
     for (auto &e : h.evk)
         cudaEventCreate(&e);
     {
-        int rc = dalloc(&h.d_step_status, 1);
+        int rc = dalloc(&h.d_step_status, 4);
         if (rc)
             return fail(rc);
-        cudaMemsetAsync(h.d_step_status, 0, sizeof(int), h.stream);
-        if (cudaMallocHost((void **)&h.h_step_status, sizeof(int)) != cudaSuccess ||
-            cudaEventCreateWithFlags(&h.ev_status, cudaEventDisableTiming) != cudaSuccess)
+        void *mapped = nullptr;
+        if (cudaHostAlloc((void **)&h.h_step_status, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
+            cudaHostGetDevicePointer(&mapped, h.h_step_status, 0) != cudaSuccess)
         {
-            h.h_step_status = nullptr;
-            set_error("cudaMallocHost / cudaEventCreate failed");
+            set_error("cudaHostAlloc failed");
             return fail(PPPM_ERR_NOMEM);
         }
         *h.h_step_status = 0;
+        struct
+        {
+            int word[2];
+            void *host;
+        } init{{0, 0}, mapped};
+        static_assert(sizeof(init) == 4 * sizeof(int), "layout of the status words");
+        if (cudaMemcpyAsync(h.d_step_status, &init, sizeof(init), cudaMemcpyHostToDevice, h.stream) != cudaSuccess)
+        {
+            set_error("device initialisation failed");
+            return fail(PPPM_ERR_CUDA);
+        }
     }
     if (cudaStreamCreateWithFlags(&h.side, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&h.side2, cudaStreamNonBlocking) != cudaSuccess ||
@@ -441,8 +426,6 @@ int pppm_destroy(pppm_handle *ph)
     dev_free(h.d_step_status);
     if (h.h_step_status)
         cudaFreeHost(h.h_step_status);
-    if (h.ev_status)
-        cudaEventDestroy(h.ev_status);
     if (h.h_pin)
         cudaFreeHost(h.h_pin);
     if (h.ev_fin)
@@ -607,7 +590,7 @@ int pppm_step(pppm_handle *ph, const float *acc, int acc_on_device, int nsteps)
         set_error("a cache state was restored: call pppm_update_mesh before stepping");
         return PPPM_ERR_STATE;
     }
-    PB_TRY(poll_step_status(h, false));
+    PB_TRY(poll_step_status(h));
     const float *dacc = nullptr;
     if (h.mesh_set)
     {
@@ -628,8 +611,7 @@ int pppm_step(pppm_handle *ph, const float *acc, int acc_on_device, int nsteps)
         }
     }
     PB_TRY(ensure_series(h, nsteps));
-    PB_TRY(step_run(h, dacc, nsteps));
-    return queue_step_status(h);
+    return step_run(h, dacc, nsteps);
 }
 
 int pppm_sync(pppm_handle *ph)
@@ -637,11 +619,7 @@ int pppm_sync(pppm_handle *ph)
     PB_TRY(check_handle(ph));
     Handle &h = ph->h;
     PB_CUDA(cudaStreamSynchronize(h.stream));
-    PB_CUDA(cudaMemcpy(h.h_step_status, h.d_step_status, sizeof(int), cudaMemcpyDeviceToHost));
-    h.status_pending = false;
-    if (*h.h_step_status & 1)
-        h.nonfinite = true;
-    return poll_step_status(h, false);
+    return poll_step_status(h);
 }
 
 struct pppm_batch

@@ -85,6 +85,7 @@ struct StepGraph
 {
     int nsteps = 0;
     bool open = false;               // a chunk of a longer call (more steps follow; see run_steps)
+    bool plain = false;              // the kernels of direct launches (short calls; see run_steps)
     std::vector<unsigned char> sig;  // the launch set it was recorded with
     cudaGraphExec_t exec = nullptr;
 };
@@ -184,10 +185,10 @@ struct Handle
     int *d_pair_flag = nullptr;  // pf scratch: 1 = recompute
     // device words: [0] status (capacity / timeout), [1] a triangle near the boundary layer, [2] centre groups
     int *d_status = nullptr;
-    int *d_step_status = nullptr;  // step status word: non-finite values seen by the step kernels
-    int *h_step_status = nullptr;  // pinned copy, written behind each pppm_step call
-    cudaEvent_t ev_status = nullptr;  // recorded after that copy
-    bool status_pending = false;   // a copy is queued and not yet looked at
+    // step status: [0] the word the step kernels raise (non-finite values), [2..3] the address of the
+    // host's word
+    int *d_step_status = nullptr;
+    int *h_step_status = nullptr;  // mapped host memory: written by the kernel that raises the word
     bool nonfinite = false;        // a non-finite value was seen (until the fields are reset)
     void *d_spec = nullptr;      // recompute scratch spectra
     size_t spec_bytes = 0;
@@ -244,6 +245,7 @@ struct Handle
     StepGraph graphs[kStepGraphs];
     StepGraph timing_graph;  // one step with event records between its kernels (measurement mode)
     int graph_next = 0;
+    int short_calls = 0;      // calls of fewer than kGraphSteps steps so far (kPlainCalls)
     long long steps_run = 0;  // steps queued so far (kBranchSteps)
     int near_blocks = 0;  // resident grid of the near kernel
     int batch_near_cells = 0;  // corrected cells the batch block map covers (grow-only, step.cu)

@@ -66,8 +66,9 @@ constexpr int kStepNonFinite = 1;
 template <typename R>
 __device__ inline void flag_nonfinite(int *status, R v)
 {
-    if (status && !isfinite(v))
-        atomicOr(status, kStepNonFinite);
+    // the first to see one also tells the host (its word is mapped; poll_step_status reads it)
+    if (status && !isfinite(v) && atomicOr(status, kStepNonFinite) == 0)
+        **(volatile int **)(status + 2) = kStepNonFinite;
 }
 
 
@@ -1351,6 +1352,7 @@ __global__ void __launch_bounds__(256) face_kernel(const __grid_constant__ StepA
                                                     const __grid_constant__ Ring<R> ring, const StepState *st, int kstep,
                                                     const __grid_constant__ FaceArgs<R> f)
 {
+    grid_dependency_wait();
     const int tri = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (tri < a0.nt)
         face_body<R>(a0, ring, bind_step(st, kstep, a0.nt), f, tri, threadIdx.x & 31);
@@ -1646,9 +1648,9 @@ void launch_step(const StepLaunch<R> &L, int k, cudaStream_t s, Handle *timed)
         }
     if (L.mesh)
     {
-        face_kernel<R><<<L.face_blocks, T, 0, s>>>(L.a, L.ring, L.st, k, L.fa);
+        launch_dependent(face_kernel<R>, L.face_blocks, T, s, L.a, L.ring, L.st, k, L.fa);
         mark(2);
-        near_kernel<R><<<L.near_blocks, T, 0, s>>>(L.a, L.ring, L.st, k, L.na, 0);
+        launch_dependent(near_kernel<R>, L.near_blocks, T, s, L.a, L.ring, L.st, k, L.na, 0);
     }
     mark(3);
 }
@@ -1895,12 +1897,15 @@ int profile_graph(Handle &h, const StepLaunch<R> &L, cudaGraphExec_t *out)
 // Calls of at least kGraphSteps steps replay a CUDA graph of their kernels, recorded on the
 // first call with that step count and launch set (the graph removes the host launch cost and
 // most of the gap between dependent kernels); shorter calls, measurement mode and calls on a
-// stream that the caller is capturing launch the kernels directly.
+// stream that the caller is capturing launch the kernels directly.  A program that goes on step by
+// step is bound by the host's launches (about 2 us each): from its kPlainCalls-th short call on a
+// handle replays those kernels too as a graph (plain: the same kernels in the same order).
 constexpr int kGraphSteps = 4;
+constexpr int kPlainCalls = 16;
 
 template <typename R>
 int graph_for(Handle &h, const StepLaunch<R> &L, int nsteps, cudaGraphExec_t *out, bool timed = false,
-              bool open = false)
+              bool open = false, bool plain = false)
 {
     const unsigned char *sig = (const unsigned char *)&L;
     StepGraph *slots = timed ? &h.timing_graph : h.graphs;
@@ -1908,7 +1913,7 @@ int graph_for(Handle &h, const StepLaunch<R> &L, int nsteps, cudaGraphExec_t *ou
     for (int i = 0; i < nslots; i++)
     {
         StepGraph &g = slots[i];
-        if (g.exec && g.nsteps == nsteps && g.open == open && g.sig.size() == sizeof(L) &&
+        if (g.exec && g.nsteps == nsteps && g.open == open && g.plain == plain && g.sig.size() == sizeof(L) &&
             memcmp(g.sig.data(), sig, sizeof(L)) == 0)
         {
             *out = g.exec;
@@ -1923,7 +1928,7 @@ int graph_for(Handle &h, const StepLaunch<R> &L, int nsteps, cudaGraphExec_t *ou
     g.exec = nullptr;
     cudaGraph_t graph = nullptr;
     PB_CUDA(cudaStreamBeginCapture(h.stream, cudaStreamCaptureModeThreadLocal));
-    if (!timed && L.mesh && h.side)
+    if (!timed && !plain && L.mesh && h.side)
         capture_pipelined<R>(h, L, nsteps, L.pairs != 0, open);
     else
     {
@@ -1945,6 +1950,7 @@ int graph_for(Handle &h, const StepLaunch<R> &L, int nsteps, cudaGraphExec_t *ou
     }
     g.nsteps = nsteps;
     g.open = open;
+    g.plain = plain;
     g.sig.assign(sig, sig + sizeof(L));
     *out = g.exec;
     return PPPM_OK;
@@ -2073,6 +2079,13 @@ int run_steps(Handle &h, const float *acc_dev, int nsteps)
         if (pipelined)
             h.launches += (chunks + 1) + (4 + (L.split && !L.linear) - per_step) * (long long)nsteps;
         h.launches += chunks;
+    }
+    else if (cs == cudaStreamCaptureStatusNone && ++h.short_calls >= kPlainCalls)
+    {
+        L.linear = 0;  // no part of these kernels: keeps the launch set the same
+        cudaGraphExec_t exec = nullptr;
+        PB_TRY(graph_for<R>(h, L, nsteps, &exec, false, false, true));
+        PB_CUDA(cudaGraphLaunch(exec, s));
     }
     else
         for (int k = 0; k < nsteps; k++)
