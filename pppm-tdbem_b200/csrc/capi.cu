@@ -144,7 +144,7 @@ void free_mesh(Handle &h)
                      (void **)&h.d_hist,       (void **)&h.d_terms,       (void **)&h.d_conv,
                      (void **)&h.d_gneu,       (void **)&h.d_gneu_old,    (void **)&h.d_face_d,
                      (void **)&h.d_nfut,       (void **)&h.d_dlast,       (void **)&h.d_part,
-                     (void **)&h.d_groups};
+                     (void **)&h.d_groups,     (void **)&h.d_p3_ref};
     for (void **q : ptrs)
     {
         dev_free(*q);

@@ -135,7 +135,7 @@ struct Handle
     int n3 = 0;
     long long p3 = 0;
     int *d_n3_cell = nullptr, *d_n3_start = nullptr;
-    int *d_p3_tri = nullptr;
+    int *d_p3_tri = nullptr, *d_p3_ref = nullptr;  // triangle; triangle * 27 + record offset
     unsigned char *d_p3_woff = nullptr;
     long long p3_cap = 0;
     unsigned *d_corr_mask = nullptr;

@@ -252,7 +252,8 @@ __global__ void compact_kernel(const int *flag, const int *pos, const int *start
 // 3^3 pairs of each corrected cell, sub-cells x fastest (particle_grid.cu:164-182);
 // woff = GridCache weight index of (cell - triangle cell) (pppm_cache.h:38-42)
 __global__ void fill_pairs3_kernel(const int *n3_cell, const int *n3_start, int n3, int res, const int *cell_start,
-                                   const int *cell_tris, int *p3_tri, unsigned char *p3_woff, unsigned *mask)
+                                   const int *cell_tris, int *p3_tri, unsigned char *p3_woff, int *p3_ref,
+                                   unsigned *mask)
 {
     // one warp per corrected cell: lane l < 27 copies sub-cell l's list to its offset in the
     // cell's list (a warp prefix sum over the 27 lengths keeps the sub-cell order)
@@ -286,6 +287,7 @@ __global__ void fill_pairs3_kernel(const int *n3_cell, const int *n3_start, int 
     {
         p3_tri[o + j] = cell_tris[b + j];
         p3_woff[o + j] = woff;
+        p3_ref[o + j] = cell_tris[b + j] * 27 + woff;
     }
     if (lane == 0)
         atomicOr(&mask[c >> 5], 1u << (c & 31));
@@ -655,16 +657,19 @@ int mesh_build(Handle &h)
     {
         dev_free(h.d_p3_tri);
         dev_free(h.d_p3_woff);
+        dev_free(h.d_p3_ref);
+        h.d_p3_ref = nullptr;
         h.d_p3_tri = nullptr;
         h.d_p3_woff = nullptr;
         long long cap = p3 + p3 / 4 + 256;
         PB_TRY(dalloc(&h.d_p3_tri, (size_t)cap));
         PB_TRY(dalloc(&h.d_p3_woff, (size_t)cap));
+        PB_TRY(dalloc(&h.d_p3_ref, (size_t)cap));
         h.p3_cap = cap;
     }
     PB_CUDA(cudaMemsetAsync(h.d_corr_mask, 0, sizeof(unsigned) * ((nc + 31) / 32), s));
     fill_pairs3_kernel<<<div_up((long long)n3 * 32, T), T, 0, s>>>(h.d_n3_cell, h.d_n3_start, n3, res, h.d_cell_start, h.d_cell_tris,
-                                                   h.d_p3_tri, h.d_p3_woff, h.d_corr_mask);
+                                                   h.d_p3_tri, h.d_p3_woff, h.d_p3_ref, h.d_corr_mask);
     h.launches++;
     PB_CHECK_LAUNCH();
 

@@ -1359,55 +1359,62 @@ __global__ void __launch_bounds__(256) face_kernel(const __grid_constant__ StepA
 }
 
 // near stage: warps stride over the corrected cells (their number changes with the mesh, the
-// grid does not).  A corrected cell's FDTD-near sum (for the next step) and BEM-near sum are the
-// sums of its pairs' terms (near_terms), lanes striding over the pair list.  prime != 0: only the
-// next step's FDTD-near sum.
+// grid does not), a half warp per cell.  A corrected cell's FDTD-near sum (for the next step) and
+// BEM-near sum are the sums of its pairs' terms (near_terms), lanes striding over the pair list.
+// prime != 0: only the next step's FDTD-near sum.
+// What bounds it: the chain of dependent loads (list bounds, pair index, terms) and the sums over
+// lanes.  A cell has 23 (res 64) to 42 (res 128) pairs, so a whole warp spent half of its lanes or
+// trips on nothing; the pair's triangle and offset come as one index and the two sums share their
+// exchanges.  Alone 3.9 -> 4.1 us (res 64) and 9.5 -> 8.2 (res 128), but beside the other branches and
+// scenes it leaves more room: a motion frame, three scenes in turn, 1256 -> 1183 us and 10.8 -> 10.6 ms.
 template <typename R>
 struct NearArgs
 {
-    const int *n3_cell, *n3_start, *p3_tri;
-    const unsigned char *p3_woff;  // the pair's record offset in 3^3
+    const int *n3_cell, *n3_start;
+    const int *p3_ref;  // per pair: triangle * 27 + record offset in 3^3
     const R *terms;
 };
 
-// the near-stage work of corrected cells warp0, warp0 + nwarps, ... < n3 of one scene
+// the near-stage work of corrected cells 2 warp0, 2 warp0 + 1, 2 (warp0 + nwarps), ... < n3 of one scene
 template <typename R>
 __device__ inline void near_body(const StepArgs &a, const Ring<R> &ring, const StepDyn &dy, const NearArgs<R> &na,
                                  int n3, int warp0, int nwarps, int lane, int prime)
 {
+    using P = typename WRec<R>::P;
     R *cur = ring.slot(dy.tnew), *nextslot = ring.slot(dy.tnew + 1);
-    for (int ci = warp0; ci < n3; ci += nwarps)
+    const int l = lane & 15;
+    const unsigned mask = 0xffffu << (lane & 16);
+    for (int ci = 2 * warp0 + (lane >> 4); ci < n3; ci += 2 * nwarps)
     {
         // the cell and its far-field value are fetched before the pair sums, so their latency
-        // overlaps the term gathers
-        const int c = lane == 0 ? na.n3_cell[ci] : 0;
-        const R far = lane == 0 && !prime ? cur[c] : (R)0;
+        // overlaps the term gathers; lane 0 finishes the FDTD-near sum, lane 8 the BEM-near sum
+        const int c = l == 0 || l == 8 ? na.n3_cell[ci] : 0;
+        const R far = l == 8 && !prime ? cur[c] : (R)0;
         const int b = na.n3_start[ci], e = na.n3_start[ci + 1];
-        R acc_f = 0, acc_b = 0;
-        for (int p = b + lane; p < e; p += 32)
+        R v[2] = {0, 0};
+        for (int p = b + l; p < e; p += 16)
         {
-            const auto t =
-                halves(((const typename WRec<R>::P *)na.terms)[(long long)na.p3_tri[p] * (kGcRecords / 2) + na.p3_woff[p]]);
-            acc_f += t.x;
-            acc_b += t.y;
+            const auto t = halves(((const P *)na.terms)[na.p3_ref[p]]);
+            v[0] += t.x;
+            v[1] += t.y;
         }
-        acc_f = warp_sum(acc_f);
-        if (!prime)
-            acc_b = warp_sum(acc_b);
-        if (lane == 0)
+        const bool up = (l & 8) != 0;
+        R x = (up ? v[1] : v[0]) + __shfl_xor_sync(mask, up ? v[0] : v[1], 8);
+#pragma unroll
+        for (int off = 4; off > 0; off >>= 1)
+            x += __shfl_xor_sync(mask, x, off);
+        if (l == 0)
+            nextslot[c] = x;
+        else if (l == 8 && !prime)
         {
-            nextslot[c] = acc_f;
-            if (!prime)
-            {
-                R v = (R)((double)far + (double)acc_b * 0.98);
-                cur[c] = v;
-                for (int l = 0; l < a.n_listen; l++)
-                    if (a.listen_cell[l] == c)
-                    {
-                        ((R *)dy.series)[dy.row * a.n_listen + l] = v;
-                        flag_nonfinite(a.status, v);
-                    }
-            }
+            const R p = (R)((double)far + (double)x * 0.98);
+            cur[c] = p;
+            for (int i = 0; i < a.n_listen; i++)
+                if (a.listen_cell[i] == c)
+                {
+                    ((R *)dy.series)[dy.row * a.n_listen + i] = p;
+                    flag_nonfinite(a.status, p);
+                }
         }
     }
 }
@@ -1606,8 +1613,7 @@ int make_launch(Handle &h, StepLaunch<R> &L)
         L.fa.status = h.d_step_status;
         L.na.n3_cell = h.d_n3_cell;
         L.na.n3_start = h.d_n3_start;
-        L.na.p3_tri = h.d_p3_tri;
-        L.na.p3_woff = h.d_p3_woff;
+        L.na.p3_ref = h.d_p3_ref;
         L.na.terms = (const R *)h.d_terms;
         L.face_blocks = (int)div_up((long long)h.nt * 32, T);
         if (h.near_blocks <= 0)
