@@ -847,7 +847,11 @@ __global__ void denom_kernel(const int *face_start, int nt, const float *area, c
         }
     }
     if (lane == 0)
-        denom[i] = face_wd ? 0.5 * (double)area[i] - sd : 0.5 * area[i] - sf;
+    {
+        const double d = face_wd ? 0.5 * (double)area[i] - sd : 0.5 * area[i] - sf;
+        denom[i] = d;
+        denom[nt + i] = 1.0 / d;
+    }
 }
 
 DevConsts make_consts(const Handle &h)
@@ -1201,7 +1205,7 @@ static int cache_alloc(Handle &h)
     PB_TRY(dalloc(&h.d_face_interp, (size_t)nt * 8));
     if (h.fp64)
         PB_TRY(dalloc(&h.d_face_interp_d, (size_t)nt * 8));
-    PB_TRY(dalloc(&h.d_face_denom, (size_t)nt));
+    PB_TRY(dalloc(&h.d_face_denom, 2 * (size_t)nt));
     PB_TRY(dalloc(&h.d_tw, (size_t)16));
     twiddle_kernel<<<1, 1, 0, s>>>(h.d_tw);
     h.launches++;

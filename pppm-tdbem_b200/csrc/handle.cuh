@@ -158,7 +158,7 @@ struct Handle
     int *d_face_corner = nullptr;
     float *d_face_interp = nullptr;
     double *d_face_interp_d = nullptr;
-    double *d_face_denom = nullptr;
+    double *d_face_denom = nullptr;  // [2][nt]: denominators, their reciprocals
 
     // ---- persistent caches
     bool gc_empty = true;

@@ -669,7 +669,7 @@ struct FaceArgs
     R *dlast;          // [nt][4]: the Dirichlet values of the last steps, by step of the call mod 4
     R *nfut;           // [nt][4]: N[t+1], N[t+2], N[t+3] of a four-step pass that starts at t
     const float *interp;
-    const double *interp_d, *denom;
+    const double *interp_d, *denom, *rdenom;  // (rdenom: 1 / denom)
     float reflect;
     // near-field terms of every triangle (see near_terms): its 54 grid-cache records
     const typename WRec<R>::T *gc_w;
@@ -1105,12 +1105,14 @@ __device__ inline void face_finish(const Ring<R> &ring, int tnew, const FaceArgs
 #pragma unroll
     for (int m = 1; m < pos; m++)
         d[m] = dlast[(slot - m) & (kPass - 1)];
-    R far_sum = 0;  // corners in order 0..7
+    R far_sum = iw * pv;  // lanes 0..7, a corner each
 #pragma unroll
-    for (int wi = 0; wi < 8; wi++)
-        far_sum += __shfl_sync(kFull, iw, wi) * __shfl_sync(kFull, pv, wi);
-    R num = far_sum * (R)f.reflect + conv;
-    const R dnew = (R)(num / f.denom[tri]);
+    for (int off = 4; off > 0; off >>= 1)
+        far_sum += __shfl_xor_sync(kFull, far_sum, off);
+    far_sum = __shfl_sync(kFull, far_sum, 0);
+    const R num = far_sum * (R)f.reflect + conv;
+    // FP32: by the double reciprocal (off from the quotient by 2^-52 before it is rounded to 24 bits)
+    const R dnew = sizeof(R) == 4 ? (R)(num * f.rdenom[tri]) : (R)(num / f.denom[tri]);
     d[0] = dnew;
     if (commit && lane < 4)
         ring.hat(1, lane, tri, hist_index(lane, tnew)) = dnew;  // lane c: copy c
@@ -1281,8 +1283,10 @@ __global__ void __launch_bounds__(256) fix_kernel(int nt, const __grid_constant_
 // outside every window of this step)
 // (one instantiation per mode: the several-step variants need more registers, which the one-step
 // path should not carry)
+// (mode 3, FP32: at most 64 registers; at 70 its blocks per SM fall from 4 to 3 and a res-128 frame
+// takes 10.80 instead of 10.55 ms)
 template <typename R, int mode>
-__global__ void __launch_bounds__(256) finish_kernel(const __grid_constant__ Ring<R> ring, const StepState *st,
+__global__ void __launch_bounds__(256, mode == 3 && sizeof(R) == 4 ? 4 : 1) finish_kernel(const __grid_constant__ Ring<R> ring, const StepState *st,
                                                       int kstep, int nt, const __grid_constant__ FaceArgs<R> f,
                                                       const R *conv, int next)
 {
@@ -1580,6 +1584,7 @@ int make_launch(Handle &h, StepLaunch<R> &L)
         L.fa.interp = h.d_face_interp;
         L.fa.interp_d = h.fp64 ? h.d_face_interp_d : nullptr;
         L.fa.denom = h.d_face_denom;
+        L.fa.rdenom = h.d_face_denom + h.nt;
         L.fa.reflect = h.prm.reflect_coeff;
         L.fa.gc_w = (const W *)h.d_gc_w;
         L.fa.gc_scale = h.fp64 ? nullptr : h.d_gc_scale;
