@@ -87,3 +87,39 @@ def test_first_steps_on_one_branch(gpu):
         # so they are compared up to there
         assert np.array_equal(out[0][0][:60], out[1][0][:60])
         assert rel_l2(out[0][1], out[1][1]) < 1e-3
+
+
+@pytest.mark.parametrize("n", [1, 3])
+def test_short_calls_replay_their_kernels(gpu, n):
+    """From a handle's 16th call of fewer than four steps on, the call's kernels are replayed as a graph;
+    moved to a new handle every 10 calls (state saved and restored), the same run launches them
+    directly.  Bit-identical."""
+    v, f, h, mn, dt, res, cell = _small()
+    calls = 40
+    acc = sine_acc(calls * n, len(f), 1500.0, dt)
+
+    def new(state=None):
+        s = Solver(res, h, dt, mn)
+        s.set_mesh(v, f)
+        s.add_listener(*cell)
+        if state is not None:
+            s.restore_state(state)
+        return s
+
+    s = new()
+    for k in range(calls):
+        s.step(acc[k * n: (k + 1) * n])
+    a, ga = s.series(), s.grid(0).copy()
+    s.close()
+    s, b = new(), []
+    for k in range(calls):
+        if k and k % 10 == 0:
+            b.append(s.series())
+            state = s.save_state()
+            s.close()
+            s = new(state)
+        s.step(acc[k * n: (k + 1) * n])
+    b.append(s.series())
+    gb = s.grid(0).copy()
+    s.close()
+    assert np.array_equal(a, np.concatenate(b)) and np.array_equal(ga, gb)
