@@ -909,7 +909,11 @@ __device__ inline void near_terms_complete(const FaceArgs<R> &f, int tri, int la
 // before the step begins (Neumann taps t..t-15 with N[t] = acc[t] already in the ring, Dirichlet
 // taps t-1..t-15), so the pipelined step graph runs it beside the stencil.  face_finish: the far
 // field at the 8 trilinear corners (from this step's stencil output), the Dirichlet update and the
-// triangle's near-field terms.  Fused or split, the arithmetic and its order are the same.
+// triangle's near-field terms.
+// Fused (direct launches, the batch's fallback) a warp walks the list alone; the recorded steps and the
+// batch take it by groups of centres, kGroupSplit warps a list (conv_groups).  The sums are associated
+// alike, so a step on its own is the same to the bit on either path: one sum per warp of
+// conv_groups, over that warp's chunks of kChunk neighbours in order, and the warps' totals added in order.
 template <typename R>
 __device__ inline R face_conv(const Ring<R> &ring, int tnew, const FaceArgs<R> &f, int tri, int lane)
 {
@@ -917,22 +921,35 @@ __device__ inline R face_conv(const Ring<R> &ring, int tnew, const FaceArgs<R> &
     using P = typename WRec<R>::P;
     const int g = lane >> 2, q = lane & 3;
     const R *base = ring.hrow(tnew & 3, 0) + window_offset(tnew, q);
-    const int b = f.face_start[tri], e = f.face_start[tri + 1];
-    P acc = make_pair2((R)0, (R)0);
-    for (int p = b + g; p < e; p += 8)
-    {
-        const W4 w4 = *(const W4 *)(f.face_w + (long long)p * kTaps + 4 * q);
-        const P sc = record_scale(f.face_scale, p, (R)0);
-        P h[4], w[4];
-        load_window(base + (long long)f.face_nbr[p] * kHistRow, h);
-        if (q == 0)
-            h[0] = with_y(h[0], (R)0);  // tap 0 of the Dirichlet history is this step's unknown: left out
+    const int e = f.face_start[tri + 1];
+    P acc[kGroupSplit];
 #pragma unroll
-        for (int i = 0; i < 4; i++)
-            w[i] = weight_pair(w4.v[i]);
-        acc = fma2(dot4<R>(w, h), sc, acc);
-    }
-    return warp_sum(pair_sum(acc));
+    for (int w = 0; w < kGroupSplit; w++)
+        acc[w] = make_pair2((R)0, (R)0);
+    for (int p0 = f.face_start[tri] + g; p0 < e; p0 += kGroupSplit * kChunk)
+#pragma unroll
+        for (int o = 0; o < kGroupSplit * kChunk / 8; o++)  // octets of neighbours, one a quad
+        {
+            const int p = p0 + 8 * o;
+            if (p >= e)
+                break;
+            const W4 w4 = *(const W4 *)(f.face_w + (long long)p * kTaps + 4 * q);
+            const P sc = record_scale(f.face_scale, p, (R)0);
+            P h[4], w[4];
+            load_window(base + (long long)f.face_nbr[p] * kHistRow, h);
+            if (q == 0)
+                h[0] = with_y(h[0], (R)0);  // tap 0 of the Dirichlet history is this step's unknown: left out
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                w[i] = weight_pair(w4.v[i]);
+            P &a = acc[o * 8 / kChunk];
+            a = fma2(dot4<R>(w, h), sc, a);
+        }
+    R sum = warp_sum(pair_sum(acc[0]));
+#pragma unroll
+    for (int w = 1; w < kGroupSplit; w++)
+        sum += warp_sum(pair_sum(acc[w]));
+    return sum;
 }
 
 // The face-pair convolution of a group of N centres that share one neighbour list, T = 1, 2 or 4

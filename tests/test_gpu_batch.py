@@ -74,6 +74,30 @@ def test_batch_matches_single_scenes(gpu):
         s.close()
 
 
+@pytest.mark.parametrize("steps", [(1, 1, 1, 1, 1), (3, 2, 1, 2, 3), (2, 50, 3, 1, 21)])
+def test_batch_of_short_runs_matches_single_scenes(gpu, steps):
+    """Runs of one to three steps (a single call of that length launches the fused face stage) beside
+    longer ones, twice in a row: the face-pair sums are associated alike, so still bit-identical."""
+    alone, together = _make(), _make()
+    b = Batch([s for s, _, _ in together])
+    for first in (0, 1):
+        rows = []
+        for (s1, acc, _), n in zip(alone, steps):
+            a = acc[first * n: first * n + n] + np.float32(0.25)  # no zero row: every step's sums count
+            s1.step(a)
+            rows.append(a)
+        b.run(rows)
+    for (s1, _, _), (s2, _, _) in zip(alone, together):
+        assert s1.t == s2.t and np.any(s1.dump("dirichlet"))
+        assert np.array_equal(s1.listeners(), s2.listeners())
+        for rel in (0, -1, -2):
+            assert np.array_equal(s1.grid(rel), s2.grid(rel))
+        assert np.array_equal(s1.dump("dirichlet"), s2.dump("dirichlet"))
+    b.close()
+    for s, _, _ in alone + together:
+        s.close()
+
+
 def test_batch_rejects_bad_sets(gpu):
     s, f, dt = _scene(20, 1, 9)
     with pytest.raises(PPPMError):

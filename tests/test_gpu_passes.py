@@ -123,3 +123,26 @@ def test_short_calls_replay_their_kernels(gpu, n):
     gb = s.grid(0).copy()
     s.close()
     assert np.array_equal(a, np.concatenate(b)) and np.array_equal(ga, gb)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_recorded_single_steps_equal_direct_launches(gpu, precision):
+    """One step per pass, recorded in calls of 13 and 4 steps, against the same steps in calls of one
+    (fused face stage): both sum a triangle's face pairs in the same association.  Bit-identical."""
+    v, f, h, mn, dt, res, cell = _small()
+    acc = sine_acc(34, len(f), 1500.0, dt)
+    out = []
+    for calls in ((13, 4, 17), (1,) * 34):
+        s = Solver(res, h, dt, mn, precision=precision)
+        s.set_option("conv_pairs", 0)
+        s.set_option("terms_pairs", 0)
+        s.set_mesh(v, f)
+        s.add_listener(*cell)
+        at = 0
+        for n in calls:
+            s.step(acc[at: at + n])
+            at += n
+        out.append((s.series(), s.grid(0).copy(), s.grid(-1).copy(), s.dump("dirichlet")))
+        s.close()
+    for a, b in zip(*out):
+        assert np.any(a) and np.array_equal(a, b)
