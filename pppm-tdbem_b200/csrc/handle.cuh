@@ -85,11 +85,11 @@ struct StepGraph
 {
     int nsteps = 0;
     bool open = false;               // a chunk of a longer call (more steps follow; see run_steps)
-    bool plain = false;              // the kernels of direct launches (short calls; see run_steps)
     std::vector<unsigned char> sig;  // the launch set it was recorded with
     cudaGraphExec_t exec = nullptr;
 };
 constexpr int kStepGraphs = 8;
+constexpr int kGraphSteps = 4;  // calls of at least this many steps go in passes (see run_steps)
 
 struct Handle
 {
@@ -243,6 +243,9 @@ struct Handle
     // ---- step launches
     StepState *d_state = nullptr;  // per-call values the step kernels read
     StepGraph graphs[kStepGraphs];
+    // calls of 1 .. kGraphSteps - 1 steps: the kernels of direct launches (see run_steps).  A slot for
+    // each length, so that a program that mixes them with longer calls keeps its kStepGraphs others
+    StepGraph plain_graphs[kGraphSteps - 1];
     StepGraph timing_graph;  // one step with event records between its kernels (measurement mode)
     int graph_next = 0;
     int short_calls = 0;      // calls of fewer than kGraphSteps steps so far (kPlainCalls)

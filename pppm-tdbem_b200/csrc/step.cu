@@ -1927,8 +1927,12 @@ int profile_graph(Handle &h, const StepLaunch<R> &L, cudaGraphExec_t *out)
 // most of the gap between dependent kernels); shorter calls, measurement mode and calls on a
 // stream that the caller is capturing launch the kernels directly.  A program that goes on step by
 // step is bound by the host's launches (about 2 us each): from its kPlainCalls-th short call on a
-// handle replays those kernels too as a graph (plain: the same kernels in the same order).
-constexpr int kGraphSteps = 4;
+// handle replays those kernels too as a graph (plain: the same kernels in the same order, in slots of
+// their own).  Recording one costs 95 us and saves 7 us a queued call (15 -> 8 us at res 32, one step;
+// nothing where the caller waits for every step, 29 us either way), so it pays for itself after
+// 14 calls: a handle that stops before the 16th is not charged for it, one that goes on pays at
+// most twice what the better choice would have cost.  (Recorded at the 2nd call instead, the first 15
+// calls take 312 instead of 270 us, the first 24 567 instead of 547.)
 constexpr int kPlainCalls = 16;
 
 template <typename R>
@@ -1936,20 +1940,20 @@ int graph_for(Handle &h, const StepLaunch<R> &L, int nsteps, cudaGraphExec_t *ou
               bool open = false, bool plain = false)
 {
     const unsigned char *sig = (const unsigned char *)&L;
-    StepGraph *slots = timed ? &h.timing_graph : h.graphs;
-    const int nslots = timed ? 1 : kStepGraphs;
+    StepGraph *slots = timed ? &h.timing_graph : plain ? &h.plain_graphs[nsteps - 1] : h.graphs;
+    const int nslots = timed || plain ? 1 : kStepGraphs;
     for (int i = 0; i < nslots; i++)
     {
         StepGraph &g = slots[i];
-        if (g.exec && g.nsteps == nsteps && g.open == open && g.plain == plain && g.sig.size() == sizeof(L) &&
+        if (g.exec && g.nsteps == nsteps && g.open == open && g.sig.size() == sizeof(L) &&
             memcmp(g.sig.data(), sig, sizeof(L)) == 0)
         {
             *out = g.exec;
             return PPPM_OK;
         }
     }
-    StepGraph &g = timed ? h.timing_graph : h.graphs[h.graph_next];
-    if (!timed)
+    StepGraph &g = slots[nslots == 1 ? 0 : h.graph_next];
+    if (nslots > 1)
         h.graph_next = (h.graph_next + 1) % kStepGraphs;
     if (g.exec)
         cudaGraphExecDestroy(g.exec);
@@ -1978,7 +1982,6 @@ int graph_for(Handle &h, const StepLaunch<R> &L, int nsteps, cudaGraphExec_t *ou
     }
     g.nsteps = nsteps;
     g.open = open;
-    g.plain = plain;
     g.sig.assign(sig, sig + sizeof(L));
     *out = g.exec;
     return PPPM_OK;
@@ -2594,6 +2597,8 @@ int step_free(Handle &h)
         g.sig.clear();
     };
     for (StepGraph &g : h.graphs)
+        release(g);
+    for (StepGraph &g : h.plain_graphs)
         release(g);
     release(h.timing_graph);
     release(h.profile_graph);
