@@ -85,6 +85,7 @@ struct StepGraph
 {
     int nsteps = 0;
     bool open = false;               // a chunk of a longer call (more steps follow; see run_steps)
+    int calls = 0;                   // short calls in a row with this launch set (kPlainCalls)
     std::vector<unsigned char> sig;  // the launch set it was recorded with
     cudaGraphExec_t exec = nullptr;
 };
@@ -248,7 +249,6 @@ struct Handle
     StepGraph plain_graphs[kGraphSteps - 1];
     StepGraph timing_graph;  // one step with event records between its kernels (measurement mode)
     int graph_next = 0;
-    int short_calls = 0;      // calls of fewer than kGraphSteps steps so far (kPlainCalls)
     long long steps_run = 0;  // steps queued so far (kBranchSteps)
     int near_blocks = 0;  // resident grid of the near kernel
     int batch_near_cells = 0;  // corrected cells the batch block map covers (grow-only, step.cu)

@@ -1926,9 +1926,10 @@ int profile_graph(Handle &h, const StepLaunch<R> &L, cudaGraphExec_t *out)
 // first call with that step count and launch set (the graph removes the host launch cost and
 // most of the gap between dependent kernels); shorter calls, measurement mode and calls on a
 // stream that the caller is capturing launch the kernels directly.  A program that goes on step by
-// step is bound by the host's launches (about 2 us each): from its kPlainCalls-th short call on a
-// handle replays those kernels too as a graph (plain: the same kernels in the same order, in slots of
-// their own).  Recording one costs 95 us and saves 7 us a queued call (15 -> 8 us at res 32, one step;
+// step is bound by the host's launches (about 2 us each): from the kPlainCalls-th short call of
+// a length in a row with the same launch set, those kernels are replayed too as a graph (plain: the same
+// kernels in the same order, in slots of their own); where the launch set keeps changing (a moving
+// ghost-cell scene, options set between calls) they stay direct.  Recording one costs 95 us and saves 7 us a queued call (15 -> 8 us at res 32, one step;
 // nothing where the caller waits for every step, 29 us either way), so it pays for itself after
 // 14 calls: a handle that stops before the 16th is not charged for it, one that goes on pays at
 // most twice what the better choice would have cost.  (Recorded at the 2nd call instead, the first 15
@@ -1985,6 +1986,24 @@ int graph_for(Handle &h, const StepLaunch<R> &L, int nsteps, cudaGraphExec_t *ou
     g.sig.assign(sig, sig + sizeof(L));
     *out = g.exec;
     return PPPM_OK;
+}
+
+// whether a short call is at least the kPlainCalls-th of its length in a row with this launch set
+template <typename R>
+bool plain_due(Handle &h, const StepLaunch<R> &L, int nsteps)
+{
+    const unsigned char *sig = (const unsigned char *)&L;
+    StepGraph &g = h.plain_graphs[nsteps - 1];
+    if (g.sig.size() != sizeof(L) || memcmp(g.sig.data(), sig, sizeof(L)) != 0)
+    {
+        if (g.exec)
+            cudaGraphExecDestroy(g.exec);
+        g.exec = nullptr;
+        g.sig.assign(sig, sig + sizeof(L));
+        g.calls = 0;
+    }
+    g.calls = std::min(g.calls + 1, kPlainCalls);
+    return g.calls >= kPlainCalls;
 }
 
 template <typename R>
@@ -2111,19 +2130,23 @@ int run_steps(Handle &h, const float *acc_dev, int nsteps)
             h.launches += (chunks + 1) + (4 + (L.split && !L.linear) - per_step) * (long long)nsteps;
         h.launches += chunks;
     }
-    else if (cs == cudaStreamCaptureStatusNone && ++h.short_calls >= kPlainCalls)
-    {
-        L.linear = 0;  // no part of these kernels: keeps the launch set the same
-        cudaGraphExec_t exec = nullptr;
-        PB_TRY(graph_for<R>(h, L, nsteps, &exec, false, false, true));
-        PB_CUDA(cudaGraphLaunch(exec, s));
-    }
     else
-        for (int k = 0; k < nsteps; k++)
+    {
+        // (no part of these kernels: keeps the launch set the same)
+        L.linear = L.split = L.pairs = L.tpairs = L.fix_groups = L.face_threads = 0;
+        if (cs == cudaStreamCaptureStatusNone && plain_due<R>(h, L, nsteps))
         {
-            launch_step<R>(L, k, s, nullptr);
-            PB_CHECK_LAUNCH();
+            cudaGraphExec_t exec = nullptr;
+            PB_TRY(graph_for<R>(h, L, nsteps, &exec, false, false, true));
+            PB_CUDA(cudaGraphLaunch(exec, s));
         }
+        else
+            for (int k = 0; k < nsteps; k++)
+            {
+                launch_step<R>(L, k, s, nullptr);
+                PB_CHECK_LAUNCH();
+            }
+    }
     h.launches += per_step * nsteps;
     if (L.ghost)
     {

@@ -177,3 +177,34 @@ def test_short_calls_keep_the_recorded_graphs(gpu):
         best.append(min(times[20:]))
         s.close()
     assert best[1] < 5 * best[0], best
+
+
+def test_short_calls_with_changing_launches_stay_direct(gpu):
+    """One-step calls whose launch set changes from call to call (here by options, 24 sets in turn; a moving
+    ghost-cell scene does so at every frame) are not recorded again and again: they cost direct launches
+    (less than twice the replayed ones); recorded in every call they took eight times as long."""
+    import itertools
+    import time
+
+    import torch
+
+    v, f, h, mn, dt, res, cell = _small()
+    acc = torch.from_numpy(sine_acc(24, len(f), 1500.0, dt)).cuda()
+    best = []
+    sets = list(itertools.product((0, 1), (0, 1), (64, 128, 256), (0, 1)))
+    for change in (False, True):
+        s = Solver(res, h, dt, mn)
+        s.set_mesh(v, f)
+        times = []
+        for cycle in range(30):
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            for k in range(len(sets)):
+                for name, value in zip(("conv_pairs", "terms_pairs", "face_threads", "stencil_vec4"), sets[k * change]):
+                    s.set_option(name, value)
+                s.step(acc[k: k + 1])
+            torch.cuda.synchronize()
+            times.append(time.perf_counter() - t0)
+        best.append(min(times[10:]))
+        s.close()
+    assert best[1] < 5 * best[0], best
