@@ -53,8 +53,10 @@ struct StepArgs
     int *status;  // the handle's step status word: kStepNonFinite once a listener sample is not finite
 };
 
-// pairs (capacity of the lists) from which the completion of the convolution goes by groups of centres
-constexpr long long kManyPairs = 1500000;
+// triangles and pairs (capacity of the lists) from which the completion of the convolution goes by
+// groups of centres (make_launch)
+constexpr int kManyTriangles = 15000;
+constexpr long long kManyPairs = 1250000;
 
 // Steps of a recorded call go in passes that stream the face pairs and the grid-cache records once
 // for several steps: four while a further step of the call follows, then pairs, then one.
@@ -1608,11 +1610,17 @@ int make_launch(Handle &h, StepLaunch<R> &L)
         L.fa.terms = (R *)h.d_terms;
         L.conv = (R *)h.d_conv;
         L.conv_blocks = conv_blocks(h.nt);
-        // By group the completion shares its gathers and index loads, by triangle it has twice the
-        // warps to hide them: 480 k pairs (in L2) 5.7 us by triangle, 6.2 by group for a pass's last
-        // step; 6.0 M pairs (from memory) 31.7 and 22.0.  By the list arrays' capacity, which only
-        // grows, so that the choice does not flicker from frame to frame.  Same sums.
-        L.fix_groups = h.pf_cap >= kManyPairs ? 1 : 0;
+        // By group the completion shares its gathers and index loads, by triangle it has twice the warps
+        // to hide them: groups pay where half a warp per triangle still fills the GPU (9472 warps) and the
+        // lists are long.  One step in a call of 128, by triangle and by group:
+        //    5120 triangles, 0.14 / 0.60 / 1.51 M pairs   13.6, 14.2   16.9, 19.7   27.5, 34.4 us
+        //   10240            0.28 / 1.21                  23.0, 23.5   27.5, 29.3
+        //   15360            0.42 / 1.80                  38.9, 39.5   37.4, 37.2
+        //   20480            0.56 / 1.36 / 2.41           63.1, 63.6   42.3, 41.5   50.2, 48.9
+        //   40960            2.71 / 4.82                  88.4, 86.3  105.2, 103.1
+        // By the list arrays' capacity, which only grows, so that the choice does not flicker from frame
+        // to frame.  Same sums.
+        L.fix_groups = h.nt >= kManyTriangles && h.pf_cap >= kManyPairs ? 1 : 0;
         L.pairs = h.conv_pairs;
         L.face_threads = h.face_threads;
         L.tpairs = h.terms_pairs ? 1 : 0;
@@ -2727,6 +2735,9 @@ __global__ void __launch_bounds__(kConvThreads, sizeof(R) == 4 ? 16 : 1) batch_c
     const PassAt p = batch_pass(*S.st, tnew);
     if (p.pos)
     {
+        // (by groups whatever the scene's size: other scenes' blocks hide the loads and fewer warps are
+        // left to them.  By triangle as alone, batches of 8 scenes of 0 to 1.3 M pairs 15.0 against 14.1 ms,
+        // of 8 small ones 8.21 against 7.82, of 2 of 50 k pairs 2.63 against 2.59)
         const int w = m.y * kGroupSplit + (int)(threadIdx.x >> 5), nw = conv_blocks(nt) * kGroupSplit;
         const int lane = threadIdx.x & 31, slot = (tnew - 1 - S.st->pair0) & (kPass - 1);
         if (p.pos == 1)

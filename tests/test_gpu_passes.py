@@ -13,9 +13,9 @@ from pppm_b200 import Solver, scenes
 pytestmark = pytest.mark.gpu
 
 
-def _run(geom, many, calls, chunk=32):
+def _run(geom, many, calls, chunk=32, precision="fp64"):
     v, f, h, mn, dt, res, cell = geom
-    s = Solver(res, h, dt, mn, precision="fp64")
+    s = Solver(res, h, dt, mn, precision=precision)
     s.set_option("conv_pairs", many[0])
     s.set_option("terms_pairs", many[1])
     s.set_option("graph_chunk", chunk)
@@ -51,18 +51,34 @@ def test_passes_match_single_steps(gpu, many, calls, chunk):
     assert rel_l2(b, a) < 1e-12 and rel_l2(gb, ga) < 1e-12 and rel_l2(db, da) < 1e-12
 
 
-def test_dense_scene_completes_by_groups(gpu):
-    """5120 triangles in a res-24 grid: more pairs than the threshold from which the completion of the
-    convolution takes a group of centres per warp (capacity 5/4 of the pairs)."""
+def _dense(sub, res, precision):
+    """A dense scene in passes against one pass per step.  FP32: the sums in another order, below 1e-6 over
+    so few steps (as test_pairs_match_single_pass_fp32)."""
     rng = np.random.default_rng(3)
-    v, f = scenes.perturbed_sphere(4, 0.1, 0.1, rng)
-    h, mn = scenes.grid_for_bbox(v.min(0), v.max(0), 24, 2.0)
+    v, f = scenes.perturbed_sphere(sub, 0.1, 0.1, rng)
+    h, mn = scenes.grid_for_bbox(v.min(0), v.max(0), res, 2.0)
     dt = np.float32(0.5 * h / (np.sqrt(3) * 340.3))
-    geom = (v.astype(np.float32), f, h, mn, dt, 24, (12, 12, 20))
-    (a, ga, da), counts = _run(geom, (0, 0), (22,))
-    (b, gb, db), _ = _run(geom, (1, 1), (22,))
-    assert counts[4] * 5 // 4 > 1500000
-    assert rel_l2(b, a) < 1e-12 and rel_l2(gb, ga) < 1e-12 and rel_l2(db, da) < 1e-12
+    geom = (v.astype(np.float32), f, h, mn, dt, res, (res // 2, res // 2, res - 4))
+    (a, ga, da), counts = _run(geom, (0, 0), (22,), precision=precision)
+    (b, gb, db), _ = _run(geom, (1, 1), (22,), precision=precision)
+    tol = 1e-12 if precision == "fp64" else 1e-6
+    assert rel_l2(b, a) < tol and rel_l2(gb, ga) < tol and rel_l2(db, da) < tol
+    return len(f), counts[4] * 5 // 4  # pairs: the lists have a quarter to spare
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_dense_scene_completes_by_groups(gpu, precision):
+    """20480 triangles in a res-56 grid, 3.6 M pairs: more triangles and pairs than the thresholds from
+    which the completion of the convolution takes a group of centres per warp (step.cu: make_launch)."""
+    nt, pairs = _dense(5, 56, precision)
+    assert nt >= 15000 and pairs >= 1250000
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_dense_scene_completes_by_triangle(gpu, precision):
+    """5120 triangles in a res-24 grid, 1.3 M pairs: as many pairs, too few triangles for groups."""
+    nt, pairs = _dense(4, 24, precision)
+    assert nt < 15000 and pairs >= 1250000
 
 
 def test_first_steps_on_one_branch(gpu):
