@@ -249,7 +249,7 @@ struct Handle
     StepGraph plain_graphs[kGraphSteps - 1];
     StepGraph timing_graph;  // one step with event records between its kernels (measurement mode)
     int graph_next = 0;
-    long long steps_run = 0;  // steps queued so far (kBranchSteps)
+    long long steps_run = 0;  // steps queued so far (branch_steps)
     int near_blocks = 0;  // resident grid of the near kernel
     int batch_near_cells = 0;  // corrected cells the batch block map covers (grow-only, step.cu)
 

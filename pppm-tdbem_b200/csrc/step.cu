@@ -1695,9 +1695,20 @@ void launch_step(const StepLaunch<R> &L, int k, cudaStream_t s, Handle *timed)
 // much again when it is destroyed, 2 us a kernel otherwise: 4.9 against 1.9 ms for the first 96 steps of a
 // new scene, and 3.5 ms less when it is closed.  A handle's first steps therefore replay graphs of
 // one branch (capture_pipelined with L.linear: the same kernels one after another as dependent
-// launches, the stencil unsplit; same results), which run 3 (res 27) to 5 us a step (res 64) slower,
-// and the branched graphs are recorded once a handle has this many steps behind or before it.
+// launches, the stencil unsplit; same results), and the branched graphs are recorded once a handle has
+// branch_steps steps behind or before it: where the time that the branches save, which grows with the
+// work that can run beside, has made up for recording and destroying them.
+// Time saved a step, and steps until recording (1.1 to 1.8 ms) and destroying (1.3 to 3.1 ms) are paid back:
+//   res 27, 320 triangles   2.7 us, 1000    res 48, 1280   3.2 us, 900    res 96, 5120   4.3 us, 750
+//   res 64, 6400 (480 k pairs)  5.5 us, 650    res 128, 40960 (6.0 M pairs)  17 us, 180
+// branch_steps gives 1000, 920, 530, 590 and 110.  The first 1000 steps of a handle at res 128 take 93 ms;
+// on one branch throughout 104.  (By the capacity of the pair list, which only grows.)
 constexpr long long kBranchSteps = 1024;
+
+long long branch_steps(const Handle &h)
+{
+    return kBranchSteps * 1000000 / (1000000 + h.pf_cap + h.n_cells);
+}
 
 // The kernels of nsteps steps as a multi-branch graph (absorbing boundary with a mesh).  Per step:
 //   side   conv(k)                       after finish(k-1): needs D[t-1] and N[t]
@@ -2029,7 +2040,7 @@ int run_steps(Handle &h, const float *acc_dev, int nsteps)
     PB_CHECK_LAUNCH();
     StepLaunch<R> L;
     PB_TRY(make_launch<R>(h, L));
-    L.linear = h.steps_run + nsteps < kBranchSteps ? 1 : 0;
+    L.linear = h.steps_run + nsteps < branch_steps(h) ? 1 : 0;
     h.steps_run += nsteps;
     const long long per_step = 1 + (h.mesh_set ? 2 : 0);
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;

@@ -13,9 +13,9 @@ from pppm_b200 import Solver, scenes
 pytestmark = pytest.mark.gpu
 
 
-def _run(geom, many, calls, chunk=32, precision="fp64"):
+def _run(geom, many, calls, chunk=32, precision="fp64", pml=0):
     v, f, h, mn, dt, res, cell = geom
-    s = Solver(res, h, dt, mn, precision=precision)
+    s = Solver(res, h, dt, mn, precision=precision, pml_width=pml)
     s.set_option("conv_pairs", many[0])
     s.set_option("terms_pairs", many[1])
     s.set_option("graph_chunk", chunk)
@@ -51,6 +51,15 @@ def test_passes_match_single_steps(gpu, many, calls, chunk):
     assert rel_l2(b, a) < 1e-12 and rel_l2(gb, ga) < 1e-12 and rel_l2(db, da) < 1e-12
 
 
+@pytest.mark.parametrize("many", [(1, 1), (1, 0), (0, 1)])
+@pytest.mark.parametrize("calls", [(4, 5, 6, 7), (41, 2, 15, 1)])
+def test_pml_passes_match_single_steps(gpu, many, calls):
+    (a, ga, da), _ = _run(_small(), (0, 0), calls, pml=4)
+    (b, gb, db), _ = _run(_small(), many, calls, pml=4)
+    assert np.all(np.isfinite(b)) and np.abs(b).max() > 0
+    assert rel_l2(b, a) < 1e-12 and rel_l2(gb, ga) < 1e-12 and rel_l2(db, da) < 1e-12
+
+
 def _dense(sub, res, precision):
     """A dense scene in passes against one pass per step.  FP32: the sums in another order, below 1e-6 over
     so few steps (as test_pairs_match_single_pass_fp32)."""
@@ -81,28 +90,36 @@ def test_dense_scene_completes_by_triangle(gpu, precision):
     assert nt < 15000 and pairs >= 1250000
 
 
-def test_first_steps_on_one_branch(gpu):
-    """A handle's first steps replay one-branch graphs, later ones (1024 steps behind or before the
-    handle) branched graphs with the split stencil: the same run in short calls and in one long call,
-    absorbing boundary and PML, FP32, bit-identical where both go in passes from the same step."""
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("pml", [0, 4])
+def test_first_steps_on_one_branch(gpu, pml, precision):
+    """A handle's first steps replay one-branch graphs, later ones (step.cu: branch_steps, at most 1024 steps
+    behind or before the handle) branched graphs with the split stencil.  The same calls on a new handle and
+    on one that has 1100 steps behind it and was set back to rest, absorbing boundary and PML: every sample
+    and the whole state (grids, auxiliary fields, histories) bit-identical."""
     v, f, h, mn, dt, res, cell = _small()
-    acc = sine_acc(1280, len(f), 1500.0, dt)
-    for pml in (0, 4):
-        out = []
-        for calls in ((64,) * 20, (1280,)):
-            s = Solver(res, h, dt, mn, pml_width=pml)
-            s.set_mesh(v, f)
-            s.add_listener(*cell)
-            at = 0
-            for n in calls:
-                s.step(acc[at: at + n])
-                at += n
-            out.append((s.series()[:64], s.grid(0).copy()))
-            s.close()
-        # the first call's 64 steps: its last four go in pairs in one run and as a pass in the other,
-        # so they are compared up to there
-        assert np.array_equal(out[0][0][:60], out[1][0][:60])
-        assert rel_l2(out[0][1], out[1][1]) < 1e-3
+    calls = (64, 37, 100, 9, 4, 33, 70, 5)
+    acc = sine_acc(1100, len(f), 1500.0, dt)
+    out = []
+    for before in (0, 1100):
+        s = Solver(res, h, dt, mn, pml_width=pml, precision=precision)
+        s.set_mesh(v, f)
+        s.add_listener(*cell)
+        if before:
+            s.step(acc[:before])
+            s.reset_fields()
+            s.rewind_listeners()
+            s.t = -1
+        at = 0
+        for n in calls:
+            s.step(acc[at: at + n])
+            at += n
+        out.append((s.series(0, at), s.grid(0).copy(), s.grid(-1).copy(), s.grid(-2).copy(), s.dump("dirichlet"),
+                    s.dump("neumann"), np.frombuffer(s.save_state(), np.uint8)))
+        s.close()
+    assert np.all(np.isfinite(out[0][0]))
+    for a, b in zip(*out):
+        assert np.any(a) and np.array_equal(a, b)
 
 
 @pytest.mark.parametrize("n", [1, 3])
@@ -141,15 +158,16 @@ def test_short_calls_replay_their_kernels(gpu, n):
     assert np.array_equal(a, np.concatenate(b)) and np.array_equal(ga, gb)
 
 
+@pytest.mark.parametrize("pml", [0, 4])
 @pytest.mark.parametrize("precision", ["fp32", "fp64"])
-def test_recorded_single_steps_equal_direct_launches(gpu, precision):
+def test_recorded_single_steps_equal_direct_launches(gpu, precision, pml):
     """One step per pass, recorded in calls of 13 and 4 steps, against the same steps in calls of one
     (fused face stage): both sum a triangle's face pairs in the same association.  Bit-identical."""
     v, f, h, mn, dt, res, cell = _small()
     acc = sine_acc(34, len(f), 1500.0, dt)
     out = []
     for calls in ((13, 4, 17), (1,) * 34):
-        s = Solver(res, h, dt, mn, precision=precision)
+        s = Solver(res, h, dt, mn, precision=precision, pml_width=pml)
         s.set_option("conv_pairs", 0)
         s.set_option("terms_pairs", 0)
         s.set_mesh(v, f)
