@@ -212,23 +212,31 @@ def algorithmic_bytes(counts, res, nt):
     # its two history windows 2 x 64 (read once whatever the number of pairs naming it), sum out
     conv = pf * 76 + nt * (8 + 128 + 4 + 4)
     conv2 = pf * 76 + nt * (8 + 128 + 4 + 4 + 8)  # + next acceleration row, second sum
-    fix = pf * 8 + nt * 20  # per pair tap-1 factor and neighbour; per triangle start, D, sums
+    conv4 = pf * 76 + nt * (8 + 128 + 4 + 4 + 24)  # + three acceleration rows, three more sums
+    # completion of a pass's later steps: per pair one, two or three tap factors and the neighbour; per
+    # triangle start, the D values, sums
+    fix = pf * 8 + nt * 20
+    fix4b = pf * 12 + nt * 24
+    fix4 = pf * 16 + nt * 28
     # per triangle: 8 corners (interp weight, cell index, far value), conv sum, denominator,
     # 4 Dirichlet copies + last D, own N and D windows, 54 grid-cache records (64 + 8), 54 terms
     # written, next Neumann value (4 copies) from the acceleration row
     corners = 8 * (4 + 4 + 4)
     finish = nt * (corners + 4 + 8 + 20 + 128 + 54 * 72 + 54 * 4 + 20)
     finish1 = finish + nt * (54 * 4 + 4)  # + partial terms of the next step
-    finish2 = nt * (corners + 4 + 8 + 20 + 3 * 54 * 4 + 20)  # terms from partials and factors
-    near = p3 * (4 + 1 + 8) + n3 * (4 + 4 + 4 + 4 + 4 + 4)
+    finish4 = finish + nt * 3 * (54 * 4 + 4)  # + partial terms of the next three steps
+    # terms from partials and one, two or three factors
+    finish2, finish4b, finish4c = (nt * (corners + 4 + 8 + 20 + (2 + j) * 54 * 4 + 20) for j in (1, 2, 3))
+    near = p3 * (4 + 8) + n3 * (4 + 4 + 4 + 4 + 4 + 4)
     nwrite = nt * 20
     face = pf * 76 + nt * (8 + 4) + finish
     # the split stencil: the corrected cells (list index, p^t, p^{t-1}, the correction, p^{t+1}) and
     # the rest of the grid (as the whole stencil without the corrected cells)
     stencil_corr = n3 * (4 + 12 + 4)
     stencil_bulk = 12 * (m ** 3 - n3) + 4 * 6 * m * m + m ** 3 // 8
-    return {"stencil": stencil, "conv": conv, "conv2": conv2, "fix": fix, "finish": finish, "finish1": finish1,
-            "finish2": finish2, "near": near, "nwrite": nwrite, "face": face, "stencil_corr": stencil_corr,
+    return {"stencil": stencil, "conv": conv, "conv2": conv2, "conv4": conv4, "fix": fix, "fix4b": fix4b, "fix4": fix4,
+            "finish": finish, "finish1": finish1, "finish2": finish2, "finish4": finish4, "finish4b": finish4b,
+            "finish4c": finish4c, "near": near, "nwrite": nwrite, "face": face, "stencil_corr": stencil_corr,
             "stencil_bulk": stencil_bulk}
 
 
@@ -302,7 +310,7 @@ def run_ours(args, ws, rank, local):
         s.add_listener(*wl.listener)
         return s
 
-    # face-stage autotuner on the first frame's mesh (set-up, untimed): one or two steps per pass
+    # face-stage autotuner on the first frame's mesh (set-up, untimed): one or several steps per pass
     # over the face pairs and over the grid-cache records, block size of the face kernels
     s0 = new_solver()
     if args.profile_frame is not None:
@@ -452,7 +460,8 @@ def run_ours(args, ws, rank, local):
     top = next(iter(kernels))
     traffic = load_traffic(args.workload).get(top)
     prof = {k: (per[k], prof[k][1]) for k in per}
-    main_path = [k for k in ("stencil", "stencil_corr", "finish", "finish1", "finish2", "near") if k in kernels]
+    main_path = [k for k in ("stencil", "stencil_corr", "finish", "finish1", "finish2", "finish4", "finish4b",
+                               "finish4c", "near") if k in kernels]
     path_bytes = sum(kind_bytes.get(k, 0.0) for k in main_path)
     path_us = sum(prof[k][0] * prof[k][1] for k in main_path)
 
@@ -570,11 +579,11 @@ def run_ours(args, ws, rank, local):
                      "kernels": kernels,
                      "main_path": {"kernels": main_path, "achieved": round(path_bytes / (path_us * 1e-6) / 1e9, 1),
                                    "frac": round(path_bytes / (path_us * 1e-6) / 1e9 / peak, 4)},
-                     "autotune": {"best": {"two_steps_per_pass": bool(opts["conv_pairs"]),
+                     "autotune": {"best": {"several_steps_per_pass": bool(opts["conv_pairs"]),
                                            "threads": opts["face_threads"],
-                                           "terms_two_steps_per_pass": bool(opts["terms_pairs"])},
-                                  "step_us_by_config": {"%s/%d/%s" % (("single", "pairs")[p], t,
-                                                                      "terms2" if m else "terms1"): round(u, 2)
+                                           "terms_several_steps_per_pass": bool(opts["terms_pairs"])},
+                                  "step_us_by_config": {"%s/%d/%s" % (("single", "passes")[p], t,
+                                                                      "termsN" if m else "terms1"): round(u, 2)
                                                         for (p, t, m), u in (tune["step_us"] or {}).items()}},
                      "update_mesh_us": round(us_update, 1), "time_step_us": round(us_per_step, 2)},
         "cpu_baseline": cpu, "e2e": e2e, "gpu_launches": int(launches), "clocks": clk,

@@ -340,19 +340,20 @@ int pppm_launch_count(pppm_handle *h, long long *count);
 int pppm_enable_timing(pppm_handle *h, int enable);
 int pppm_kernel_times(pppm_handle *h, float *us_stencil, float *us_face, float *us_near, int *timed_steps);
 /* No counterpart in the reference.  Measurement mode per kernel: where the recorded step graphs
- * run the split face stage (absorbing boundary, PPPM method, mesh set), steps in measurement mode
+ * run the split face stage (PPPM method, mesh set), steps in measurement mode
  * go in groups of four through a recorded graph of exactly those kernels (Neumann write, then per
- * step the face-pair convolution, the stencil, finish, near), serialised on the handle's stream
+ * step the face-pair convolution or its completion, the stencil, finish, near; the passes are the
+ * call's: four steps, at its end pairs), serialised on the handle's stream
  * with an event between consecutive kernels; remaining steps and other handles time the fused
  * kernels.  Per kind: us_per_launch[k] = mean event-to-event time of its launches, launches[k]
  * their number (both arrays of nkinds entries, nkinds <= PPPM_KERNEL_KINDS). */
 #define PPPM_KERNEL_STENCIL 0 /* FDTD / absorbing-boundary stencil (or the PML stencil)       */
 #define PPPM_KERNEL_CONV 1    /* face-pair convolution, one step per pass                    */
 #define PPPM_KERNEL_CONV2 2   /* face-pair convolution, two steps per pass                   */
-#define PPPM_KERNEL_FIX 3     /* completion of the second step of a two-step pass            */
+#define PPPM_KERNEL_FIX 3     /* completion of the second step of a pass                     */
 #define PPPM_KERNEL_FINISH 4  /* far field, Dirichlet update, near-field terms in one pass    */
 #define PPPM_KERNEL_FINISH1 5 /* ... first step of a two-step pass over the grid-cache records */
-#define PPPM_KERNEL_FINISH2 6 /* ... second step (completion of its terms)                    */
+#define PPPM_KERNEL_FINISH2 6 /* ... second step of a pass (completion of its terms)          */
 #define PPPM_KERNEL_NEAR 7    /* corrected cells: sums of the near-field terms                */
 #define PPPM_KERNEL_NWRITE 8  /* Neumann history write of a call's first step                 */
 #define PPPM_KERNEL_FACE 9    /* the fused face stage of direct launches                      */
@@ -364,7 +365,9 @@ int pppm_kernel_times(pppm_handle *h, float *us_stencil, float *us_face, float *
 #define PPPM_KERNEL_FIX4 14    /* completion of the last step of a four-step pass              */
 #define PPPM_KERNEL_FINISH4 15 /* finish, first step of a four-step pass over the records      */
 #define PPPM_KERNEL_FINISH4C 16 /* ... its last step (completion of its terms)                 */
-#define PPPM_KERNEL_KINDS 17
+#define PPPM_KERNEL_FIX4B 17   /* completion of the third step of a four-step pass             */
+#define PPPM_KERNEL_FINISH4B 18 /* ... finish of its third step (completion of its terms)      */
+#define PPPM_KERNEL_KINDS 19
 int pppm_kernel_profile(pppm_handle *h, int nkinds, float *us_per_launch, long long *launches);
 /* No counterpart in the reference.  Duration of each step kernel kind on the current mesh and
  * state: reps back-to-back launches of the kind (those of the next step) recorded as one CUDA

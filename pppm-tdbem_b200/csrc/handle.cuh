@@ -237,9 +237,14 @@ struct Handle
     // stencil, finish, near), end
     static constexpr int kProfileEvents = 3 + 5 * kProfileSteps;
     cudaEvent_t evk[kProfileEvents] = {};
-    int evk_kind[kProfileEvents] = {};
-    int evk_used = 0;  // event marks of the recorded profile graph
-    StepGraph profile_graph;  // kProfileSteps split-stage steps with events between the kernels
+    // kProfileSteps recorded steps with events between the kernels: [0] a call's last steps, [1] steps
+    // that others of their call follow
+    struct StepProfile
+    {
+        StepGraph graph;
+        int kind[kProfileEvents] = {};  // the kernel between events i and i + 1
+        int used = 0;                   // events
+    } profile[2];
 
     // ---- step launches
     StepState *d_state = nullptr;  // per-call values the step kernels read

@@ -1854,15 +1854,30 @@ void capture_pipelined(Handle &h, const StepLaunch<R> &L, int nsteps, bool pair,
 
 __global__ void empty_kernel() {}
 
+// the kinds (PPPM_KERNEL_*) of a step's convolution or completion, and of its finish
+inline int conv_kind(PassAt p)
+{
+    if (p.pos)
+        return p.pos == 1 ? PPPM_KERNEL_FIX : p.pos == 2 ? PPPM_KERNEL_FIX4B : PPPM_KERNEL_FIX4;
+    return p.size == kPass ? PPPM_KERNEL_CONV4 : p.size == 2 ? PPPM_KERNEL_CONV2 : PPPM_KERNEL_CONV;
+}
+inline int finish_kind(int mode)
+{
+    constexpr int kinds[7] = {PPPM_KERNEL_FINISH,  PPPM_KERNEL_FINISH1, PPPM_KERNEL_FINISH2, PPPM_KERNEL_FINISH4,
+                              PPPM_KERNEL_FINISH2, PPPM_KERNEL_FINISH4B, PPPM_KERNEL_FINISH4C};
+    return kinds[mode];
+}
+
 // Measurement mode per kernel: the kernels of Handle::kProfileSteps steps exactly as
-// capture_pipelined issues them for a call of that many steps, but serialised on the handle's
-// stream with an event record between consecutive kernels; evk_kind[i] names the kind of the
-// kernel between events i and i + 1.  (A call of kProfileSteps = 4 steps goes in pairs.)
+// capture_pipelined issues them, but serialised on the handle's stream with an event record between
+// consecutive kernels; kind[i] names the kernel between events i and i + 1.  open: steps of a longer call
+// (a pass of four); otherwise a call's last four steps (two pairs).
 template <typename R>
-int profile_graph(Handle &h, const StepLaunch<R> &L, cudaGraphExec_t *out)
+int profile_graph(Handle &h, const StepLaunch<R> &L, bool open, cudaGraphExec_t *out)
 {
     const unsigned char *sig = (const unsigned char *)&L;
-    StepGraph &g = h.profile_graph;
+    Handle::StepProfile &prof = h.profile[open ? 1 : 0];
+    StepGraph &g = prof.graph;
     if (g.exec && g.sig.size() == sizeof(L) && memcmp(g.sig.data(), sig, sizeof(L)) == 0)
     {
         *out = g.exec;
@@ -1873,6 +1888,7 @@ int profile_graph(Handle &h, const StepLaunch<R> &L, cudaGraphExec_t *out)
     g.exec = nullptr;
     const int T = 256, nt = L.a.nt, n = Handle::kProfileSteps;
     const bool pair = L.pairs != 0;
+    const long long total = open ? n + (1ll << 40) : n;
     cudaStream_t s = h.stream;
     int e = 0;
     bool overflow = false;
@@ -1882,19 +1898,19 @@ int profile_graph(Handle &h, const StepLaunch<R> &L, cudaGraphExec_t *out)
             overflow = true;
             return;
         }
-        h.evk_kind[e] = kind;
+        prof.kind[e] = kind;
         cudaEventRecordWithFlags(h.evk[e++], s, cudaEventRecordExternal);
     };
     cudaGraph_t graph = nullptr;
     PB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     mark(PPPM_KERNEL_NWRITE);
-    nwrite_kernel<R><<<div_up(nt, T), T, 0, s>>>(L.ring, L.st, 0, nt, L.fa, neumann_needs(0, n, pair));
+    nwrite_kernel<R><<<div_up(nt, T), T, 0, s>>>(L.ring, L.st, 0, nt, L.fa, neumann_needs(0, total, pair));
     mark(PPPM_KERNEL_EMPTY);
     empty_kernel<<<1, 32, 0, s>>>();
     for (int k = 0; k < n; k++)
     {
-        const PassAt p = pass_at(k, n, pair);
-        mark(p.pos ? PPPM_KERNEL_FIX : p.size > 1 ? PPPM_KERNEL_CONV2 : PPPM_KERNEL_CONV);
+        const PassAt p = pass_at(k, total, pair);
+        mark(conv_kind(p));
         launch_conv<R>(L, k, p, s);
         if (L.split)
         {
@@ -1908,11 +1924,14 @@ int profile_graph(Handle &h, const StepLaunch<R> &L, cudaGraphExec_t *out)
         else
         {
             mark(PPPM_KERNEL_STENCIL);
-            stencil_kernel<R><<<L.sp.nb_bd + L.sp.nb_in, T, 0, s>>>(L.a, L.ring, L.st, k, L.sp, L.corr_mask);
+            if (L.pml)
+                pml_kernel<R><<<dim3(L.pml_blocks, L.a.res - 2), T, 0, s>>>(L.a, L.ring, L.st, k, L.corr_mask, 0);
+            else
+                stencil_kernel<R><<<L.sp.nb_bd + L.sp.nb_in, T, 0, s>>>(L.a, L.ring, L.st, k, L.sp, L.corr_mask);
         }
-        const int mode = finish_mode(k, n, L.tpairs != 0);
-        mark(mode == 1 ? PPPM_KERNEL_FINISH1 : mode == 2 ? PPPM_KERNEL_FINISH2 : PPPM_KERNEL_FINISH);
-        launch_finish<R>(L, k, mode, p.pos, k + 1 < n ? neumann_needs(k + 1, n, pair) : 0, s, false);
+        const int mode = finish_mode(k, total, L.tpairs != 0);
+        mark(finish_kind(mode));
+        launch_finish<R>(L, k, mode, p.pos, k + 1 < n ? neumann_needs(k + 1, total, pair) : 0, s, false);
         mark(PPPM_KERNEL_NEAR);
         near_kernel<R><<<L.near_blocks, T, 0, s>>>(L.a, L.ring, L.st, k, L.na, 0);
     }
@@ -1922,7 +1941,7 @@ int profile_graph(Handle &h, const StepLaunch<R> &L, cudaGraphExec_t *out)
         err = cudaGraphInstantiate(&g.exec, graph, 0);
     if (graph)
         cudaGraphDestroy(graph);
-    h.evk_used = overflow ? 0 : e;
+    prof.used = overflow ? 0 : e;
     if (overflow)
     {
         g.exec = nullptr;
@@ -2048,30 +2067,33 @@ int run_steps(Handle &h, const float *acc_dev, int nsteps)
     if (h.timing && cs == cudaStreamCaptureStatusNone)
     {
         // Measurement mode.  Where the recorded graphs run the split face stage, groups of
-        // kProfileSteps steps replay the profile graph (those kernels serialised, events between
+        // kProfileSteps steps replay the profile graphs (the call's kernels serialised, events between
         // them); the other steps replay a one-step graph of the fused kernels with event records
         // between them.  Either way each kernel's duration is measured the way it runs inside a
         // recorded graph (no host launch gaps); the step state is rewritten per replay.
         int done = 0;
-        if (L.mesh && !L.pml && h.side && nsteps >= Handle::kProfileSteps)
+        L.linear = 0;  // the branches' kernels, whatever the handle's age
+        if (L.mesh && h.side && nsteps >= Handle::kProfileSteps)
         {
-            cudaGraphExec_t pexec = nullptr;
-            PB_TRY(profile_graph<R>(h, L, &pexec));
             const int n = Handle::kProfileSteps;
             for (; done + n <= nsteps; done += n)
             {
+                const bool more = done + n < nsteps;
+                const Handle::StepProfile &prof = h.profile[more ? 1 : 0];
+                cudaGraphExec_t pexec = nullptr;
+                PB_TRY(profile_graph<R>(h, L, more, &pexec));
                 StepState sk{stt.tnew0 + done, stt.n3, stt.row0 + done,
                              acc_dev ? acc_dev + (long long)done * h.nt : nullptr};
                 sk.series = h.d_series;
                 set_state_kernel<<<1, 1, 0, s>>>(h.d_state, sk);
                 PB_CHECK_LAUNCH();
                 PB_CUDA(cudaGraphLaunch(pexec, s));
-                PB_CUDA(cudaEventSynchronize(h.evk[h.evk_used - 1]));
-                for (int i = 0; i + 1 < h.evk_used; i++)
+                PB_CUDA(cudaEventSynchronize(h.evk[prof.used - 1]));
+                for (int i = 0; i + 1 < prof.used; i++)
                 {
                     float ms = 0;
                     cudaEventElapsedTime(&ms, h.evk[i], h.evk[i + 1]);
-                    const int kind = h.evk_kind[i];
+                    const int kind = prof.kind[i];
                     h.kind_us[kind] += 1000.0 * ms;
                     h.kind_n[kind]++;
                     if (kind == PPPM_KERNEL_EMPTY)
@@ -2519,11 +2541,13 @@ int time_kernels(Handle &h, int reps, float *us)
         case PPPM_KERNEL_CONV2: launch_conv<R>(L, 0, PassAt{2, 0}, s); break;
         case PPPM_KERNEL_CONV4: launch_conv<R>(L, 0, PassAt{kPass, 0}, s); break;
         case PPPM_KERNEL_FIX: launch_conv<R>(L, 1, PassAt{2, 1}, s); break;
+        case PPPM_KERNEL_FIX4B: launch_conv<R>(L, 2, PassAt{kPass, 2}, s); break;
         case PPPM_KERNEL_FIX4: launch_conv<R>(L, kPass - 1, PassAt{kPass, kPass - 1}, s); break;
         case PPPM_KERNEL_FINISH: launch_finish<R>(L, 0, 0, 0, 0, s, false); break;
         case PPPM_KERNEL_FINISH1: launch_finish<R>(L, 0, 1, 0, 0, s, false); break;
         case PPPM_KERNEL_FINISH2: launch_finish<R>(L, 0, 2, 1, 0, s, false); break;
         case PPPM_KERNEL_FINISH4: launch_finish<R>(L, 0, 3, 0, 0, s, false); break;
+        case PPPM_KERNEL_FINISH4B: launch_finish<R>(L, 0, 5, 2, 0, s, false); break;
         case PPPM_KERNEL_FINISH4C: launch_finish<R>(L, 0, 6, 3, 0, s, false); break;
         case PPPM_KERNEL_NEAR: near_kernel<R><<<L.near_blocks, T, 0, s>>>(L.a, L.ring, L.st, 0, L.na, 0); break;
         case PPPM_KERNEL_FACE: face_kernel<R><<<L.face_blocks, T, 0, s>>>(L.a, L.ring, L.st, 0, L.fa); break;
@@ -2544,7 +2568,8 @@ int time_kernels(Handle &h, int reps, float *us)
                          PPPM_KERNEL_FIX,          PPPM_KERNEL_FINISH,       PPPM_KERNEL_FINISH1,
                          PPPM_KERNEL_FINISH2,      PPPM_KERNEL_NEAR,         PPPM_KERNEL_FACE,
                          PPPM_KERNEL_STENCIL_BULK, PPPM_KERNEL_STENCIL_CORR, PPPM_KERNEL_CONV4,
-                         PPPM_KERNEL_FIX4,         PPPM_KERNEL_FINISH4,      PPPM_KERNEL_FINISH4C};
+                         PPPM_KERNEL_FIX4B,        PPPM_KERNEL_FIX4,         PPPM_KERNEL_FINISH4,
+                         PPPM_KERNEL_FINISH4B,     PPPM_KERNEL_FINISH4C};
     // the near kernel also writes the FDTD-near sums of the step after next into the slot two
     // ahead, which is time t-1, a level the next step still reads: kept aside and put back
     const size_t slot_bytes = (size_t)h.n_cells * sizeof(R);
@@ -2643,7 +2668,8 @@ int step_free(Handle &h)
     for (StepGraph &g : h.plain_graphs)
         release(g);
     release(h.timing_graph);
-    release(h.profile_graph);
+    for (auto &p : h.profile)
+        release(p.graph);
     dev_free(h.d_state);
     h.d_state = nullptr;
     return PPPM_OK;

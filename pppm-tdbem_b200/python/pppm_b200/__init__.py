@@ -556,7 +556,8 @@ class Solver:
         check(lib.pppm_enable_timing(self.h, 1 if on else 0), "enable_timing")
 
     KERNEL_KINDS = ("stencil", "conv", "conv2", "fix", "finish", "finish1", "finish2", "near", "nwrite", "face",
-                    "empty", "stencil_bulk", "stencil_corr", "conv4", "fix4", "finish4", "finish4c")
+                    "empty", "stencil_bulk", "stencil_corr", "conv4", "fix4", "finish4", "finish4c",
+                    "fix4b", "finish4b")
 
     def kernel_profile(self):
         """{kind: (mean us per launch, launches)} of the kernels timed in measurement mode

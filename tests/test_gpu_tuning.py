@@ -157,7 +157,8 @@ def test_kernel_timing_leaves_the_run_unchanged(gpu, precision):
         s.step(acc[:60])
         if timed:
             t = s.time_kernels(5)
-            for k in ("stencil", "conv", "conv2", "fix", "finish", "finish1", "finish2", "near", "face"):
+            for k in ("stencil", "conv", "conv2", "fix", "finish", "finish1", "finish2", "near", "face", "conv4",
+                      "fix4b", "fix4", "finish4", "finish4b", "finish4c"):
                 assert t.get(k, 0) > 0, (k, t)
         s.step(acc[60:])
         out.append((s.listeners(), s.grid(0), s.grid(-1), s.dump("dirichlet")))
@@ -202,8 +203,8 @@ def test_split_stencil_is_bit_identical(gpu, precision):
 @pytest.mark.parametrize("split", [0, 1])
 def test_measurement_mode_profiles_every_kernel(gpu, split):
     """Measurement mode (pppm_enable_timing) with the split face stage: groups of four steps replay
-    the recorded graph's kernels serialised with events between them; every kind is counted once
-    per launch and timed, and the run stays finite."""
+    the recorded graph's kernels serialised with events between them, a pass of four while steps of the
+    call follow; every kind is counted once per launch and timed, and the run stays finite."""
     v0, f, h, mn, dt = sphere_small()
     s = Solver(24, h, dt, mn)
     s.set_option("split_stencil", split)
@@ -223,9 +224,36 @@ def test_measurement_mode_profiles_every_kernel(gpu, split):
         assert n["stencil_bulk"] == 40 and n["stencil_corr"] == 40 and n["stencil"] == 2
     else:
         assert n["stencil"] == 42 and "stencil_bulk" not in n
-    assert n["conv2"] == 20 and n["fix"] == 20 and n["near"] == 42 and n["face"] == 2
-    assert n["finish1"] == 20 and n["finish2"] == 10 and n["finish"] == 10
+    assert n["conv4"] == 10 and n["fix"] == 10 and n["fix4b"] == 10 and n["fix4"] == 10
+    assert n["near"] == 42 and n["face"] == 2
+    assert n["finish4"] == 10 and n["finish2"] == 10 and n["finish4b"] == 10 and n["finish4c"] == 10
     assert n["nwrite"] == 10 and n["empty"] == 10
+    assert not {"conv", "conv2", "finish", "finish1"} & set(n)
+
+
+@pytest.mark.parametrize("pml", [0, 4])
+def test_measurement_mode_runs_the_call(gpu, pml):
+    """In calls of whole groups of four steps, measurement mode launches the passes of the unmeasured call (at
+    a call's end two pairs): the counts say so, and series, fields and histories are bit-identical."""
+    v0, f, h, mn, dt = sphere_small()
+    acc = sine_acc(56, len(f), 1500.0, dt)
+    out = []
+    for timed in (False, True):
+        s = Solver(24, h, dt, mn, pml_width=pml)
+        s.set_mesh(v0, f)
+        s.add_listener(20, 20, 20)
+        s.enable_timing(timed)
+        for a, b in ((0, 4), (4, 24), (24, 56)):
+            s.step(acc[a:b])
+        out.append((s.listeners(), s.grid(0), s.grid(-1), s.grid(-2), s.dump("dirichlet"), s.dump("neumann")))
+        n = {k: c for k, (us, c) in s.kernel_profile().items()}
+        s.close()
+    for a, b in zip(*out):
+        assert np.any(a) and np.array_equal(a, b)
+    assert n["conv4"] == 11 and n["fix4"] == 11 and n["fix4b"] == 11 and n["finish4"] == 11 and n["finish4c"] == 11
+    assert n["conv2"] == 6 and n["fix"] == 17 and n["finish1"] == 6 and n["finish2"] == 14 and n["finish"] == 3
+    assert n["near"] == 56 and n["nwrite"] == 14 and "face" not in n
+    assert n.get("stencil", 0) == (56 if pml else 0)
 
 
 def _edge_series(axis, cell, split, steps=150, chunk=23, profile=False):
