@@ -311,17 +311,18 @@ int pppm_pair_weights_static(int device, void *stream, float dt, float dl, float
 int pppm_set_option(pppm_handle *h, int option, int value);
 int pppm_get_option(pppm_handle *h, int option, int *value);
 /* No counterpart in the reference.  Autotuner of the face stage, on the current mesh and state.
- * Phase 1 times kernels alone: two steps of the face-pair convolution in 6 configurations
- * (candidate i < 6: PPPM_OPT_CONV_PAIRS = i / 3, threads = {64, 128, 256}[i % 3]), then two steps
+ * Phase 1, a report, times kernels alone: two steps of the face-pair convolution in 6 configurations
+ * (candidate i < 6: PPPM_OPT_CONV_PAIRS = i / 3, threads of the completion = {64, 128, 256}[i % 3]; with
+ * i >= 3 the two-step pass of a call's last steps), then two steps
  * of the rest of the face stage with the near-field terms one pass per step (candidate 6) or two
- * steps per pass (candidate 7), reps launches of each kernel.  Phase 2 (absorbing boundary) times
+ * steps per pass (candidate 7), reps launches of each kernel.  Phase 2 times
  * 64 recorded steps (zero accelerations) of each of PPPM_TUNE_CONFIGS option sets (config j: conv_pairs = j / 6,
  * threads = {64, 128, 256}[(j / 2) % 3], terms_pairs = j % 2) from a device snapshot of the
  * fields and histories (a warm-up replay, then a timed one; best of min(reps, 3)) and sets the options to
- * the fastest (with a PML, phase 1 decides).  us_out (may be NULL; 2 * PPPM_TUNE_CANDIDATES +
+ * the fastest.  us_out (may be NULL; 2 * PPPM_TUNE_CANDIDATES +
  * PPPM_TUNE_CONFIGS floats): microseconds per launch of candidate i's first kernel (us_out[2 i])
  * and second kernel (us_out[2 i + 1]), then microseconds per step of each config; *best (may be
- * NULL): the config chosen (or, with a PML, the convolution candidate).  The fields, histories,
+ * NULL): the config chosen (or, with a PML, the convolution candidate of that config).  The fields, histories,
  * time and recorded listener samples are as before the call; it allocates a snapshot of the
  * fields and histories for its duration and records CUDA graphs, so it must not be called while
  * the handle's stream is being captured.  Needs a mesh and the PPPM method. */

@@ -2210,14 +2210,16 @@ int run_steps(Handle &h, const float *acc_dev, int nsteps)
     return PPPM_OK;
 }
 
-// Autotuner of the face stage: on the handle's current mesh and state, time the face-pair
-// convolution of two consecutive steps in every candidate configuration - one pass per step
-// (conv, conv) or one pass for both (conv2, fix) - at 64, 128 and 256 threads per block, each of
-// the two launches reps times back to back on the handle's stream between CUDA events; then the
+// Autotuner of the face stage, on the handle's current mesh and state.  Phase 1 is a report of kernels
+// alone: the face-pair convolution of two consecutive steps, one pass per step (conv, conv) or one pass
+// for both (conv2, fix: what a call's last steps run; before them passes are of four), with the
+// completion at 64, 128 and 256 threads per block (the convolution's blocks are kConvThreads always), each
+// of the two launches reps times back to back on the handle's stream between CUDA events; then the
 // rest of the face stage with the near-field terms one or two steps per pass.  The kernels write
 // only scratch sums and derived terms, so no state of the scene changes.  us[2 i], us[2 i + 1]:
 // microseconds per launch of the first and second kernel of candidate i, in the order
 // (pairs 0, 64), (pairs 0, 128), (pairs 0, 256), (pairs 1, 64), ..., finish single, finish pairs.
+// Phase 2 times recorded steps and decides.
 constexpr int kTuneThreads[3] = {64, 128, 256};
 constexpr int kTuneConfigs = 12;     // conv_pairs x face threads x terms_pairs (phase 2)
 constexpr int kTuneGraphSteps = 64;  // recorded steps timed per configuration
@@ -2250,8 +2252,6 @@ int autotune(Handle &h, int reps, float *us, int *best)
         run(c, 1);
     }
     PB_CHECK_LAUNCH();
-    int bi = 0;
-    float tot[kConv];
     for (int c = 0; c < kConv; c++)
     {
         PB_CUDA(cudaEventRecord(h.ev[0], s));
@@ -2267,14 +2267,11 @@ int autotune(Handle &h, int reps, float *us, int *best)
         PB_CUDA(cudaEventElapsedTime(&mb, h.ev[1], h.ev[2]));
         us[2 * c] = 1000.0f * ma / reps;
         us[2 * c + 1] = 1000.0f * mb / reps;
-        tot[c] = us[2 * c] + us[2 * c + 1];
-        if (tot[c] < tot[bi])
-            bi = c;
     }
     // the rest of the face stage (finish, the near-field terms): one pass per step, or two steps
-    // per pass (candidates 9 and 10), at the chosen block size
+    // per pass (candidates 6 and 7), at the handle's block size
     {
-        const int FT = kTuneThreads[bi % 3], nb = div_up((long long)nt * 32, FT);
+        const int FT = h.face_threads, nb = div_up((long long)nt * 32, FT);
         for (int c = kConv; c < kConv + 2; c++)
         {
             const bool two = c != kConv;
@@ -2310,14 +2307,8 @@ int autotune(Handle &h, int reps, float *us, int *best)
         h.launches += 4LL * reps + 4;
     }
     h.launches += 2LL * reps * kConv + 2 * kConv + 1;
-    h.conv_pairs = bi / 3;
-    h.face_threads = kTuneThreads[bi % 3];
-    h.terms_pairs = us[2 * kConv + 2] + us[2 * kConv + 3] < us[2 * kConv] + us[2 * kConv + 1];
-    *best = bi;
-    if (!h.side || h.prm.pml_width > 0)
-        return PPPM_OK;  // no two-branch step graphs: the kernel timings decide
 
-    // Phase 2: the kernels compete inside the two-branch step graph (the convolution beside the
+    // Phase 2: the kernels compete inside the branched step graph (the convolution beside the
     // stencil and the near stage, the finish on the critical path), which isolated launches do not
     // show.  Time kTuneGraphSteps recorded steps (zero accelerations) of every configuration from
     // one device snapshot of the fields and histories: per candidate and rep, restore the snapshot,
@@ -2326,26 +2317,36 @@ int autotune(Handle &h, int reps, float *us, int *best)
     // (conv_pairs = i / 6, threads = {64, 128, 256}[(i / 2) % 3], terms_pairs = i % 2).  The steps
     // write listener rows past the recorded ones, which the next call overwrites; the fields and
     // histories are restored from the snapshot at the end; h.t and the series count do not move.
-    // histories: the copies, then the two canonical rings
-    const size_t gbytes = (size_t)h.n_cells * h.real_size, cbytes = (size_t)4 * nt * kHistRow * h.real_size,
-                 rbytes = (size_t)nt * kRing * h.real_size, hbytes = cbytes + 2 * rbytes;
+    // fields: the grids, with a PML its auxiliary fields; histories: the copies, then the two canonical rings
+    const bool pml = h.prm.pml_width > 0;
+    const size_t gbytes = (size_t)h.n_cells * h.real_size, fbytes = (pml ? 21 : 3) * gbytes,
+                 cbytes = (size_t)4 * nt * kHistRow * h.real_size, rbytes = (size_t)nt * kRing * h.real_size,
+                 hbytes = cbytes + 2 * rbytes;
     const size_t abytes = (size_t)kTuneGraphSteps * nt * sizeof(float);
     void *snap = nullptr;
-    PB_TRY(dev_alloc(&snap, 3 * gbytes + hbytes + abytes));
+    const int src = dev_alloc(&snap, fbytes + hbytes + abytes);
+    if (src == PPPM_ERR_NOMEM && pml)
+    {
+        // no room for a copy of the auxiliary fields: the options stay
+        cudaGetLastError();
+        *best = h.conv_pairs * 3 + (h.face_threads == 64 ? 0 : h.face_threads == 128 ? 1 : 2);
+        return PPPM_OK;
+    }
+    PB_TRY(src);
     // zero accelerations for the timed steps (the code paths of a call with accelerations)
-    const float *zacc = (const float *)((char *)snap + 3 * gbytes + hbytes);
+    const float *zacc = (const float *)((char *)snap + fbytes + hbytes);
     PB_CUDA(cudaMemsetAsync((void *)zacc, 0, abytes, s));
     auto copy_state = [&](bool save) -> cudaError_t {
         cudaError_t e = cudaSuccess;
-        for (int i = 0; i < 3 && e == cudaSuccess; i++)
-            e = save ? cudaMemcpyAsync((char *)snap + i * gbytes, h.grid[i], gbytes, cudaMemcpyDeviceToDevice, s)
-                     : cudaMemcpyAsync(h.grid[i], (char *)snap + i * gbytes, gbytes, cudaMemcpyDeviceToDevice, s);
-        void *hist[3] = {h.d_hist, h.d_neumann, h.d_dirichlet};
-        const size_t hb[3] = {cbytes, rbytes, rbytes};
-        char *at = (char *)snap + 3 * gbytes;
-        for (int i = 0; i < 3 && e == cudaSuccess; at += hb[i], i++)
-            e = save ? cudaMemcpyAsync(at, hist[i], hb[i], cudaMemcpyDeviceToDevice, s)
-                     : cudaMemcpyAsync(hist[i], at, hb[i], cudaMemcpyDeviceToDevice, s);
+        void *part[9] = {h.grid[0], h.grid[1], h.grid[2], h.pml[0], h.pml[1], h.pml[2],
+                         h.d_hist,  h.d_neumann, h.d_dirichlet};
+        const size_t a = pml ? 6 * gbytes : 0;
+        const size_t bytes[9] = {gbytes, gbytes, gbytes, a, a, a, cbytes, rbytes, rbytes};
+        char *at = (char *)snap;
+        for (int i = 0; i < 9 && e == cudaSuccess; at += bytes[i], i++)
+            if (bytes[i])
+                e = save ? cudaMemcpyAsync(at, part[i], bytes[i], cudaMemcpyDeviceToDevice, s)
+                         : cudaMemcpyAsync(part[i], at, bytes[i], cudaMemcpyDeviceToDevice, s);
         return e;
     };
     const int keep_pairs = h.conv_pairs, keep_threads = h.face_threads;
@@ -2358,7 +2359,7 @@ int autotune(Handle &h, int reps, float *us, int *best)
     // the interior stencil one or four cells per thread (FP32, res % 4 == 0): time the bulk launch
     // (no listeners; the snapshot restore below undoes its writes) both ways and keep the faster
     const int keep_vec4 = h.stencil_vec4;
-    if (!h.fp64 && h.res % 4 == 0 && e == cudaSuccess)
+    if (!h.fp64 && !pml && h.res % 4 == 0 && e == cudaSuccess)
     {
         float tv[2] = {0, 0};
         set_state_kernel<<<1, 1, 0, s>>>(h.d_state, sg);
@@ -2445,7 +2446,7 @@ int autotune(Handle &h, int reps, float *us, int *best)
     h.conv_pairs = gbest / 6;
     h.face_threads = kTuneThreads[(gbest / 2) % 3];
     h.terms_pairs = (gbest & 1) != 0;
-    *best = gbest;
+    *best = pml ? gbest / 2 : gbest;  // with a PML the number of its convolution candidate
     return PPPM_OK;
 }
 

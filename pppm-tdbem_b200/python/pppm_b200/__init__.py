@@ -535,9 +535,10 @@ class Solver:
         return v.value
 
     def autotune(self, reps=20):
-        """Time the face-stage candidates on the current mesh (pppm_autotune) and keep the
-        fastest.  Returns {"us": {(pairs, threads): us per two steps}, "launch_us":
-        {(pairs, threads): (first kernel, second kernel) us per launch}, "best": (pairs, threads)}."""
+        """Time the launch options on the current mesh (pppm_autotune) and keep the fastest set of
+        whole recorded steps, "step_us": {(pairs, threads, terms): us per step}.  Also reported, kernels alone:
+        "us": {(pairs, threads): us per two steps}, "launch_us": {(pairs, threads): (first kernel, second
+        kernel) us per launch}; chosen: "best": (pairs, threads), "terms_pairs", "stencil_vec4"."""
         n = len(self.TUNE_CANDIDATES)
         us = (ctypes.c_float * (2 * (n + 2) + len(self.TUNE_CONFIGS)))()
         best = ctypes.c_int()

@@ -120,6 +120,26 @@ def test_autotune_keeps_results(gpu):
     assert rel_l2(got, ref) < 1e-3
 
 
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_autotune_with_pml(gpu, precision):
+    """A PML handle's calls replay the same passes: the recorded steps of every option set decide, and
+    the whole state, auxiliary fields included, is as before."""
+    v, f, h, mn, dt = sphere_small()
+    s = Solver(24, h, dt, mn, pml_width=4, precision=precision)
+    s.set_mesh(v, f)
+    s.add_listener(20, 20, 20)
+    s.step(sine_acc(50, len(f), 1500.0, dt))
+    before = s.save_state(), s.listeners(), s.t
+    tune = s.autotune(reps=3)
+    assert tune["step_us"] is not None and all(u > 0 for u in tune["step_us"].values())
+    chosen = (s.get_option("conv_pairs"), s.get_option("face_threads"), s.get_option("terms_pairs"))
+    assert chosen == min(tune["step_us"], key=tune["step_us"].get)
+    assert np.array_equal(before[0], s.save_state()) and np.array_equal(before[1], s.listeners()) and s.t == before[2]
+    s.step(sine_acc(20, len(f), 1500.0, dt, first=50))
+    assert np.all(np.isfinite(s.listeners()))
+    s.close()
+
+
 def test_bad_options_rejected(gpu):
     v, f, h, mn, dt = sphere_small()
     s = Solver(24, h, dt, mn)
