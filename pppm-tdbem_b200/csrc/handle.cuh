@@ -14,8 +14,8 @@
 //                  Dirichlet taps are one aligned load
 //   cell CSR       cell_start[res^3 + 1] / cell_tris[nt] (sorted by triangle id per cell),
 //                  same for base cells
-//   3^3 pairs      n3 corrected cells: n3_cell, n3_start[n3 + 1]; p3 pairs: p3_tri, p3_woff
-//                  (the pair's record offset in the triangle's grid-cache records)
+//   3^3 pairs      n3 corrected cells: n3_cell, n3_start[n3 + 1]; p3 pairs: p3_tri, p3_ref
+//                  (triangle * 27 + the pair's record offset in the triangle's grid-cache records)
 //   near terms     terms[nt][27][2]: each triangle's 54 grid-cache records convolved with its own
 //                  history in the current step (step.cu); a corrected cell sums its pairs' terms
 //   face pairs     face_start[nt + 1] per centre triangle; pf pairs: face_nbr; dense
@@ -136,8 +136,7 @@ struct Handle
     int n3 = 0;
     long long p3 = 0;
     int *d_n3_cell = nullptr, *d_n3_start = nullptr;
-    int *d_p3_tri = nullptr, *d_p3_ref = nullptr;  // triangle; triangle * 27 + record offset
-    unsigned char *d_p3_woff = nullptr;
+    int *d_p3_tri = nullptr, *d_p3_ref = nullptr;
     long long p3_cap = 0;
     unsigned *d_corr_mask = nullptr;
 

@@ -250,10 +250,9 @@ __global__ void compact_kernel(const int *flag, const int *pos, const int *start
 }
 
 // 3^3 pairs of each corrected cell, sub-cells x fastest (particle_grid.cu:164-182);
-// woff = GridCache weight index of (cell - triangle cell) (pppm_cache.h:38-42)
+// p3_ref = triangle * 27 + GridCache weight index of (cell - triangle cell) (pppm_cache.h:38-42)
 __global__ void fill_pairs3_kernel(const int *n3_cell, const int *n3_start, int n3, int res, const int *cell_start,
-                                   const int *cell_tris, int *p3_tri, unsigned char *p3_woff, int *p3_ref,
-                                   unsigned *mask)
+                                   const int *cell_tris, int *p3_tri, int *p3_ref, unsigned *mask)
 {
     // one warp per corrected cell: lane l < 27 copies sub-cell l's list to its offset in the
     // cell's list (a warp prefix sum over the 27 lengths keeps the sub-cell order)
@@ -265,12 +264,12 @@ __global__ void fill_pairs3_kernel(const int *n3_cell, const int *n3_start, int 
     const int c = n3_cell[i];
     const int x = c / (res * res), y = (c / res) % res, z = c % res;
     int b = 0, len = 0;
-    unsigned char woff = 0;
+    int woff = 0;
     if (lane < 27)
     {
         const int dx = lane % 3 - 1, dy = lane / 3 % 3 - 1, dz = lane / 9 - 1;
         const int sc = ((x + dx) * res + (y + dy)) * res + (z + dz);
-        woff = (unsigned char)((1 - dx) + 3 * (1 - dy) + 9 * (1 - dz));
+        woff = (1 - dx) + 3 * (1 - dy) + 9 * (1 - dz);
         b = cell_start[sc];
         len = cell_start[sc + 1] - b;
     }
@@ -286,7 +285,6 @@ __global__ void fill_pairs3_kernel(const int *n3_cell, const int *n3_start, int 
     for (int j = 0; j < len; j++)
     {
         p3_tri[o + j] = cell_tris[b + j];
-        p3_woff[o + j] = woff;
         p3_ref[o + j] = cell_tris[b + j] * 27 + woff;
     }
     if (lane == 0)
@@ -656,20 +654,17 @@ int mesh_build(Handle &h)
     if (p3 > h.p3_cap)
     {
         dev_free(h.d_p3_tri);
-        dev_free(h.d_p3_woff);
         dev_free(h.d_p3_ref);
         h.d_p3_ref = nullptr;
         h.d_p3_tri = nullptr;
-        h.d_p3_woff = nullptr;
         long long cap = p3 + p3 / 4 + 256;
         PB_TRY(dalloc(&h.d_p3_tri, (size_t)cap));
-        PB_TRY(dalloc(&h.d_p3_woff, (size_t)cap));
         PB_TRY(dalloc(&h.d_p3_ref, (size_t)cap));
         h.p3_cap = cap;
     }
     PB_CUDA(cudaMemsetAsync(h.d_corr_mask, 0, sizeof(unsigned) * ((nc + 31) / 32), s));
     fill_pairs3_kernel<<<div_up((long long)n3 * 32, T), T, 0, s>>>(h.d_n3_cell, h.d_n3_start, n3, res, h.d_cell_start, h.d_cell_tris,
-                                                   h.d_p3_tri, h.d_p3_woff, h.d_p3_ref, h.d_corr_mask);
+                                                   h.d_p3_tri, h.d_p3_ref, h.d_corr_mask);
     h.launches++;
     PB_CHECK_LAUNCH();
 
