@@ -2954,12 +2954,12 @@ int batch_tables(Batch &b, const std::vector<int> &active)
         S.na = L.na;
         S.st = h.d_state;
         S.conv = L.conv;
-        // near-stage warps stride over the scene's corrected cells (their count is read on the
-        // device), so the block map may exceed it: it grows with headroom and never shrinks, so a
+        // near-stage warps, two cells a warp, stride over the scene's corrected cells (their count is
+        // read on the device), so the block map may exceed it: it grows with headroom and never shrinks, so a
         // moving scene, whose count changes at every update_mesh, keeps its recorded batch graphs
         if (h.n3 > h.batch_near_cells)
             h.batch_near_cells = h.n3 + h.n3 / 8 + 256;
-        const int near_blocks = std::max(1, div_up((long long)h.batch_near_cells * 32, T));
+        const int near_blocks = std::max(1, div_up((long long)h.batch_near_cells * 16, T));
         S.near_warps = near_blocks * (T / 32);
         const int corr_blocks = std::max(1, div_up((long long)h.batch_near_cells, T));
         S.corr_threads = corr_blocks * T;
