@@ -86,7 +86,9 @@ int pppm_set_mesh(pppm_handle *h, const float *verts, int nv, const int *tris, i
 
 /* Replaces PPPMSolver::update_mesh(verts) (pppm.h:97-109): same topology, new vertex
  * positions; lists rebuilt, caches refreshed under the reference's recompute criteria
- * (pppm_cache.h:65-70, 123-128).  verts_on_device != 0: verts is a device pointer. */
+ * (pppm_cache.h:65-70, 123-128).  A failed update (a triangle outside the grid's interior, say) leaves tables
+ * that no call may use: with the PPPM method steps, batched runs, the adjoint, the tuner and cache imports
+ * return PPPM_ERR_STATE until an update or pppm_set_mesh succeeds.  verts_on_device != 0: verts is a device pointer. */
 int pppm_update_mesh(pppm_handle *h, const float *verts, int verts_on_device);
 
 /* Replaces nsteps calls of PPPMSolver::update_grid_and_face(acc) (pppm.h:138-145).

@@ -128,6 +128,7 @@ void free_mesh(Handle &h)
     adjoint_free(h);
     ghost_free(h);
     h.mesh_version++;
+    h.tables_broken = false;
     cache_free(h);
     void **ptrs[] = {(void **)&h.d_verts,      (void **)&h.d_tris,        (void **)&h.d_center,
                      (void **)&h.d_normal,     (void **)&h.d_area,        (void **)&h.d_cellc,
@@ -215,6 +216,15 @@ int d2h(Handle &h, std::vector<T> &v, const void *src, size_t n)
 }  // namespace
 
 extern "C" {
+
+// whether the mesh tables may be read (Handle::tables_broken)
+static int need_tables(const Handle &h)
+{
+    if (!h.tables_broken)
+        return PPPM_OK;
+    set_error("the last pppm_update_mesh failed: call it again with a mesh that it accepts");
+    return PPPM_ERR_STATE;
+}
 
 // The step status as far as it has reached the host: PPPM_ERR_NAN once a step kernel saw a
 // non-finite Dirichlet value or listener sample (it writes the host's mapped word; a queued copy and
@@ -552,6 +562,7 @@ int pppm_update_mesh(pppm_handle *ph, const float *verts, int verts_on_device)
         const int rc = mesh_build(h);
         if (rc != PPPM_OK)
         {
+            h.tables_broken = h.prm.method == PPPM_METHOD_PPPM;
             join_grid_cache(h);
             return rc;
         }
@@ -565,7 +576,12 @@ int pppm_update_mesh(pppm_handle *ph, const float *verts, int verts_on_device)
         PB_TRY(ghost_build(h));
         return PPPM_OK;
     }
-    PB_TRY(cache_refresh(h));
+    {
+        const int rc = cache_refresh(h);
+        h.tables_broken = rc != PPPM_OK;
+        if (rc != PPPM_OK)
+            return rc;
+    }
     PB_TRY(step_prime(h));
     return PPPM_OK;
 }
@@ -589,6 +605,7 @@ int pppm_step(pppm_handle *ph, const float *acc, int acc_on_device, int nsteps)
         set_error("a cache state was restored: call pppm_update_mesh before stepping");
         return PPPM_ERR_STATE;
     }
+    PB_TRY(need_tables(h));
     PB_TRY(poll_step_status(h));
     const float *dacc = nullptr;
     if (h.mesh_set)
@@ -676,6 +693,7 @@ int pppm_batch_run(pppm_batch *b, const float *const *acc, const int *nsteps, in
             return PPPM_ERR_ARG;
         if (nsteps[i] == 0)
             continue;
+        PB_TRY(need_tables(h));
         cudaSetDevice(h.prm.device);
         if (acc_on_device)
             dacc[i] = acc[i];
@@ -722,6 +740,7 @@ int pppm_adjoint(pppm_handle *ph, const void *dL_dsignal, int nsteps, int on_dev
         set_error("a cache state was restored: call pppm_update_mesh before the adjoint");
         return PPPM_ERR_STATE;
     }
+    PB_TRY(need_tables(h));
     cudaSetDevice(h.prm.device);
     const size_t gb = (size_t)nsteps * nl * h.real_size, ob = (size_t)nsteps * h.nt * h.real_size;
     if (on_device)
@@ -1241,6 +1260,7 @@ int pppm_import_grid_cache(pppm_handle *ph, const void *records, size_t bytes)
         return PPPM_ERR_STATE;
     if (!records || bytes < (size_t)h.nt * 54 * 72)
         return PPPM_ERR_ARG;
+    PB_TRY(need_tables(h));
     h.mesh_version++;
     PB_TRY(cache_import_grid(h, records));
     PB_TRY(step_prime(h));
@@ -1256,6 +1276,7 @@ int pppm_import_face_cache(pppm_handle *ph, const int *face_pairs, const void *r
         return PPPM_ERR_STATE;
     if (!face_pairs || !records || npairs < 0)
         return PPPM_ERR_ARG;
+    PB_TRY(need_tables(h));
     h.mesh_version++;
     PB_TRY(cache_import_face(h, face_pairs, records, npairs));
     PB_TRY(step_prime(h));
@@ -1388,6 +1409,7 @@ int pppm_autotune(pppm_handle *ph, int reps, float *us_out, int *best)
         return PPPM_ERR_ARG;
     }
     Handle &h = ph->h;
+    PB_TRY(need_tables(h));
     cudaSetDevice(h.prm.device);
     float us[2 * PPPM_TUNE_CANDIDATES + PPPM_TUNE_CONFIGS] = {0};
     int b = 0;
@@ -1424,6 +1446,7 @@ int pppm_time_kernels(pppm_handle *ph, int reps, int nkinds, float *us_per_launc
     PB_CUDA(cudaStreamIsCapturing(h.stream, &cs));
     if (cs != cudaStreamCaptureStatusNone)
         return PPPM_ERR_STATE;
+    PB_TRY(need_tables(h));
     float us[PPPM_KERNEL_KINDS];
     PB_TRY(step_time_kernels(h, reps, us));
     PB_CUDA(cudaStreamSynchronize(h.stream));

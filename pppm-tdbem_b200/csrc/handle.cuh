@@ -264,6 +264,9 @@ struct Handle
     // ---- adjoint (adjoint.cu): transposed tables and adjoint state, built on first use
     long long mesh_version = 0;  // bumped whenever the lists or weight tables change
     bool tables_stale = false;   // a cache state was restored: no step until update_mesh
+    // the last mesh update failed: lists and weight tables of two geometries (their offsets may lie past the
+    // arrays), which no kernel may read until an update succeeds
+    bool tables_broken = false;
     struct Adjoint *adj = nullptr;
 
     // ---- pinned host words for batched reads of device counts (read_ints)

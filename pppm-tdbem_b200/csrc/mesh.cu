@@ -651,8 +651,10 @@ int mesh_build(Handle &h)
     h.pf = pf;
 
     // ---- 3^3 pairs and corrected-cell mask
+    // (a capacity is 0 while its arrays are replaced, so that an update after a failed allocation makes them)
     if (p3 > h.p3_cap)
     {
+        h.p3_cap = 0;
         dev_free(h.d_p3_tri);
         dev_free(h.d_p3_ref);
         h.d_p3_ref = nullptr;
@@ -671,6 +673,7 @@ int mesh_build(Handle &h)
     // ---- 4^3 lists
     if (p4 > h.n4_cap)
     {
+        h.n4_cap = 0;
         dev_free(h.d_n4_tris);
         h.d_n4_tris = nullptr;
         long long cap = p4 + p4 / 4 + 256;
@@ -685,6 +688,7 @@ int mesh_build(Handle &h)
     // ---- face pairs per centre triangle
     if (pf > h.pf_cap)
     {
+        h.pf_cap = 0;
         dev_free(h.d_face_nbr);
         dev_free(h.d_face_pool);
         dev_free(h.d_face_w);

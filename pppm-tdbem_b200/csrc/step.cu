@@ -2453,7 +2453,7 @@ int autotune(Handle &h, int reps, float *us, int *best)
 template <typename R>
 int prime(Handle &h)
 {
-    if (!h.mesh_set || h.n3 == 0)
+    if (!h.mesh_set || h.n3 == 0 || h.tables_broken)
         return PPPM_OK;
     if (!h.d_state)
         PB_TRY(dalloc(&h.d_state, 1));

@@ -8,8 +8,8 @@ import numpy as np
 import pytest
 
 import pppm_b200
-from helpers import sine_acc, sphere_small
-from pppm_b200 import PPPMError, Solver
+from helpers import rel_l2, sine_acc, sphere_small
+from pppm_b200 import Batch, PPPMError, Solver
 
 pytestmark = pytest.mark.gpu
 
@@ -50,6 +50,44 @@ def test_finite_run_reports_nothing(gpu):
     for _ in range(3):
         s.step(sine_acc(30, len(f), 1500.0, dt))
     s.sync()
+    s.close()
+
+
+def test_failed_mesh_update_is_not_stepped(gpu):
+    """An update that is refused leaves the lists of one geometry and the offsets of another: nothing reads
+    them until an update succeeds, and the run goes on from there."""
+    v, f, h, mn, dt = sphere_small()
+    s = Solver(24, h, dt, mn)
+    s.set_mesh(v, f)
+    s.add_listener(20, 20, 20)
+    acc = sine_acc(20, len(f), 1500.0, dt)
+    s.step(acc)
+    out = v.copy()
+    out[: len(v) // 2] += np.float32(24 * h)
+    with pytest.raises(PPPMError):
+        s.update_mesh(out)
+    b = Batch([s])
+    for call in (lambda: s.step(acc), lambda: s.step(acc[:1]), lambda: b.run([acc]), lambda: s.adjoint(np.ones((4, 1))),
+                 s.autotune, s.time_kernels, lambda: s.import_grid_cache(np.zeros(len(f) * 54 * 72, np.uint8))):
+        with pytest.raises(PPPMError) as e:
+            call()
+        assert e.value.status == pppm_b200.ERR_STATE
+    assert s.t == 19
+    s.reset_fields()
+    s.update_mesh(v)
+    s.rewind_listeners()
+    s.t = -1
+    s.step(acc)
+    s.sync()
+    got = s.series()
+    b.close()
+    s.close()
+    s = Solver(24, h, dt, mn)
+    s.set_mesh(v, f)
+    s.add_listener(20, 20, 20)
+    s.step(acc)
+    # (the records are those of the same geometry, refreshed in another order of events)
+    assert np.abs(got).max() > 0 and rel_l2(got, s.series()) < 1e-5
     s.close()
 
 
