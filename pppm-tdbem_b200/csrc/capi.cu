@@ -724,6 +724,12 @@ int pppm_adjoint(pppm_handle *ph, const void *dL_dsignal, int nsteps, int on_dev
         set_error("adjoint needs a mesh");
         return PPPM_ERR_STATE;
     }
+    if (h.prm.method != PPPM_METHOD_PPPM)
+    {
+        // (its handles hold no face pairs, grid-cache records, interpolation or denominators to read)
+        set_error("adjoint needs the PPPM method");
+        return PPPM_ERR_STATE;
+    }
     const int nl = (int)h.listen_xyz.size() / 3;
     for (int k = 0; k < 3 * nl; k++)
         if (h.listen_xyz[k] < 1 || h.listen_xyz[k] > h.res - 2)

@@ -244,3 +244,10 @@ def test_adjoint_rejects(gpu):
     with pytest.raises(PPPMError):
         s.adjoint(np.zeros((4, 1)))
     s.close()
+    # the ghost-cell method has no tables for the reverse step
+    s = Solver(24, h, dt, mn, method="ghost")
+    s.set_mesh(v, f)
+    s.add_listener(20, 12, 12)
+    with pytest.raises(PPPMError):
+        s.adjoint(np.zeros((4, 1)))
+    s.close()
