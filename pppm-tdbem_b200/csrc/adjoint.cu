@@ -1009,11 +1009,13 @@ int run_adjoint(Handle &h, const R *g, int nsteps, R *out, int fresh)
             A.chunk = nullptr;
             A.chunk_sig.clear();
             cudaGraph_t graph = nullptr;
-            PB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+            // (on the handle's own stream: the caller's may be one that cannot be captured, or one that other
+            // threads launch into)
+            PB_CUDA(cudaStreamBeginCapture(h.side, cudaStreamCaptureModeThreadLocal));
             for (int j = 0; j < kAdjChunk; j++)
-                adj_launch_step<R>(a, dst, j, s);
-            advance_adj_kernel<<<1, 1, 0, s>>>(dst, kAdjChunk);
-            cudaError_t e = cudaStreamEndCapture(s, &graph);
+                adj_launch_step<R>(a, dst, j, h.side);
+            advance_adj_kernel<<<1, 1, 0, h.side>>>(dst, kAdjChunk);
+            cudaError_t e = cudaStreamEndCapture(h.side, &graph);
             if (e == cudaSuccess)
                 e = cudaGraphInstantiate(&A.chunk, graph, 0);
             if (graph)

@@ -1998,17 +1998,20 @@ int graph_for(Handle &h, const StepLaunch<R> &L, int nsteps, cudaGraphExec_t *ou
         cudaGraphExecDestroy(g.exec);
     g.exec = nullptr;
     cudaGraph_t graph = nullptr;
-    PB_CUDA(cudaStreamBeginCapture(h.stream, cudaStreamCaptureModeThreadLocal));
+    // (short calls run on any stream of the caller's, also one that cannot be captured or that other threads
+    // launch into: recorded on the handle's own)
+    cudaStream_t s = plain ? h.side : h.stream;
+    PB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     if (!timed && !plain && L.mesh && h.side)
         capture_pipelined<R>(h, L, nsteps, L.pairs != 0, open);
     else
     {
         for (int k = 0; k < nsteps; k++)
-            launch_step<R>(L, k, h.stream, timed ? &h : nullptr);
+            launch_step<R>(L, k, s, timed ? &h : nullptr);
         if (open)
-            advance_state_kernel<<<1, 1, 0, h.stream>>>(const_cast<StepState *>(L.st), nsteps, L.a.nt);
+            advance_state_kernel<<<1, 1, 0, s>>>(const_cast<StepState *>(L.st), nsteps, L.a.nt);
     }
-    cudaError_t e = cudaStreamEndCapture(h.stream, &graph);
+    cudaError_t e = cudaStreamEndCapture(s, &graph);
     if (e == cudaSuccess)
         e = cudaGraphInstantiate(&g.exec, graph, 0);
     if (graph)

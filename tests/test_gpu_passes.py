@@ -182,6 +182,25 @@ def test_recorded_single_steps_equal_direct_launches(gpu, precision, pml):
         assert np.any(a) and np.array_equal(a, b)
 
 
+def test_short_calls_on_a_stream_that_cannot_be_captured(gpu):
+    """Calls of one to three steps and a gradient over less than 128 reverse steps on the legacy default
+    stream, which cannot be captured: their kernels are recorded on a stream of the handle's own.  The same
+    bits as on a stream that the handle makes."""
+    v, f, h, mn, dt, res, cell = _small()
+    acc = sine_acc(60, len(f), 1500.0, dt)
+    out = []
+    for stream in (None, 1):  # 1: cudaStreamLegacy
+        s = Solver(res, h, dt, mn, stream=stream)
+        s.set_mesh(v, f)
+        s.add_listener(*cell)
+        for k in range(0, 60, 3):
+            s.step(acc[k: k + 3])
+        out.append((s.series(), s.grid(0).copy(), s.adjoint(np.ones((60, 1), np.float32))))
+        s.close()
+    for a, b in zip(*out):
+        assert np.any(a) and np.array_equal(a, b)
+
+
 def test_short_calls_keep_the_recorded_graphs(gpu):
     """A program that steps in eight lengths (as many as a handle keeps recorded graphs) with calls of one
     to three steps between: the short calls' graphs have slots of their own, so no longer call is
