@@ -1179,6 +1179,9 @@ __device__ inline void write_neumann(const Ring<R> &ring, const StepState *st, i
                                      int tri, int lane, int what)
 {
     const StepDyn dn = bind_step(st, kstep, nt);
+    // N[t+1] takes the slot of N[t-15], tap 15 of the window that the warp's near-field terms read: no lane
+    // may write before every lane has read (the terms' own exchanges join four lanes only)
+    __syncwarp();
     if (what & 1)
     {
         if (lane < 5)
