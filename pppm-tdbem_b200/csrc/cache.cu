@@ -801,9 +801,10 @@ inline long long gather_face_threads(long long pf)
 // list order in the working precision (pppm.cu:172-193)
 // One warp per triangle: lanes fetch 32 factors at a time, every lane then adds them in list
 // order, so the sum rounds exactly like a sequential loop.  Also writes each pair's
-// double-layer tap 1 with its scale applied (the factor of D[t-1] in the convolution, as the
-// step evaluates it) into d1 (float for FP32 handles, double for FP64), which the two-step
-// convolution of the step reads (step.cu: fix_kernel).
+// double-layer taps 1, 2 and 3 with their scale applied (the factors of D[t-1], D[t-2], D[t-3] in the
+// convolution, as the step evaluates it) into d, one array of `pitch` values per tap (float for FP32
+// handles, double for FP64), which the completion of a pass's later steps reads (step.cu: face_fix), and the
+// denominators' reciprocals behind the denominators.
 __global__ void denom_kernel(const int *face_start, int nt, const float *area, const __half2 *face_w,
                              const float2 *face_scale, const double2 *face_wd, double *denom, void *d, long long pitch)
 {
@@ -1215,7 +1216,7 @@ static int cache_alloc(Handle &h)
     return PPPM_OK;
 }
 
-// The grid-cache refresh (recompute flags, records, the completion factors of the two-step terms)
+// The grid-cache refresh (recompute flags, records, the completion factors of the passes' terms)
 // on stream gs
 static int grid_cache_refresh(Handle &h, cudaStream_t gs)
 {

@@ -11,7 +11,7 @@
 //   face      per triangle (one warp): far field at the face by trilinear interpolation of
 //             the 8 corner cells, the face-to-face convolution over its 4^3 list, and the
 //             Dirichlet update (pppm.cu:116-193) - three reference kernels fused.
-//   near      per corrected cell (one warp): p = far + 0.98 * sum(BEM-near weights . history)
+//   near      per corrected cell (half a warp): p = far + 0.98 * sum(BEM-near weights . history)
 //             (pppm.cu:53-113) and, in the same pass over the same pairs and history taps, the
 //             FDTD-near sum of the NEXT step (its taps are t-14..t, all final now), stored in
 //             the grid slot the next stencil writes.  One pass over the pair list per step
@@ -578,7 +578,7 @@ __global__ void __launch_bounds__(256) pml_kernel(const __grid_constant__ StepAr
 // The FP32 sums run two layers wide: fma.rn.f32x2 multiplies a tap's (single, double) weights by
 // its (N, D) values, so a tap costs two conversions and one multiply-add, and a record's two sums
 // meet its scales (-single, double) once.  Measured on the convolution and the near-field terms at
-// 6400 triangles, where both were bound by instruction issue: see conv_groups and near_terms2.
+// 6400 triangles, where both were bound by instruction issue: see conv_groups and near_terms4.
 // sum over 4 taps of weights times history, both layers
 template <typename R>
 __device__ inline typename WRec<R>::P dot4(const typename WRec<R>::P (&w)[4], const typename WRec<R>::P (&h)[4])
@@ -1713,7 +1713,7 @@ long long branch_steps(const Handle &h)
     return kBranchSteps * 1000000 / (1000000 + h.pf_cap + h.n_cells);
 }
 
-// The kernels of nsteps steps as a multi-branch graph (absorbing boundary with a mesh).  Per step:
+// The kernels of nsteps steps as a multi-branch graph (with a mesh).  Per step:
 //   side   conv(k)                       after finish(k-1): needs D[t-1] and N[t]
 //   main   stencil(k) -> finish(k) -> near(k)   finish waits for conv(k) too
 // so each step's face-pair convolution (the heavy part of the face stage) runs beside the
@@ -1728,7 +1728,9 @@ long long branch_steps(const Handle &h)
 // The bulk writes p^{t+1} at other cells than the main branch reads or writes in the meantime (the
 // near stage's next-step sums go to corrected cells of slot t+2 = t-1, which the bulk reads only
 // elsewhere), so it leaves the step's critical path.  Only used under stream capture: main =
-// h.stream, side = h.side, bulk = h.side2, joined back before the end.
+// h.stream, side = h.side, bulk = h.side2, joined back before the end.  (capture_pipelined; the PML's update
+// is not split.)
+
 // after a chunk graph of g steps (run_steps): the call's state moves on by g steps
 __global__ void advance_state_kernel(StepState *st, int g, int nt)
 {
@@ -1738,10 +1740,6 @@ __global__ void advance_state_kernel(StepState *st, int g, int nt)
         st->acc += (long long)g * nt;
 }
 
-// open: the nsteps steps are a chunk of a longer call (run_steps), so the last of them is no
-// call's last step (nsteps is a multiple of kPass then, so the passes are those of the whole
-// call); a kernel after the joins moves the call's state on by nsteps for the next chunk, whose
-// first kernel writes what its first step needs.
 // the face-pair convolution of step k, or the completion of its sum
 template <typename R>
 void launch_conv(const StepLaunch<R> &L, int k, PassAt p, cudaStream_t s, bool dependent = false)
@@ -1797,6 +1795,10 @@ void launch_finish(const StepLaunch<R> &L, int k, int mode, int conv_pos, int ne
     }
 }
 
+// open: the nsteps steps are a chunk of a longer call (run_steps), so the last of them is no
+// call's last step (nsteps is a multiple of kPass then, so the passes are those of the whole
+// call); a kernel after the joins moves the call's state on by nsteps for the next chunk, whose
+// first kernel writes what its first step needs.
 template <typename R>
 void capture_pipelined(Handle &h, const StepLaunch<R> &L, int nsteps, bool pair, bool open)
 {
