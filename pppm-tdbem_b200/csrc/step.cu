@@ -1054,7 +1054,7 @@ __device__ inline void group_conv(const R *window, const FaceArgs<R> &f, const C
 // two would share more, but take registers that cost more warps than that gains: four centres,
 // 6400 triangles, conv4 13.0 against 12.2 us).  Measured, four steps against two passes over two steps
 // by the kernel before this one: res 64 (480 k pairs, in L2) 13.3 against 21.0 us, res 128 (6.0 M
-// pairs, 431 MB, from HBM) 119 against 198 us.  Weights by bulk copies into shared memory (two stages
+// pairs, 431 MB of weights and scales, from HBM) 119 against 198 us.  Weights by bulk copies into shared memory (two stages
 // a warp) were slower in both (18.7 and 150 us): the pass is then bound by its instructions.
 template <typename R, int T>
 __device__ inline void conv_groups(const Ring<R> &ring, int tnew, const FaceArgs<R> &f, int blk, int nblk, R *conv)

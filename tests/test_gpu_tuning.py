@@ -1,8 +1,8 @@
 """Launch options of the recorded step graphs and the face-stage autotuner, on the B200.
 
-The two-step face-pair convolution (conv2 + fix: one pass over the pairs' weights for two
-consecutive steps) sums the same products as one pass per step, with the term of D[t] added after
-the rest instead of among it.  Tolerances: FP64 series of the two variants within 1e-12 relative
+The face-pair convolution of several steps (conv4 or conv2 + fix: one pass over the pairs' weights for four or
+two consecutive steps) sums the same products as one pass per step, with the terms of the pass's own
+Dirichlet values added after the rest instead of among it.  Tolerances: FP64 series of the two variants within 1e-12 relative
 L2 over 300 steps (the algebra is the same); FP32 within 1e-6 over the first 50 steps and 1e-4
 over 300 (reassociation only: the scheme amplifies rounding differences step after step, and
 summing the same pairs in reverse order already moves a 300-step FP32 series by ~3e-5); both
